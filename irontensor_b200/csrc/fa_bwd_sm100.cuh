@@ -363,7 +363,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     } else if (warp == 0) {
       // ------------------------------------------------------------ TMA producer
       // (K, V and the first query tile's loads were issued by this thread before the CTA-wide set-up barrier.)
-      if (lane == 0) {
+      if (elect_one()) {
         int g = 0, qi = i0, t = 0;   // iteration 0
         for (int n = 1; n < n_iter; ++n) {
           advance(g, qi, t);
@@ -372,7 +372,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       }
     } else if (warp == 1) {
       // ------------------------------------------------------------ MMA issuer (one thread)
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t IDESC_SS = make_idesc(128, 128, false, false);   // S^T, dP^T
         constexpr uint32_t IDESC_ND = make_idesc(128, D, false, true);      // dV, dK (B N-major)
         constexpr uint32_t IDESC_DQ = make_idesc(128, D, true, true);       // dQ (A M-major, B N-major)
@@ -494,7 +494,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       // Adds each staged 128 x 32 chunk of a dQ tile into the fp32 accumulator (TMA reduce-add) and hands the
       // staging buffers back to the drain warps.  A thread of its own: the drain warps then never wait for a
       // reduce to be issued or for its read of shared memory to finish.
-      if (lane == 0) {
+      if (elect_one()) {
         bool ok = true;
         int g = 0;
         int g_q = 0, qi = i0, t_q = 0;

@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(288, 1) fa_fwd_f32_sm100_kernel(const FwdF32Pa
     }
   } else if (warp == 8) {
     // ------------------------------------------------------------ MMA issuer (one thread)
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC_S = make_idesc(128, 128, false, false);
       constexpr uint32_t IDESC_PV = make_idesc(128, T::DP, false, true);
       const uint32_t q_addr = smem_addr(smem + T::SMEM_Q), k_addr = smem_addr(smem + T::SMEM_K),

@@ -192,7 +192,7 @@ fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     } else if (warp == 0) {
       // ------------------------------------------------------------ TMA producer
       // (the query tile and K tile 0 were issued by this thread before the set-up barrier)
-      if (lane == 0) {
+      if (elect_one()) {
         for (int i = 1; i < nkv; ++i) {
           const int st = i % T::STAGES;
           const uint32_t ph = (i / T::STAGES) & 1;
@@ -208,7 +208,7 @@ fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       // because K runs two tiles ahead of V (S(j+2) is issued while P(j) is still being computed) and a
       // wait for a free V stage must not hold back the next K tile.
       // (V tile 0 was issued by thread 0 before the set-up barrier)
-      if (lane == 0) {
+      if (elect_one()) {
         for (int i = 1; i < nkv; ++i) {
           const int st = i % T::STAGES;
           const uint32_t ph = (i / T::STAGES) & 1;
@@ -223,7 +223,7 @@ fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       // ------------------------------------------------------------ MMA issuer for S = Q K^T (one thread)
       // The two MMA streams have no ordering between them (S and P have separate TMEM columns), so each
       // has its own issuing thread: while one sits in a barrier wait the other keeps the tensor core fed.
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t IDESC_S = make_idesc(128, 128, false, false);
         const uint32_t k_addr = smem_addr(smem + T::SMEM_K);
         auto issue_s = [&](int j) {   // S(j) = Q * K(j)^T into S buffer j&1: Q from TMEM, K K-major from shared memory
@@ -252,7 +252,7 @@ fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       }
     } else if (warp == 2) {
       // ------------------------------------------------------------ MMA issuer for O += P V (one thread)
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t IDESC_PV = make_idesc(128, D, false, true);
         const uint32_t v_addr = smem_addr(smem + T::SMEM_V);
         bool ok = true;

@@ -225,7 +225,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     } else if (warp == 0) {
       // ------------------------------------------------------------ TMA producer
       // (the first item's query tiles and key/value tile 0 were issued by this thread before the set-up barrier)
-      if (lane == 0) {
+      if (elect_one()) {
         uint32_t g = 0;               // key/value tiles issued so far
         uint32_t q_uses[2] = {0, 0};  // items so far that had query tile t
         bool ok = true;
@@ -247,7 +247,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       }
     } else if (warp == 1) {
       // ------------------------------------------------------------ MMA issuer (one thread)
-      if (lane == 0) {
+      if (elect_one()) {
         constexpr uint32_t IDESC_S = make_idesc(128, 128, false, false);
         constexpr uint32_t IDESC_PV = make_idesc(128, D, false, true);
         const uint32_t q_addr = smem_addr(smem + T::SMEM_Q);
@@ -331,7 +331,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       }
     } else if (warp == 3) {
       // ------------------------------------------------------------ work-item scheduler (one thread)
-      if (lane == 0 && prm.work_counter != nullptr) {
+      if (prm.work_counter != nullptr && elect_one()) {
         for (uint32_t n = 0;; ++n) {
           // the slot's previous item (n - 2) has been released by every role
           if (n >= 2 && !mbar_wait(&sched_empty[n & 1], ((n >> 1) - 1) & 1, abort_flag, prm.status, DEV_ERR_TIMEOUT_EMPTY)) break;

@@ -145,7 +145,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   if (!run) {
     // nothing to do
   } else if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       prefetch_tensormap(&tmap_a);
       prefetch_tensormap(&tmap_b);
       int it = 0;   // stage use counter
@@ -180,7 +180,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t IDESC = make_idesc(T::BM, T::BN, LAYOUT == 2, LAYOUT != 0);
       int it = 0, t = 0;
       bool ok = true;
@@ -209,7 +209,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       }
     }
   } else if (warp == 3) {
-    if (RS && lane == 0) {
+    if (RS && elect_one()) {
       // reduce-add issuer: pieces in the order the epilogue produces them
       int g = 0;
       bool ok = true;
