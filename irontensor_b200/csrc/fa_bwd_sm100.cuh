@@ -66,6 +66,7 @@ struct BwdParams {
   const float* lse2_pad;   // [BH, S_pad] LSE * log2(e), +inf in the padding
   const float* delta_pad;  // [BH, S_pad] rowsum(dO*O), 0 in the padding
   float* dq_accum;         // [BH, S, D] fp32, zeroed by the caller
+  const float2* rope_table;   // [S][head_dim / 2] (cos, sin) for the rotation of dK back, or null
   __nv_bfloat16* dk;       // [BH, S, D]
   __nv_bfloat16* dv;       // [BH, S, D]
   int* status;
@@ -73,7 +74,8 @@ struct BwdParams {
   int S_pad;
   int BH;
   int causal;
-  float scale;             // 1/sqrt(D)
+  int head_dim;            // columns of the tensors: D, or fewer in the PAD instantiations
+  float scale;             // 1/sqrt(head_dim)
   float scale_log2;        // scale * log2(e)
 };
 
@@ -83,12 +85,14 @@ struct BwdParams {
 // row).  A row is read by 16 lanes (16 bytes per lane at head_dim 128, 8 at 64), so a warp covers two
 // rows per load; all eight loads of a lane are issued before the first is used (with one row per warp
 // the kernel ran at 70 % of the HBM rate for want of bytes in flight, and 4-byte loads at head_dim 64
-// kept half as many bytes in flight as at 128).
-template <int D>
+// kept half as many bytes in flight as at 128).  PAD: rows of head_dim < D columns; the lanes past them stay at zero.
+// ROPE: the launch also builds the rotary table (an instantiation of its own: the code of the sines alone cost 4 of 45 us).
+template <int D, bool PAD = false, bool ROPE = false>
 __global__ void fa_bwd_prepare_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                                       const float* __restrict__ lse, float* __restrict__ lse2_pad,
                                       float* __restrict__ delta_pad, float* __restrict__ dq_accum, int S, int S_pad,
-                                      int BH, ptx::TensorStrides st) {
+                                      int BH, int head_dim, ptx::TensorStrides st, float2* __restrict__ rope_table,
+                                      const __grid_constant__ RopeFreqs freqs) {
   constexpr int NP = 4;            // passes; a pass covers two rows, one per half-warp
   constexpr int RW = 2 * NP;       // rows per warp; S_pad is a multiple of 128, so they share a head
   constexpr int EL = D / 16;       // elements per lane and row: 8 (D = 128) or 4 (D = 64)
@@ -96,7 +100,11 @@ __global__ void fa_bwd_prepare_kernel(const __nv_bfloat16* __restrict__ o, const
   const int sub = lane & 15, half = lane >> 4;
   ptx::grid_dep_wait();     // O and LSE come from the kernel in front (the forward); the accumulator it clears may still be read
   ptx::grid_dep_launch();   // the main kernel may set itself up meanwhile; it waits for this pass before its first load
-  const long long row0 = ((static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * RW;
+  const long long tid = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const long long row0 = (tid >> 5) * RW;
+  // The rotation of dQ and dK back needs each position's sines and cosines once per head: evaluated here once per call, not
+  // by the finish pass and the dK epilogue.
+  if (ROPE) rope_fill_table(rope_table, S, head_dim >> 1, freqs, tid, static_cast<long long>(gridDim.x) * blockDim.x);
   if (row0 >= static_cast<long long>(BH) * S_pad) return;
   const int bh = static_cast<int>(row0 / S_pad);
   const int s0 = static_cast<int>(row0 % S_pad);
@@ -106,7 +114,7 @@ __global__ void fa_bwd_prepare_kernel(const __nv_bfloat16* __restrict__ o, const
     a[r] = make_uint4(0u, 0u, 0u, 0u);
     b[r] = make_uint4(0u, 0u, 0u, 0u);
     const int s_ = s0 + 2 * r + half;
-    if (s_ < S) {
+    if (s_ < S && (!PAD || sub * EL < head_dim)) {
       const size_t base = static_cast<size_t>(st.slice(bh) + static_cast<long long>(s_) * st.row);
       if (EL == 8) {
         a[r] = reinterpret_cast<const uint4*>(o + base)[sub];
@@ -125,9 +133,12 @@ __global__ void fa_bwd_prepare_kernel(const __nv_bfloat16* __restrict__ o, const
   for (int r = 0; r < NP; ++r) {
     const int s_ = s0 + 2 * r + half;
     if (s_ < S) {
-      float* acc_row = dq_accum + (static_cast<size_t>(bh) * S + s_) * D;   // the accumulator is always [BH, S, D]
+      float* acc_row = dq_accum + (static_cast<size_t>(bh) * S + s_) * (PAD ? head_dim : D);   // the accumulator is always [BH, S, head_dim]
       const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (EL == 8) {   // 512 bytes per row: two 256-byte halves, each written by the 16 lanes at once
+      if (PAD) {
+        if (sub * 4 < head_dim) reinterpret_cast<float4*>(acc_row)[sub] = z;
+        if (EL == 8 && 64 + sub * 4 < head_dim) reinterpret_cast<float4*>(acc_row)[16 + sub] = z;
+      } else if (EL == 8) {   // 512 bytes per row: two 256-byte halves, each written by the 16 lanes at once
         reinterpret_cast<float4*>(acc_row)[sub] = z;
         reinterpret_cast<float4*>(acc_row)[16 + sub] = z;
       } else {
@@ -168,11 +179,11 @@ __global__ void fa_bwd_prepare_kernel(const __nv_bfloat16* __restrict__ o, const
 }
 
 // ------------------------------------------------------------------ (3) finish
-// With freqs.enabled the gradient is rotated back through the rotary embedding on its way out
+// With a rotary table the gradient is rotated back through the rotary embedding on its way out
 // (src/shaders/backward/rope.metal:25-62), so dq is the gradient of the un-rotated queries.
 __global__ void fa_bwd_finish_kernel(const float* __restrict__ dq_accum, __nv_bfloat16* __restrict__ dq,
                                      size_t n_vec4, float scale, int S, int D, ptx::TensorStrides st,
-                                     const __grid_constant__ RopeFreqs freqs) {
+                                     const float2* __restrict__ rope_table) {
   ptx::grid_dep_wait();   // every reduce-add of the main kernel has landed
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n_vec4) return;
@@ -182,13 +193,9 @@ __global__ void fa_bwd_finish_kernel(const float* __restrict__ dq_accum, __nv_bf
   const int d = static_cast<int>(e - row * D);
   const int bh = static_cast<int>(row / S);
   const int s_ = static_cast<int>(row - static_cast<size_t>(bh) * S);
-  if (freqs.enabled) {
-    float c, sn;
-    rope_sincos(freqs, s_ + freqs.position_offset, d >> 1, &c, &sn);
-    const float a0 = v.x * c + v.y * sn, a1 = v.y * c - v.x * sn;
-    rope_sincos(freqs, s_ + freqs.position_offset, (d >> 1) + 1, &c, &sn);
-    const float b0 = v.z * c + v.w * sn, b1 = v.w * c - v.z * sn;
-    v = make_float4(a0, a1, b0, b1);
+  if (rope_table != nullptr) {
+    const float4 cs = *reinterpret_cast<const float4*>(rope_table + static_cast<size_t>(s_) * (D >> 1) + (d >> 1));
+    v = make_float4(v.x * cs.x + v.y * cs.y, v.y * cs.x - v.x * cs.y, v.z * cs.z + v.w * cs.w, v.w * cs.z - v.z * cs.w);
   }
   uint2 w;
   w.x = ptx::pack_bf16(v.x * scale, v.y * scale);
@@ -197,12 +204,13 @@ __global__ void fa_bwd_finish_kernel(const float* __restrict__ dq_accum, __nv_bf
 }
 
 // ------------------------------------------------------------------ (2) main kernel
-template <int D, int KT = 1>
+// PAD: tensors with fewer columns than D (see fa_fwd_sm100.cuh): zero-filled on load, the contractions over the head
+// dimension and the widths of dV, dK and dQ stop at the last 16-column step that holds data.
+template <int D, int KT = 1, bool PAD = false>
 __global__ void __launch_bounds__(512, 1)
 fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
-                    const __grid_constant__ CUtensorMap tmap_dq, const BwdParams prm,
-                    const __grid_constant__ RopeFreqs freqs) {
+                    const __grid_constant__ CUtensorMap tmap_dq, const BwdParams prm) {
   using T = BwdTraits<D, KT>;
   using namespace ptx;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -374,8 +382,9 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       // ------------------------------------------------------------ MMA issuer (one thread)
       if (elect_one()) {
         constexpr uint32_t IDESC_SS = make_idesc(128, 128, false, false);   // S^T, dP^T
-        constexpr uint32_t IDESC_ND = make_idesc(128, D, false, true);      // dV, dK (B N-major)
-        constexpr uint32_t IDESC_DQ = make_idesc(128, D, true, true);       // dQ (A M-major, B N-major)
+        const int d_steps = PAD ? (prm.head_dim + 15) >> 4 : D / 16;        // 16-column steps that hold data
+        const uint32_t IDESC_ND = make_idesc(128, PAD ? d_steps * 16 : D, false, true);   // dV, dK (B N-major)
+        const uint32_t IDESC_DQ = make_idesc(128, PAD ? d_steps * 16 : D, true, true);    // dQ (A M-major, B N-major)
         const uint32_t k_addr = smem_addr(smem + T::SMEM_K);
         const uint32_t v_addr = smem_addr(smem + T::SMEM_V);
         const uint32_t q_addr = smem_addr(smem + T::SMEM_Q);
@@ -393,6 +402,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             if (kk == D / 32) mid();
+            if (PAD && kk >= d_steps) continue;
             umma_ss(tmem_base + T::COL_ST, sdesc_advance(da, kmajor_off(kk)), sdesc_advance(db, kmajor_off(kk)),
                     IDESC_SS, kk > 0);
           }
@@ -404,6 +414,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             if (kk == D / 32) mid();
+            if (PAD && kk >= d_steps) continue;
             umma_ss(tmem_base + T::COL_DPT, sdesc_advance(da, kmajor_off(kk)), sdesc_advance(db, kmajor_off(kk)),
                     IDESC_SS, kk > 0);
           }
@@ -502,6 +513,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           const int bh_q = bh0 + g_q;
 #pragma unroll
           for (int c = 0; c < D / 32; ++c, ++g) {
+            if (PAD && c * 32 >= prm.head_dim) break;
             const int buf = g & 1;
             if (!mbar_wait(&dqs_full[buf], static_cast<uint32_t>(g >> 1) & 1, abort_flag, prm.status, DEV_ERR_TIMEOUT_SOFTMAX)) {
               ok = false;
@@ -639,19 +651,26 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           for (int c = 0; c < HC / 16; ++c) {
             tmem_ld_x16(t_lane + col + c * 16, ra);
             tmem_wait_ld();
-            if (which && freqs.enabled) {   // dK leaves through the inverse rotary rotation of its key position
+            if (which && prm.rope_table != nullptr && k_row < S) {   // dK leaves through the inverse rotary rotation of its key position
+              const int d0 = half * HC + c * 16;
+              const float4* tab = reinterpret_cast<const float4*>(
+                  prm.rope_table + static_cast<size_t>(k_row) * ((PAD ? prm.head_dim : D) >> 1) + (d0 >> 1));
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                float cs, sn;
-                rope_sincos(freqs, k_row + freqs.position_offset, (half * HC + c * 16) / 2 + j, &cs, &sn);
-                const float g0 = __uint_as_float(ra[2 * j]), g1 = __uint_as_float(ra[2 * j + 1]);
-                ra[2 * j] = __float_as_uint(g0 * cs + g1 * sn);
-                ra[2 * j + 1] = __float_as_uint(g1 * cs - g0 * sn);
+              for (int j = 0; j < 4; ++j) {
+                if (PAD && d0 + 4 * j >= prm.head_dim) break;
+                const float4 cs = tab[j];   // (cos, sin) of two pairs
+                const float g0 = __uint_as_float(ra[4 * j]), g1 = __uint_as_float(ra[4 * j + 1]);
+                const float h0 = __uint_as_float(ra[4 * j + 2]), h1 = __uint_as_float(ra[4 * j + 3]);
+                ra[4 * j] = __float_as_uint(g0 * cs.x + g1 * cs.y);
+                ra[4 * j + 1] = __float_as_uint(g1 * cs.x - g0 * cs.y);
+                ra[4 * j + 2] = __float_as_uint(h0 * cs.z + h1 * cs.w);
+                ra[4 * j + 3] = __float_as_uint(h1 * cs.z - h0 * cs.w);
               }
             }
             if (k_row < S) {
 #pragma unroll
               for (int v4 = 0; v4 < 2; ++v4) {
+                if (PAD && half * HC + c * 16 + v4 * 8 >= prm.head_dim) break;
                 uint4 w;
                 w.x = pack_bf16(__uint_as_float(ra[v4 * 8 + 0]) * f, __uint_as_float(ra[v4 * 8 + 1]) * f);
                 w.y = pack_bf16(__uint_as_float(ra[v4 * 8 + 2]) * f, __uint_as_float(ra[v4 * 8 + 3]) * f);
@@ -690,6 +709,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         mbar_arrive(dq_empty);
 #pragma unroll
         for (int c = 0; c < D / 32; ++c, ++g) {
+          if (PAD && c * 32 >= prm.head_dim) break;
           const int buf = g & 1;
           const uint32_t use = static_cast<uint32_t>(g >> 1);
           uint8_t* stage = smem + T::SMEM_DQS + buf * T::BLOCK_BYTES;

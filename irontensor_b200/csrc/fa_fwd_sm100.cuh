@@ -2,7 +2,7 @@
 // CTA sharing each K/V tile.  The launcher uses it for head_dim 64 and for sequences below 5120 keys
 // (fa_fwd_pp_sm100.cuh takes head_dim 128 from 5120 keys on).
 //
-// Replaces, for bf16 tensors with head_dim 64 or 128, the reference project's forward kernels
+// Replaces, for bf16 tensors (head_dim 64 or 128, and any other multiple of 8 up to 128 zero-padded to those), the reference project's forward kernels
 // (src/shaders/flash_attention.metal:45-163 online softmax; :167-223 exact softmax) and adds the
 // per-row log-sum-exp output the fused backward needs.
 //
@@ -53,7 +53,8 @@ struct FwdParams {
   int S;
   int BH;
   int causal;
-  float scale_log2;     // 1/sqrt(D) * log2(e)
+  float scale_log2;     // 1/sqrt(head_dim) * log2(e)
+  int head_dim;         // columns of the tensors: D, or fewer in the PAD instantiations
   int kv_group;         // query heads per K/V head (grouped-query attention; 1 otherwise)
   int group_slices;     // fa_fwd_sm100_kernel: slices per group of its work-item order
   int* work_counter;    // fa_fwd_sm100_kernel: zeroed before the launch when the grid is smaller than the number of work items, else null
@@ -64,7 +65,10 @@ struct FwdParams {
   float* dec_part_ml;   // [B*H, n_splits, 2] reference maximum (log2 domain) and row sum of each split
 };
 
-template <int D>
+// PAD: tensors with fewer columns than D (any multiple of 8).  TMA fills the missing columns of every tile with zeros, so
+// the shared-memory image is that of a D-column tensor; the MMAs run over the 16-column steps that hold data and the store
+// stops at the last real column.  Instantiations of their own, so that the loops of the full-width kernels stay compile-time.
+template <int D, bool PAD = false>
 __global__ void __launch_bounds__(384, 1)
 fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const FwdParams prm) {
@@ -249,7 +253,8 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       // ------------------------------------------------------------ MMA issuer (one thread)
       if (elect_one()) {
         constexpr uint32_t IDESC_S = make_idesc(128, 128, false, false);
-        constexpr uint32_t IDESC_PV = make_idesc(128, D, false, true);
+        const int d_steps = PAD ? (prm.head_dim + 15) >> 4 : D / 16;   // 16-column steps that hold data
+        const uint32_t IDESC_PV = make_idesc(128, PAD ? d_steps * 16 : D, false, true);
         const uint32_t q_addr = smem_addr(smem + T::SMEM_Q);
         const uint32_t k_addr = smem_addr(smem + T::SMEM_K);
         const uint32_t v_addr = smem_addr(smem + T::SMEM_V);
@@ -258,6 +263,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           const uint64_t dk = make_sdesc(k_addr + st * T::TILE_BYTES, 16, 1024);
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
+            if (PAD && kk >= d_steps) break;
             const uint32_t off = (kk >> 2) * T::BLOCK_BYTES + (kk & 3) * 32;
             umma_ss(tmem_base + t * 128, sdesc_advance(dq, off), sdesc_advance(dk, off), IDESC_S, kk > 0);
           }
@@ -465,6 +471,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       if (q_row < S) {
 #pragma unroll
         for (int v = 0; v < D / 8; ++v) {
+          if (PAD && v * 8 >= prm.head_dim) break;
           uint4 w;
           w.x = pack_bf16(__uint_as_float(r[v * 8 + 0]) * inv_l, __uint_as_float(r[v * 8 + 1]) * inv_l);
           w.y = pack_bf16(__uint_as_float(r[v * 8 + 2]) * inv_l, __uint_as_float(r[v * 8 + 3]) * inv_l);

@@ -212,9 +212,12 @@ cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<Args>(args))...);
 }
 
-// The tensor-core kernels take bf16 tensors with head_dim 64 or 128 and at least one full tile.
+// The tensor-core kernels take bf16 tensors whose rows TMA can address (a multiple of 8 columns = 16 bytes); rows past the
+// sequence and columns past head_dim are zero-filled on load.  head_dim other than 64 and 128 runs the PAD instantiations of
+// the next larger of the two (B2 H16 S1003 D96, grouped heads, forward + backward: 4.8 ms on the CUDA-core kernels, 0.14 ms).
+// Below 48 rows, or 16 columns, most of a 128 x 64 tile would be padding and the CUDA-core kernels are as quick.
 bool use_sm100_path(it_dtype dtype, int32_t S, int32_t D) {
-  return dtype == IT_BF16 && (D == 64 || D == 128) && S >= 128;
+  return dtype == IT_BF16 && (D & 7) == 0 && D >= 16 && S >= 48;
 }
 
 int round_dp(int D) { return D <= 16 ? 16 : D <= 32 ? 32 : D <= 64 ? 64 : 128; }
@@ -330,20 +333,21 @@ it_status launch_bwd_generic(it_ctx* ctx, cudaStream_t s, int BH, int S, int D, 
 // The two tensor-core forward kernels: one query tile per CTA with the softmax groups alternating over key
 // tiles (long sequences: the tensor core never waits for a softmax), or two query tiles per CTA sharing
 // each K/V tile (short sequences: half as many CTA start-ups per unit of work).
-template <int D, bool PP>
-it_status launch_fwd_sm100(it_ctx* ctx, it_stream* stream, int B, int H, int S, int causal, const void* q, const void* k,
-                           const void* v, void* o, float* lse, const it::TensorStrides& stv,
+template <int D, bool PP, bool PAD = false>
+it_status launch_fwd_sm100(it_ctx* ctx, it_stream* stream, int B, int H, int S, int head_dim, int causal, const void* q,
+                           const void* k, const void* v, void* o, float* lse, const it::TensorStrides& stv,
                            const it::TensorStrides& skv, const it::TensorStrides& sq) {
+  static_assert(!(PP && PAD), "the long-sequence kernel takes full-width tensors only");
   const int BH = B * H;
   const int Hkv = H / skv.group;
   cudaStream_t s = stream->s;
   using T = std::conditional_t<PP, it::FwdPPTraits<D>, it::FwdTraits<D>>;
-  auto kernel = PP ? it::fa_fwd_pp_sm100_kernel<D> : it::fa_fwd_sm100_kernel<D>;
+  auto kernel = PP ? it::fa_fwd_pp_sm100_kernel<D> : it::fa_fwd_sm100_kernel<D, PAD>;
   CUtensorMap mq, mk, mv;
   it_status st;
-  if ((st = make_tmap(ctx, &mq, q, B, H, S, D, sq, 128)) != IT_OK) return st;
-  if ((st = make_tmap(ctx, &mk, k, B, Hkv, S, D, skv, 128)) != IT_OK) return st;
-  if ((st = make_tmap(ctx, &mv, v, B, Hkv, S, D, skv, 128)) != IT_OK) return st;
+  if ((st = make_tmap(ctx, &mq, q, B, H, S, head_dim, sq, 128)) != IT_OK) return st;
+  if ((st = make_tmap(ctx, &mk, k, B, Hkv, S, head_dim, skv, 128)) != IT_OK) return st;
+  if ((st = make_tmap(ctx, &mv, v, B, Hkv, S, head_dim, skv, 128)) != IT_OK) return st;
   static std::atomic<bool> attr_set[16];   // zero-initialised; setting an attribute twice is harmless
   if (!attr_set[ctx->device & 15]) {
     IT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES));
@@ -357,7 +361,8 @@ it_status launch_fwd_sm100(it_ctx* ctx, it_stream* stream, int B, int H, int S, 
   p.S = S;
   p.BH = BH;
   p.causal = causal;
-  p.scale_log2 = (1.0f / sqrtf(static_cast<float>(D))) * 1.4426950408889634f;
+  p.head_dim = head_dim;
+  p.scale_log2 = (1.0f / sqrtf(static_cast<float>(head_dim))) * 1.4426950408889634f;
   p.kv_group = skv.group;
   // Slices whose work items the two-query-tile kernel hands out together (heaviest pairs of all of them first): as many
   // as have 40 MB of K and V at head_dim 128, 96 MB at head_dim 64, in groups of equal size.  Measured on B200 (causal): at
@@ -404,29 +409,32 @@ it_status launch_fwd_sm100(it_ctx* ctx, it_stream* stream, int B, int H, int S, 
 }
 
 struct BwdWorkspace {
-  size_t dq_accum_off, lse2_off, delta_off, total;
+  size_t dq_accum_off, lse2_off, delta_off, rope_off;
+  size_t plain, total;   // bytes needed without / with the rotary table
   int S_pad;
 };
-BwdWorkspace bwd_workspace_layout(it_dtype dtype, int64_t BH, int64_t S, int64_t D) {
+BwdWorkspace bwd_workspace_layout(it_dtype dtype, int64_t BH, int64_t S, int64_t D, bool cuda_cores = false) {
   BwdWorkspace w{};
   auto up = [](size_t x) { return (x + 255) & ~static_cast<size_t>(255); };
-  if (use_sm100_path(dtype, static_cast<int32_t>(S), static_cast<int32_t>(D))) {
+  if (!cuda_cores && use_sm100_path(dtype, static_cast<int32_t>(S), static_cast<int32_t>(D))) {
     w.S_pad = static_cast<int>((S + 127) / 128 * 128);
     w.dq_accum_off = 0;
     w.lse2_off = up(static_cast<size_t>(BH) * S * D * 4);
     w.delta_off = w.lse2_off + up(static_cast<size_t>(BH) * w.S_pad * 4);
-    w.total = w.delta_off + up(static_cast<size_t>(BH) * w.S_pad * 4);
+    w.rope_off = w.delta_off + up(static_cast<size_t>(BH) * w.S_pad * 4);
   } else {
     w.S_pad = static_cast<int>(S);
     w.delta_off = 0;
-    w.total = up(static_cast<size_t>(BH) * S * 4);
+    w.rope_off = up(static_cast<size_t>(BH) * S * 4);
   }
-  if (w.total == 0) w.total = 256;
+  const bool table = (D & 1) == 0 && !cuda_cores && use_sm100_path(dtype, static_cast<int32_t>(S), static_cast<int32_t>(D));
+  w.plain = std::max<size_t>(w.rope_off, 256);
+  w.total = std::max<size_t>(w.rope_off + (table ? up(static_cast<size_t>(S) * (D / 2) * sizeof(float2)) : 0), 256);
   return w;
 }
 
-template <int D>
-it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int causal, const void* q, const void* k,
+template <int D, bool PAD = false>
+it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int head_dim, int causal, const void* q, const void* k,
                            const void* v, const void* o, const void* d_o, const float* lse, void* dq, void* dk,
                            void* dv, uint8_t* ws, const BwdWorkspace& w, const it::TensorStrides& stv,
                            const it::TensorStrides& skv, const it::RopeFreqs& rf, const it::TensorStrides& sq) {
@@ -435,15 +443,15 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
   using T = it::BwdTraits<D>;
   CUtensorMap mq, mk, mv, mdo;
   it_status st;
-  if ((st = make_tmap(ctx, &mq, q, B, H, S, D, sq, 128)) != IT_OK) return st;
-  if ((st = make_tmap(ctx, &mk, k, B, Hkv, S, D, skv, 128)) != IT_OK) return st;
-  if ((st = make_tmap(ctx, &mv, v, B, Hkv, S, D, skv, 128)) != IT_OK) return st;
-  if ((st = make_tmap(ctx, &mdo, d_o, B, H, S, D, stv, 128)) != IT_OK) return st;
-  // fp32 dQ accumulator [BH, S, D]: boxes of 32 columns x 128 rows for the TMA reduce-add
+  if ((st = make_tmap(ctx, &mq, q, B, H, S, head_dim, sq, 128)) != IT_OK) return st;
+  if ((st = make_tmap(ctx, &mk, k, B, Hkv, S, head_dim, skv, 128)) != IT_OK) return st;
+  if ((st = make_tmap(ctx, &mv, v, B, Hkv, S, head_dim, skv, 128)) != IT_OK) return st;
+  if ((st = make_tmap(ctx, &mdo, d_o, B, H, S, head_dim, stv, 128)) != IT_OK) return st;
+  // fp32 dQ accumulator [BH, S, head_dim]: boxes of 32 columns x 128 rows for the TMA reduce-add
   CUtensorMap mdq;
   {
-    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(S), static_cast<cuuint64_t>(BH)};
-    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(D) * 4, static_cast<cuuint64_t>(S) * D * 4};
+    const cuuint64_t dims[3] = {static_cast<cuuint64_t>(head_dim), static_cast<cuuint64_t>(S), static_cast<cuuint64_t>(BH)};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(head_dim) * 4, static_cast<cuuint64_t>(S) * head_dim * 4};
     const cuuint32_t box[3] = {32, 128, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = ctx->encode(&mdq, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, ws + w.dq_accum_off, dims, strides, box, estr,
@@ -453,28 +461,30 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
   }
   static std::atomic<bool> attr_set[16];   // zero-initialised; setting an attribute twice is harmless
   if (!attr_set[ctx->device & 15]) {
-    IT_CUDA(cudaFuncSetAttribute(it::fa_bwd_sm100_kernel<D, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    IT_CUDA(cudaFuncSetAttribute(it::fa_bwd_sm100_kernel<D, 1, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  it::BwdTraits<D, 1>::SMEM_BYTES));
     if constexpr (D == 64)
-      IT_CUDA(cudaFuncSetAttribute(it::fa_bwd_sm100_kernel<D, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      IT_CUDA(cudaFuncSetAttribute(it::fa_bwd_sm100_kernel<D, 2, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    it::BwdTraits<D, 2>::SMEM_BYTES));
     attr_set[ctx->device & 15] = true;
   }
   float* dq_accum = reinterpret_cast<float*>(ws + w.dq_accum_off);
   float* lse2 = reinterpret_cast<float*>(ws + w.lse2_off);
   float* delta = reinterpret_cast<float*>(ws + w.delta_off);
-  const size_t n_dq = static_cast<size_t>(BH) * S * D;
+  float2* rope_table = rf.enabled ? reinterpret_cast<float2*>(ws + w.rope_off) : nullptr;
+  const size_t n_dq = static_cast<size_t>(BH) * S * head_dim;
   const long long rows_pad = static_cast<long long>(BH) * w.S_pad;
   if (ctx->timing >= 3) IT_CUDA(cudaEventRecord(ctx->ev[2][0], s));
-  IT_CUDA(launch_dependent(it::fa_bwd_prepare_kernel<D>, static_cast<unsigned>((rows_pad / 8 + 7) / 8), 256, 0, s,   // 8 rows per warp, 8 warps
+  IT_CUDA(launch_dependent(rf.enabled ? it::fa_bwd_prepare_kernel<D, PAD, true> : it::fa_bwd_prepare_kernel<D, PAD>, static_cast<unsigned>((rows_pad / 8 + 7) / 8), 256, 0, s,   // 8 rows per warp, 8 warps
                            static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(d_o), lse, lse2, delta, dq_accum, S,
-                           w.S_pad, BH, stv));
+                           w.S_pad, BH, head_dim, stv, rope_table, rf));
   it::BwdParams p;
   p.st = stv;
   p.st_kv = skv;
   p.lse2_pad = lse2;
   p.delta_pad = delta;
   p.dq_accum = dq_accum;
+  p.rope_table = rope_table;
   p.dk = static_cast<__nv_bfloat16*>(dk);
   p.dv = static_cast<__nv_bfloat16*>(dv);
   p.status = ctx->d_status;
@@ -482,7 +492,8 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
   p.S_pad = w.S_pad;
   p.BH = BH;
   p.causal = causal;
-  p.scale = 1.0f / sqrtf(static_cast<float>(D));
+  p.head_dim = head_dim;
+  p.scale = 1.0f / sqrtf(static_cast<float>(head_dim));
   p.scale_log2 = p.scale * 1.4426950408889634f;
   const int n_kt = (S + 127) / 128;
   // At head_dim 64 a CTA can own two key tiles (tensor memory holds four accumulators of 64 columns): half as many
@@ -499,12 +510,12 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
   if (ctx->timing) IT_CUDA(cudaEventRecord(ctx->ev[1][0], s));
   if constexpr (D == 64) {
     if (two_tiles)
-      IT_CUDA(launch_dependent(it::fa_bwd_sm100_kernel<D, 2>, static_cast<unsigned>((n_kt + 1) / 2) * B * Hkv, T::THREADS,
-                               it::BwdTraits<D, 2>::SMEM_BYTES, s, mq, mk, mv, mdo, mdq, p, rf));
+      IT_CUDA(launch_dependent(it::fa_bwd_sm100_kernel<D, 2, PAD>, static_cast<unsigned>((n_kt + 1) / 2) * B * Hkv, T::THREADS,
+                               it::BwdTraits<D, 2>::SMEM_BYTES, s, mq, mk, mv, mdo, mdq, p));
   }
   if (!two_tiles)
-    IT_CUDA(launch_dependent(it::fa_bwd_sm100_kernel<D, 1>, static_cast<unsigned>(n_kt) * B * Hkv, T::THREADS, T::SMEM_BYTES, s,
-                             mq, mk, mv, mdo, mdq, p, rf));
+    IT_CUDA(launch_dependent(it::fa_bwd_sm100_kernel<D, 1, PAD>, static_cast<unsigned>(n_kt) * B * Hkv, T::THREADS, T::SMEM_BYTES, s,
+                             mq, mk, mv, mdo, mdq, p));
   if (ctx->timing) {
     IT_CUDA(cudaEventRecord(ctx->ev[1][1], s));
     ctx->ev_valid[1] = true;
@@ -512,7 +523,7 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
   if (ctx->timing >= 3) IT_CUDA(cudaEventRecord(ctx->ev[3][0], s));
   const size_t n4 = n_dq / 4;
   IT_CUDA(launch_dependent(it::fa_bwd_finish_kernel, static_cast<unsigned>((n4 + 255) / 256), 256, 0, s,
-                           static_cast<const float*>(dq_accum), static_cast<__nv_bfloat16*>(dq), n4, p.scale, S, D, sq, rf));
+                           static_cast<const float*>(dq_accum), static_cast<__nv_bfloat16*>(dq), n4, p.scale, S, head_dim, sq, static_cast<const float2*>(rope_table)));
   if (ctx->timing >= 3) {
     IT_CUDA(cudaEventRecord(ctx->ev[3][1], s));
     ctx->ev_valid[3] = true;
@@ -642,6 +653,7 @@ it_status launch_decode_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int Hkv
   p.S = kv_len;
   p.BH = B * H;
   p.causal = 0;
+  p.head_dim = D;
   p.scale_log2 = (1.0f / sqrtf(static_cast<float>(D))) * 1.4426950408889634f;
   p.kv_group = G;
   p.group_slices = 1;
@@ -930,7 +942,7 @@ static it_status attention_fwd_impl(it_ctx* ctx, it_stream* stream, it_dtype dty
   it::TensorStrides sq = sv;
   if (qkv_row != 0) {   // q, k and v are column ranges of one [batch, seq, qkv_row] buffer
     if (!use_sm100_path(dtype, S, D))
-      return fail(IT_ERR_UNSUPPORTED_SHAPE, "the packed layout needs bf16, head_dim 64 or 128 and seq >= 128");
+      return fail(IT_ERR_UNSUPPORTED_SHAPE, "the packed layout needs bf16, a head_dim that is a multiple of 8 from 16 on, and seq >= 48");
     sq.row = skv.row = qkv_row;
     sq.batch = skv.batch = qkv_row * S;
   }
@@ -940,11 +952,10 @@ static it_status attention_fwd_impl(it_ctx* ctx, it_stream* stream, it_dtype dty
     // IT_FWD_KERNEL=pp|two in the environment overrides the choice (A/B runs).
     const char* force = getenv("IT_FWD_KERNEL");
     const bool pp = (force != nullptr) ? (force[0] == 'p') : ((D == 128) && (S >= 5120));
-    if (D == 128)
-      return pp ? launch_fwd_sm100<128, true>(ctx, stream, B, H, S, causal != 0, q, k, v, o, lse, sv, skv, sq)
-                : launch_fwd_sm100<128, false>(ctx, stream, B, H, S, causal != 0, q, k, v, o, lse, sv, skv, sq);
-    return pp ? launch_fwd_sm100<64, true>(ctx, stream, B, H, S, causal != 0, q, k, v, o, lse, sv, skv, sq)
-              : launch_fwd_sm100<64, false>(ctx, stream, B, H, S, causal != 0, q, k, v, o, lse, sv, skv, sq);
+    auto launch = D == 128 ? (pp ? launch_fwd_sm100<128, true> : launch_fwd_sm100<128, false>)
+                  : D == 64 ? (pp ? launch_fwd_sm100<64, true> : launch_fwd_sm100<64, false>)
+                  : D > 64 ? launch_fwd_sm100<128, false, true> : launch_fwd_sm100<64, false, true>;
+    return launch(ctx, stream, B, H, S, D, causal != 0, q, k, v, o, lse, sv, skv, sq);
   }
   return dtype == IT_F32 ? launch_fwd_generic<float>(ctx, stream->s, BH, S, D, causal != 0, q, k, v, o, lse, sv, skv)
                          : launch_fwd_generic<__nv_bfloat16>(ctx, stream->s, BH, S, D, causal != 0, q, k, v, o, lse, sv, skv);
@@ -997,7 +1008,8 @@ static it_status attention_bwd_impl(it_ctx* ctx, it_stream* stream, it_dtype dty
                                     int32_t S, int32_t D, int32_t causal, const void* q, const void* k, const void* v,
                                     const void* o, const void* d_o, const float* lse, void* dq, void* dk, void* dv,
                                     void* workspace, size_t workspace_bytes, bool bshd,
-                                    const it::RopeFreqs& rf = make_rope_freqs(0, 1.f, 0, false), long long qkv_row = 0) {
+                                    const it::RopeFreqs& rf = make_rope_freqs(0, 1.f, 0, false), long long qkv_row = 0,
+                                    bool built_in_scratch = false, bool cuda_cores = false) {
   it_status st = check_common(ctx, stream, dtype, B, H, S, D);
   if (st != IT_OK) return st;
   if (H > 0 && (st = check_kv_heads(H, Hkv)) != IT_OK) return st;
@@ -1009,9 +1021,10 @@ static it_status attention_bwd_impl(it_ctx* ctx, it_stream* stream, it_dtype dty
   if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o) || !aligned16(d_o) || !aligned16(dq) ||
       !aligned16(dk) || !aligned16(dv))
     return fail(IT_ERR_ALIGNMENT, "tensors must be 16-byte aligned");
-  const BwdWorkspace w = bwd_workspace_layout(dtype, BH, S, D);
-  if (workspace == nullptr || workspace_bytes < w.total)
-    return fail(IT_ERR_INVALID_ARG, "workspace of %zu bytes needed, %zu given", w.total, workspace_bytes);
+  const BwdWorkspace w = bwd_workspace_layout(dtype, BH, S, D, cuda_cores);
+  const size_t need = built_in_scratch ? w.plain : w.total;
+  if (workspace == nullptr || workspace_bytes < need)
+    return fail(IT_ERR_INVALID_ARG, "workspace of %zu bytes needed, %zu given", need, workspace_bytes);
   if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
     return fail(IT_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
   IT_CUDA(cudaSetDevice(ctx->device));
@@ -1021,14 +1034,14 @@ static it_status attention_bwd_impl(it_ctx* ctx, it_stream* stream, it_dtype dty
   it::TensorStrides sq = sv;
   if (qkv_row != 0) {   // q, k, v (and dq, dk, dv) are column ranges of one [batch, seq, qkv_row] buffer each
     if (!use_sm100_path(dtype, S, D))
-      return fail(IT_ERR_UNSUPPORTED_SHAPE, "the packed layout needs bf16, head_dim 64 or 128 and seq >= 128");
+      return fail(IT_ERR_UNSUPPORTED_SHAPE, "the packed layout needs bf16, a head_dim that is a multiple of 8 from 16 on, and seq >= 48");
     sq.row = skv.row = qkv_row;
     sq.batch = skv.batch = qkv_row * S;
   }
-  if (use_sm100_path(dtype, S, D)) {
-    return D == 128
-               ? launch_bwd_sm100<128>(ctx, stream->s, B, H, S, causal != 0, q, k, v, o, d_o, lse, dq, dk, dv, ws, w, sv, skv, rf, sq)
-               : launch_bwd_sm100<64>(ctx, stream->s, B, H, S, causal != 0, q, k, v, o, d_o, lse, dq, dk, dv, ws, w, sv, skv, rf, sq);
+  if (!cuda_cores && use_sm100_path(dtype, S, D)) {
+    auto launch = D == 128 ? launch_bwd_sm100<128> : D == 64 ? launch_bwd_sm100<64>
+                  : D > 64 ? launch_bwd_sm100<128, true> : launch_bwd_sm100<64, true>;
+    return launch(ctx, stream->s, B, H, S, D, causal != 0, q, k, v, o, d_o, lse, dq, dk, dv, ws, w, sv, skv, rf, sq);
   }
   float* delta = reinterpret_cast<float*>(ws + w.delta_off);
   return dtype == IT_F32
@@ -1304,7 +1317,12 @@ it_status it_flash_attention_bwd_noalloc(it_ctx* ctx, it_stream* stream, it_dtyp
   it_status st = check_common(ctx, stream, dtype, B, H, S, D);
   if (st != IT_OK) return st;
   if (S == 0 || B * H == 0) return IT_OK;
-  const size_t need = bwd_workspace_layout(dtype, static_cast<int64_t>(B) * H, S, D).total;
+  // A shape whose dQ accumulator does not fit runs on the CUDA-core kernels, which need two orders of magnitude less scratch;
+  // the full-width tensor-core shapes (head_dim 64 or 128, a full tile of rows) are refused instead, as ever.
+  const int64_t BH = static_cast<int64_t>(B) * H;
+  const bool full_width = (D == 64 || D == 128) && S >= 128;
+  const bool cuda_cores = !full_width && bwd_workspace_layout(dtype, BH, S, D).plain > IT_NOALLOC_SCRATCH_BYTES;
+  const size_t need = bwd_workspace_layout(dtype, BH, S, D, cuda_cores).plain;
   if (need > IT_NOALLOC_SCRATCH_BYTES)
     return fail(IT_ERR_UNSUPPORTED_SHAPE,
                 "this shape needs %zu bytes of scratch; the built-in scratch of the allocation-free backward holds %u",
@@ -1325,8 +1343,8 @@ it_status it_flash_attention_bwd_noalloc(it_ctx* ctx, it_stream* stream, it_dtyp
   }
   // The regular entry point clears the dQ accumulator and rewrites the per-row arrays on every call,
   // so nothing left in the array by an earlier call is read.
-  return it_flash_attention_bwd(ctx, stream, dtype, B, H, S, D, causal, q, k, v, o, d_o, lse, dq, dk, dv, scratch,
-                                IT_NOALLOC_SCRATCH_BYTES);
+  return attention_bwd_impl(ctx, stream, dtype, B, H, H, S, D, causal, q, k, v, o, d_o, lse, dq, dk, dv, scratch,
+                            IT_NOALLOC_SCRATCH_BYTES, false, make_rope_freqs(0, 1.f, 0, false), 0, true, cuda_cores);
 }
 
 it_status it_host_step_destroy(it_host_step* hs) {

@@ -65,14 +65,21 @@ rope_qk_kernel(const ST* __restrict__ q_in, const ST* __restrict__ k_in, ST* __r
   }
 }
 
-// (cos, sin) of every (sequence index, dimension pair): [S][D/2] float2.  Built once per call by kernels
-// that would otherwise evaluate the same sine and cosine in every column tile (the fused QKV projection).
+// (cos, sin) of every (sequence index, dimension pair): [S][D/2] float2.  Built once per call for kernels that would
+// otherwise evaluate the same sine and cosine once per head (the attention backward) or per column tile (the fused QKV
+// projection).  `first` and `stride` number the threads that share the work.
+__device__ __forceinline__ void rope_fill_table(float2* table, int S, int half, const RopeFreqs& freqs, long long first, long long stride) {
+  const long long n = static_cast<long long>(S) * half;
+  for (long long i = first; i < n; i += stride) {
+    const int pos = static_cast<int>(i / half), pair = static_cast<int>(i - static_cast<long long>(pos) * half);
+    float c, s;
+    rope_sincos(freqs, pos + freqs.position_offset, pair, &c, &s);
+    table[i] = make_float2(c, s);
+  }
+}
 __global__ void rope_table_kernel(float2* __restrict__ table, int S, int half, const __grid_constant__ RopeFreqs freqs) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= S * half) return;
-  float c, s;
-  rope_sincos(freqs, i / half + freqs.position_offset, i % half, &c, &s);
-  table[i] = make_float2(c, s);
+  rope_fill_table(table, S, half, freqs, static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x,
+                  static_cast<long long>(gridDim.x) * blockDim.x);
 }
 
 }  // namespace it
