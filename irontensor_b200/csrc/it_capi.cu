@@ -25,6 +25,7 @@
 #include "fa_decode.cuh"
 #include "fa_fwd_pp_sm100.cuh"
 #include "fa_fwd_f32_sm100.cuh"
+#include "fa_bwd_f32_sm100.cuh"
 #include "gemm_sm100.cuh"
 #include "fa_generic.cuh"
 #include "selftest_sm100.cuh"
@@ -220,6 +221,11 @@ bool use_sm100_path(it_dtype dtype, int32_t S, int32_t D) {
   return dtype == IT_BF16 && (D & 7) == 0 && D >= 16 && S >= 48;
 }
 
+// The fp32 backward on the tensor cores.
+bool use_f32_bwd_sm100(it_dtype dtype, int32_t S, int32_t D) {
+  return dtype == IT_F32 && (D & 3) == 0 && D <= 64 && S >= 32;
+}
+
 int round_dp(int D) { return D <= 16 ? 16 : D <= 32 ? 32 : D <= 64 ? 64 : 128; }
 
 template <typename ST>
@@ -330,6 +336,45 @@ it_status launch_bwd_generic(it_ctx* ctx, cudaStream_t s, int BH, int S, int D, 
   return IT_OK;
 }
 
+it_status launch_bwd_f32_sm100(it_ctx* ctx, cudaStream_t s, int BH, int S, int D, int causal, const void* q, const void* k, const void* v,
+                               const void* o, const void* d_o, const float* lse, void* dq, void* dk, void* dv, float* delta,
+                               float2* rope_table, const it::TensorStrides& st, const it::TensorStrides& skv, const it::RopeFreqs& rf) {
+  using T = it::BwdF32Traits;
+  static std::atomic<bool> attr_set[16];
+  if (!attr_set[ctx->device & 15]) {
+    IT_CUDA(cudaFuncSetAttribute(it::fa_bwd_f32_sm100_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES));
+    attr_set[ctx->device & 15] = true;
+  }
+  const long long rows = static_cast<long long>(BH) * S;
+  IT_CUDA(launch_dependent(it::fa_bwd_f32_prepare_kernel, static_cast<unsigned>((rows + 63) / 64), 256, 0, s, static_cast<const float*>(o),
+                           static_cast<const float*>(d_o), delta, rows, S, D, st, rope_table, rf));
+  it::BwdF32Params p;
+  p.q = static_cast<const float*>(q);
+  p.k = static_cast<const float*>(k);
+  p.v = static_cast<const float*>(v);
+  p.d_o = static_cast<const float*>(d_o);
+  p.lse = lse;
+  p.delta = delta;
+  p.dq = static_cast<float*>(dq);
+  p.dk = static_cast<float*>(dk);
+  p.dv = static_cast<float*>(dv);
+  p.rope_table = rope_table;
+  p.st = st;
+  p.st_kv = skv;
+  p.status = ctx->d_status;
+  p.S = S;
+  p.D = D;
+  p.BH = BH;
+  p.causal = causal;
+  p.scale = 1.0f / sqrtf(static_cast<float>(D));
+  p.scale_log2 = p.scale * 1.4426950408889634f;
+  const unsigned n_tiles = (S + T::BM - 1) / T::BM;
+  IT_CUDA(launch_dependent(it::fa_bwd_f32_sm100_kernel, n_tiles * (BH + BH / skv.group), T::THREADS, T::SMEM_BYTES, s, p));
+  ctx->launches += 2;
+  IT_CUDA(cudaGetLastError());
+  return IT_OK;
+}
+
 // The two tensor-core forward kernels: one query tile per CTA with the softmax groups alternating over key
 // tiles (long sequences: the tensor core never waits for a softmax), or two query tiles per CTA sharing
 // each K/V tile (short sequences: half as many CTA start-ups per unit of work).
@@ -427,7 +472,8 @@ BwdWorkspace bwd_workspace_layout(it_dtype dtype, int64_t BH, int64_t S, int64_t
     w.delta_off = 0;
     w.rope_off = up(static_cast<size_t>(BH) * S * 4);
   }
-  const bool table = (D & 1) == 0 && !cuda_cores && use_sm100_path(dtype, static_cast<int32_t>(S), static_cast<int32_t>(D));
+  const bool table = (D & 1) == 0 && !cuda_cores && (use_sm100_path(dtype, static_cast<int32_t>(S), static_cast<int32_t>(D)) ||
+                                                     use_f32_bwd_sm100(dtype, static_cast<int32_t>(S), static_cast<int32_t>(D)));
   w.plain = std::max<size_t>(w.rope_off, 256);
   w.total = std::max<size_t>(w.rope_off + (table ? up(static_cast<size_t>(S) * (D / 2) * sizeof(float2)) : 0), 256);
   return w;
@@ -1044,6 +1090,9 @@ static it_status attention_bwd_impl(it_ctx* ctx, it_stream* stream, it_dtype dty
     return launch(ctx, stream->s, B, H, S, D, causal != 0, q, k, v, o, d_o, lse, dq, dk, dv, ws, w, sv, skv, rf, sq);
   }
   float* delta = reinterpret_cast<float*>(ws + w.delta_off);
+  if (!cuda_cores && use_f32_bwd_sm100(dtype, S, D) && getenv("IT_F32_CUDA_CORES") == nullptr)
+    return launch_bwd_f32_sm100(ctx, stream->s, BH, S, D, causal != 0, q, k, v, o, d_o, lse, dq, dk, dv, delta,
+                                rf.enabled ? reinterpret_cast<float2*>(ws + w.rope_off) : nullptr, sv, skv, rf);
   return dtype == IT_F32
              ? launch_bwd_generic<float>(ctx, stream->s, BH, S, D, causal != 0, q, k, v, o, d_o, lse, dq, dk, dv, delta, sv, skv, rf)
              : launch_bwd_generic<__nv_bfloat16>(ctx, stream->s, BH, S, D, causal != 0, q, k, v, o, d_o, lse, dq, dk, dv, delta,

@@ -92,3 +92,27 @@ def test_noalloc_backward_of_a_padded_shape_beyond_the_scratch(it_ctx):
     want = ol.bwd(*[gu.to_host(t[sl].contiguous()) for t in (q, k, v, d_o)], True)
     for got, w, name in zip(g, want, ("dQ", "dK", "dV")):
         check_bf16(gu.to_host(got[sl].contiguous()), w, name)
+
+
+@pytest.mark.parametrize("B,S,H,Hkv,D,causal,rope", [
+    (2, 32, 4, 4, 64, True, False), (1, 33, 3, 3, 20, False, False), (1, 127, 2, 2, 64, True, True), (2, 128, 4, 2, 32, True, False),
+    (1, 129, 4, 4, 64, False, True), (1, 257, 6, 2, 60, True, True), (1, 400, 2, 1, 4, False, False), (1, 640, 4, 4, 64, True, False),
+])
+def test_fp32_backward_on_the_tensor_cores(it_ctx, B, S, H, Hkv, D, causal, rope):
+    """The split-operand fp32 backward at the edges of its tiles.  Tolerance: the path's 1e-4; the operands carry 24 bits and
+    the sums are fp32, so the error is that of fp32 sums of a few hundred terms of order one (1e-6 to 1e-5)."""
+    from irontensor_b200 import Tensor, attention_gqa, attention_gqa_backward
+    q, _, _, d_o = [np.ascontiguousarray(t.transpose(0, 2, 1, 3)) for t in seeded(940 + S, B, H, S, D)]
+    _, k, v, _ = [np.ascontiguousarray(t.transpose(0, 2, 1, 3)) for t in seeded(941 + S, B, Hkv, S, D)]
+    tq, tk, tv, tdo = (Tensor.from_f32_slice(t.reshape(-1), list(t.shape)) for t in (q, k, v, d_o))
+    o = attention_gqa(tq, tk, tv, causal)
+    dq, dk, dv = attention_gqa_backward(tdo, tq, tk, tv, o, causal, rope_base=10000.0 if rope else None, position_offset=7)
+    assert it_ctx.poll_status() == 0
+    rdq, rdk, rdv = ol.gqa_bwd(q, k, v, d_o, causal)
+    if rope:
+        rdq, rdk = ol.rope(rdq, 10000.0, 7, inverse=True), ol.rope(rdk, 10000.0, 7, inverse=True)
+    for got, want, name in ((dq, rdq, "dQ"), (dk, rdk, "dK"), (dv, rdv, "dV")):
+        g = got.to_f32_host()
+        assert not np.isnan(g).any()
+        assert np.abs(g - want).max() <= 1e-4, f"{name}: {np.abs(g - want).max():.2e}"
+        assert np.linalg.norm(g - want) <= 1e-5 * np.linalg.norm(want), name
