@@ -57,7 +57,7 @@ struct FwdParams {
   int head_dim;         // columns of the tensors: D, or fewer in the PAD instantiations
   int kv_group;         // query heads per K/V head (grouped-query attention; 1 otherwise)
   int group_slices;     // fa_fwd_sm100_kernel: slices per group of its work-item order
-  int* work_counter;    // fa_fwd_sm100_kernel: zeroed before the launch when the grid is smaller than the number of work items, else null
+  int* work_counter;    // fa_fwd_sm100_kernel: zero before and after the launch, when the grid is smaller than the number of work items; else null
   // decode instantiation of the long-sequence kernel only (one new token against a key/value cache):
   int dec_tiles_per_split;   // key tiles per CTA
   int dec_n_splits;
@@ -343,7 +343,11 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           if (n >= 2 && !mbar_wait(&sched_empty[n & 1], ((n >> 1) - 1) & 1, abort_flag, prm.status, DEV_ERR_TIMEOUT_EMPTY)) break;
           int idx = static_cast<int>(blockIdx.x);
           if (n > 0) {
-            idx = G + atomicAdd(prm.work_counter, 1);
+            const int drawn = atomicAdd(prm.work_counter, 1);
+            // n_items draws are made in all: n_items - G that find an item and the G that end the CTAs.  The last one leaves the
+            // counter at zero for the next launch on this stream, so no memset stands in front of the launch.
+            if (drawn == n_items - 1) *prm.work_counter = 0;
+            idx = G + drawn;
             if (idx >= n_items) idx = -1;
           }
           sched_item[n & 1] = idx;

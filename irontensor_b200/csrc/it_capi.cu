@@ -433,10 +433,9 @@ it_status launch_fwd_sm100(it_ctx* ctx, it_stream* stream, int B, int H, int S, 
   p.work_counter = nullptr;
   if (!PP && grid > ctx->sm_count) {
     // One CTA per SM; each draws its next work item from a counter (one per stream: launches on a stream run one
-    // after the other), zeroed in front of the launch.  IT_FWD_ONE_ITEM_PER_CTA=1 launches one CTA per item instead.
+    // after the other), which the launch leaves at zero.  IT_FWD_ONE_ITEM_PER_CTA=1 launches one CTA per item instead.
     const char* one = getenv("IT_FWD_ONE_ITEM_PER_CTA");
     if (stream->d_work != nullptr && (one == nullptr || one[0] != '1')) {
-      IT_CUDA(cudaMemsetAsync(stream->d_work, 0, sizeof(int), s));
       stream->work_used = true;
       p.work_counter = stream->d_work;
       grid = ctx->sm_count;
@@ -796,6 +795,7 @@ it_status it_ctx_create(int device, it_ctx** out) {
   c->encode = reinterpret_cast<EncodeTiledFn>(fn);
   if (cudaMalloc(&c->d_status, sizeof(int)) != cudaSuccess || cudaMemset(c->d_status, 0, sizeof(int)) != cudaSuccess ||
       cudaMalloc(&c->d_work_pool, it_ctx::WORK_SLOTS * sizeof(int)) != cudaSuccess ||
+      cudaMemset(c->d_work_pool, 0, it_ctx::WORK_SLOTS * sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&c->h_status, sizeof(int)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->status_stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete c;
@@ -1514,6 +1514,8 @@ it_status it_attention_status_poll(it_ctx* ctx, it_stream* stream, int32_t* devi
   if (rc != IT_OK) return rc;
   *device_status = word;
   if (*device_status != 0) {
+    // a launch that gave up may not have made all its draws: the work-item counters start over as well
+    IT_CUDA(cudaMemsetAsync(ctx->d_work_pool, 0, it_ctx::WORK_SLOTS * sizeof(int), stream->s));
     IT_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), stream->s));
     IT_CUDA(cudaStreamSynchronize(stream->s));
     return fail(IT_ERR_TIMEOUT, "a bounded wait inside a kernel ran out (device status %d)", *device_status);
