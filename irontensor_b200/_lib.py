@@ -106,6 +106,31 @@ def load():
     return _lib
 
 
+class _Missing:
+    """Stands in for _host_ops before it is built (the package can be imported to build it); using it raises."""
+
+    def __init__(self, why):
+        class TensorBase:
+            def __init__(self, *a):
+                raise ImportError(why)
+        self.TensorBase, self.setup = TensorBase, (lambda *a: None)
+        self._why = why
+
+    def __getattr__(self, name):
+        raise ImportError(self._why)
+
+
+def host_ops():
+    """The native host side of the ops (csrc/host_ops.cpp)."""
+    import torch  # noqa: F401  (the extension links torch's libraries)
+    try:
+        from . import _host_ops
+        return _host_ops
+    except ImportError as e:
+        return _Missing(f"irontensor_b200/_host_ops.so cannot be loaded ({e}): build it with `python -m irontensor_b200.build` "
+                        "(there is no CPU or PyTorch fallback)")
+
+
 def check(status):
     if status != IT_OK:
         raise ITError(status, load().it_last_error().decode("utf-8", "replace"))

@@ -11,6 +11,10 @@ Where the reference asserts (panics), these raise AssertionError with the same m
 torch is used for plumbing only: device memory, the current CUDA stream and pinned host buffers.
 All arithmetic runs in libirontensor_b200.so; if that library cannot be loaded, or no CUDA device
 is present, every op raises -- there is no fallback.
+
+An op's ordinary case (tensors that fit together, nothing empty) is checked, allocated and launched by the native function of
+the same name in _host_ops (csrc/host_ops.cpp): a launch-bound call spends 5 us on the host instead of 30 to 130.  It answers
+None to anything else, and the Python code below it then raises the reference's assertion or handles the case.
 """
 import ctypes
 import enum
@@ -19,6 +23,8 @@ import threading
 import numpy as np
 
 from . import _lib, synth
+
+_host_ops = _lib.host_ops()
 
 
 class Precision(enum.Enum):
@@ -166,25 +172,27 @@ class CommandBatch:
         _state.pending = None
 
 
-class Tensor:
+class Tensor(_host_ops.TensorBase):
     """Device-resident tensor: buffer + shape + precision (src/tensor.rs:11-15).
 
+    The base class holds the torch CUDA tensor (float32 or bfloat16) and has the accessors shape(), precision(), numel(),
+    data_ptr() and torch(), and `lse`: the side output of the attention ops, a Tensor [B,H,S] fp32, None elsewhere.
     The reference's buffers are unified memory, so `as_f32_slice` aliases GPU memory
     (src/tensor.rs:136-148); here it synchronises the stream and copies device -> host."""
 
     def __init__(self, data, shape, precision):
-        self._data = data            # flat torch CUDA tensor (float32 or bfloat16)
-        self._shape = list(shape)
-        self._precision = precision
-        self.lse = None              # side output of flash_attention: Tensor [B,H,S] fp32
+        self._set(data.view(list(shape)))    # `data`: a torch CUDA tensor of that many elements
+
+    @property
+    def _data(self):
+        return self.torch().view(-1)
 
     # -- constructors (src/tensor.rs:63-118, 205-240)
     @staticmethod
     def zeros(shape, precision=Precision.FP32):
         torch = _torch()
         dt = torch.float32 if precision is Precision.FP32 else torch.bfloat16
-        n = int(np.prod(shape)) if len(shape) else 1
-        return Tensor(torch.zeros(max(n, 1), dtype=dt, device="cuda")[:n], shape, precision)
+        return Tensor(torch.zeros(list(shape), dtype=dt, device="cuda"), shape, precision)
 
     @staticmethod
     def from_f32_slice(data, shape):
@@ -212,8 +220,7 @@ class Tensor:
         """Uninitialised storage, for outputs a kernel overwrites completely."""
         torch = _torch()
         dt = torch.float32 if precision is Precision.FP32 else torch.bfloat16
-        n = int(np.prod(shape)) if len(shape) else 1
-        return Tensor(torch.empty(max(n, 1), dtype=dt, device="cuda")[:n], shape, precision)
+        return Tensor(torch.empty(list(shape), dtype=dt, device="cuda"), shape, precision)
 
     # -- explicit, stream-ordered copies to and from page-locked host memory
     def upload_from(self, host):
@@ -231,63 +238,50 @@ class Tensor:
         return host
 
     # -- accessors
-    def shape(self):
-        return list(self._shape)
-
-    def precision(self):
-        return self._precision
-
-    def numel(self):
-        return int(np.prod(self._shape)) if self._shape else 1
-
     def byte_size(self):
-        return self.numel() * self._precision.byte_size()
+        return self.numel() * self.precision().byte_size()
 
     def is_bf16(self):
-        return self._precision is Precision.BF16
+        return self.precision() is Precision.BF16
 
     def is_f32(self):
-        return self._precision is Precision.FP32
-
-    def data_ptr(self):
-        return self._data.data_ptr()
-
-    def torch(self):
-        return self._data.view(self._shape)
+        return self.precision() is Precision.FP32
 
     def as_f32_slice(self):
-        assert self._precision is Precision.FP32, "Tensor is not FP32"
+        assert self.precision() is Precision.FP32, "Tensor is not FP32"
         host = self._data.cpu().numpy()      # drains the stream
-        context(self._data.device.index).check_status()   # a kernel that gave up leaves garbage here: raise instead
+        context(self.torch().device.index).check_status()   # a kernel that gave up leaves garbage here: raise instead
         return host
 
     def as_bf16_slice(self):
-        assert self._precision is Precision.BF16, "Tensor is not BF16"
+        assert self.precision() is Precision.BF16, "Tensor is not BF16"
         torch = _torch()
         host = self._data.view(torch.int16).cpu().numpy().view(np.uint16)
-        context(self._data.device.index).check_status()
+        context(self.torch().device.index).check_status()
         return host
 
     def to_f32_host(self):
         """Values as fp32 on the host, whatever the storage precision."""
-        if self._precision is Precision.FP32:
-            return self.as_f32_slice().reshape(self._shape)
-        return synth.bf16_bits_to_f32(self.as_bf16_slice()).reshape(self._shape)
+        if self.precision() is Precision.FP32:
+            return self.as_f32_slice().reshape(self.shape())
+        return synth.bf16_bits_to_f32(self.as_bf16_slice()).reshape(self.shape())
 
     def view(self, new_shape):
-        n = int(np.prod(new_shape))
-        assert n == self.numel(), f"Cannot view tensor with {self.numel()} elements as shape {list(new_shape)}"
-        t = Tensor(self._data, new_shape, self._precision)
+        t = self._reshaped(new_shape)
+        assert t is not None, f"Cannot view tensor with {self.numel()} elements as shape {list(new_shape)}"
         return t
 
     def to_bf16(self):
-        if self._precision is Precision.BF16:
-            return Tensor(self._data.clone(), self._shape, Precision.BF16)
-        return Tensor.from_f32_as_bf16(self.as_f32_slice(), self._shape)
+        if self.precision() is Precision.BF16:
+            return Tensor(self.torch().clone(), self.shape(), Precision.BF16)
+        return Tensor.from_f32_as_bf16(self.as_f32_slice(), self.shape())
 
     def to_f32(self):
         torch = _torch()
-        return Tensor(self._data.to(torch.float32), self._shape, Precision.FP32)
+        return Tensor(self.torch().to(torch.float32), self.shape(), Precision.FP32)
+
+
+_host_ops.setup(Tensor, Precision.FP32, Precision.BF16, _lib.check, lambda device: context(device))
 
 
 def _dtype_code(p):
@@ -422,6 +416,9 @@ def flash_attention(q, k, v, causal):
 
     Accepts FP32 tensors like the reference and additionally BF16 (all three alike).  The per-row
     log-sum-exp the fused backward needs is attached to the result as `.lse`."""
+    out = _host_ops.flash_attention(q, k, v, causal)
+    if out is not None:
+        return out
     p = q.precision()
     assert p in (Precision.FP32, Precision.BF16)
     assert k.precision() is p and v.precision() is p, "Q, K and V must have the same precision"
@@ -452,6 +449,9 @@ def attention(q, k, v, causal):
     like the reference, and BF16.  The result carries `.lse` ([batch, heads, seq]) for
     attention_backward.  K/V may have another sequence length when not causal, as in the reference
     (src/ops/attention.rs:304,349-352); that case runs on the CUDA-core kernels."""
+    out = _host_ops.attention(q, k, v, causal)
+    if out is not None:
+        return out
     p = q.precision()
     assert k.precision() is p and v.precision() is p
     qs, ks, vs = q.shape(), k.shape(), v.shape()
@@ -483,6 +483,9 @@ def attention_backward(grad_output, q, k, v, o, causal=True):
     """(dQ, dK, dV) for attention(): every tensor is [batch, seq, heads, head_dim]; `o` is attention()'s
     result (with its `.lse`).  The layout-fused counterpart of attention_backward_recompute: the reference
     transposes the gradient in and the three gradients out (src/train/backward.rs:102,114-116)."""
+    out = _host_ops.attention_backward(grad_output, q, k, v, o, causal)
+    if out is not None:
+        return out
     p = q.precision()
     B, S, H, D = q.shape()
     for t in (grad_output, k, v, o):
@@ -504,6 +507,9 @@ def attention_gqa(q, k, v, causal=True):
     kv_heads dividing heads.  Equal to attention(q, repeat_kv(k), repeat_kv(v), causal) of the reference
     (src/train/forward.rs:117-139; repeat_kv_gpu, src/ops/repeat_kv.rs:68-149) without the expanded copies:
     query head h reads K/V head h // (heads // kv_heads).  The result carries `.lse` for attention_gqa_backward."""
+    out = _host_ops.attention_gqa(q, k, v, causal)
+    if out is not None:
+        return out
     p = q.precision()
     assert k.precision() is p and v.precision() is p
     assert len(q.shape()) == 4 and len(k.shape()) == 4 and len(v.shape()) == 4, "Q, K and V must be 4D"
@@ -523,6 +529,9 @@ def attention_gqa(q, k, v, causal=True):
 
 def rope(input, base=10000.0, position_offset=0):
     """Rotary position embedding of one [batch, seq, heads, head_dim] tensor (src/ops/rope.rs:22-75)."""
+    out = _host_ops.rope_qk(input, None, base, position_offset, False)
+    if out is not None:
+        return out
     assert len(input.shape()) == 4, "Input must be 4D [batch, seq_len, num_heads, head_dim]"
     B, S, H, D = input.shape()
     assert D % 2 == 0, "head_dim must be even for RoPE"
@@ -535,6 +544,9 @@ def rope(input, base=10000.0, position_offset=0):
 def rope_qk(q, k, base=10000.0, position_offset=0, inverse=False):
     """rope(q) and rope(k) (src/train/forward.rs:111-112) as one launch; k may have fewer heads.  `inverse`
     gives the backward rotation (rope_backward, src/ops/backward/rope.rs)."""
+    out = _host_ops.rope_qk(q, k, base, position_offset, inverse)
+    if out is not None:
+        return out
     B, S, H, D = q.shape()
     Hkv = k.shape()[2]
     assert k.shape() == [B, S, Hkv, D] and k.precision() is q.precision() and D % 2 == 0
@@ -550,6 +562,9 @@ def attention_gqa_backward(grad_output, q, k, v, o, causal=True, rope_base=None,
     src/train/backward.rs:102-122; src/ops/repeat_kv.rs:151-232).  With `rope_base`, q and k are the rotated
     tensors the forward attended over and dQ, dK come back as gradients of the un-rotated ones: the
     reference's two rope_backward passes (src/train/backward.rs:129,132) folded into this call."""
+    out = _host_ops.attention_gqa_backward(grad_output, q, k, v, o, causal, rope_base, position_offset)
+    if out is not None:
+        return out
     p = q.precision()
     B, S, H, D = q.shape()
     Hkv = k.shape()[2]
@@ -576,6 +591,9 @@ def attention_decode(q, k_cache, v_cache, kv_len):
     [batch, max_len, kv_heads, head_dim] whose first `kv_len` positions are valid (the new token's key and value
     included).  Equals the last row of the causal attention the reference's generator recomputes from scratch for
     every token (src/inference/generator.rs:146-200).  The result carries `.lse` ([batch, heads])."""
+    out = _host_ops.attention_decode(q, k_cache, v_cache, kv_len)
+    if out is not None:
+        return out
     p = q.precision()
     assert k_cache.precision() is p and v_cache.precision() is p
     assert len(q.shape()) == 3 and len(k_cache.shape()) == 4 and k_cache.shape() == v_cache.shape()
@@ -593,6 +611,9 @@ def attention_decode(q, k_cache, v_cache, kv_len):
 
 def linear_forward(input, weight):
     """output = input @ weight.T (src/train/helpers.rs:48-53) for BF16 tensors: input [n, in], weight [out, in]."""
+    out = _host_ops.linear_forward(input, weight)
+    if out is not None:
+        return out
     assert input.precision() is Precision.BF16 and weight.precision() is Precision.BF16, "linear_forward takes BF16 tensors"
     n, k = input.shape()
     out_dim, k2 = weight.shape()
@@ -607,6 +628,9 @@ def qkv_rope_forward(x, w_qkv, heads, kv_heads, head_dim, rope_base=10000.0, pos
     projections of src/train/forward.rs:101-103 and the two rope() calls of :111-112, written directly in the
     [batch, seq, heads, head_dim] layout attention_gqa reads.  rope_base None: no rotation.  packed=True returns ONE
     tensor [batch, seq, (heads + 2*kv_heads)*head_dim] (q_rope | k_rope | v per token) for attention_packed."""
+    out = _host_ops.qkv_rope_forward(x, w_qkv, heads, kv_heads, head_dim, 0.0 if rope_base is None else rope_base, position_offset, packed)
+    if out is not None:
+        return out
     assert x.precision() is Precision.BF16 and w_qkv.precision() is Precision.BF16
     B, S, hidden = x.shape()
     assert w_qkv.shape() == [(heads + 2 * kv_heads) * head_dim, hidden], "w_qkv must be [Wq; Wk; Wv] stacked by rows"
@@ -626,6 +650,9 @@ def qkv_rope_forward(x, w_qkv, heads, kv_heads, head_dim, rope_base=10000.0, pos
 def attention_packed(qkv, heads, kv_heads, head_dim, causal=True):
     """Grouped-query attention on the packed projection output [batch, seq, (heads + 2*kv_heads)*head_dim]
     (qkv_rope_forward(..., packed=True)).  Returns O [batch, seq, heads, head_dim] with `.lse`."""
+    out = _host_ops.attention_packed(qkv, heads, kv_heads, head_dim, causal)
+    if out is not None:
+        return out
     B, S, W = qkv.shape()
     assert qkv.precision() is Precision.BF16 and W == (heads + 2 * kv_heads) * head_dim
     out = Tensor.empty([B, S, heads, head_dim], Precision.BF16)
@@ -638,6 +665,10 @@ def attention_packed_backward(grad_output, qkv, o, heads, kv_heads, head_dim, ca
     """Gradient of attention_packed with respect to the packed tensor, in the same layout (dq | dk | dv per token, dk and dv
     summed over each group, dq and dk rotated back when rope_base is given): ready to be the one `grad_output` of
     linear_backward for the stacked weights [Wq; Wk; Wv]."""
+    out = _host_ops.attention_packed_backward(grad_output, qkv, o, heads, kv_heads, head_dim, causal,
+                                              0.0 if rope_base is None else rope_base, position_offset)
+    if out is not None:
+        return out
     B, S, W = qkv.shape()
     assert grad_output.shape() == [B, S, heads, head_dim] and o.lse is not None
     dqkv = Tensor.empty([B, S, W], Precision.BF16)
@@ -651,6 +682,9 @@ def attention_packed_backward(grad_output, qkv, o, heads, kv_heads, head_dim, ca
 def linear_backward(grad_output, input, weight):
     """(grad_input, grad_weight) = (grad_output @ weight, grad_output.T @ input) (src/train/helpers.rs:61-76);
     grad_input BF16 [n, in], grad_weight FP32 [out, in] (the reference returns FP32 gradients)."""
+    out = _host_ops.linear_backward(grad_output, input, weight)
+    if out is not None:
+        return out
     n, out_dim = grad_output.shape()
     k = input.shape()[1]
     assert input.shape() == [n, k] and weight.shape() == [out_dim, k]
@@ -666,6 +700,9 @@ def attention_backward_recompute(grad_output, q, k, v, o=None, lse=None, causal=
     The reference takes (grad_output, q, k, v) and is always causal.  Pass the forward's `o` and
     `lse` (flash_attention's result and its `.lse`) to skip the recomputation; without them the
     forward is run again here, which is what "recompute" means for the fused path."""
+    out = _host_ops.attention_backward_recompute(grad_output, q, k, v, o, lse, causal)
+    if out is not None:
+        return out
     p = q.precision()
     for t in (grad_output, k, v):
         assert t.precision() is p, "all tensors must have the same precision"
