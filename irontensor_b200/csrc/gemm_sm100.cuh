@@ -8,10 +8,10 @@
 //   LAYOUT 0 (NT): A [M,K], B [N,K]   -> both K-major           y  = x W^T
 //   LAYOUT 1 (NN): A [M,K], B [K,N]   -> A K-major, B N-major   dx = dy W
 //   LAYOUT 2 (TN): A [K,M], B [K,N]   -> A M-major, B N-major   dW = dy^T x
-// Persistent kernel, one CTA per SM, tiles of 128 x 256 handed out round-robin in an order that keeps the
+// Persistent kernel, one CTA per SM, tiles of 128 x 256 (or 128, or 64 columns, where those fill the GPU better) handed out round-robin in an order that keeps the
 // tiles of the CTAs running at one time close together (gemm_tile_coords):
-//   warp 0     : TMA producer, a four-stage ring of (A 128x64, B 256x64) blocks, 128-byte swizzle
-//   warp 1     : MMA issuer, tcgen05.mma 128x256x16, two accumulators of 256 TMEM columns so that the
+//   warp 0     : TMA producer, a ring of four (six, eight) stages of (A 128x64, B 256x64) blocks, 128-byte swizzle
+//   warp 1     : MMA issuer, tcgen05.mma 128x256x16, two accumulators of 256 TMEM columns each so that the
 //                next tile's MMAs run while the previous tile is stored
 //   warp 2     : TMEM allocation / release
 //   warps 4-7  : epilogue, a thread per row: TMEM -> registers -> bf16/fp32 -> global
@@ -23,8 +23,9 @@
 
 namespace it {
 
+template <int BN_ = 256>
 struct GemmTraits {
-  static constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4;
+  static constexpr int BM = 128, BN = BN_, BK = 64, STAGES = BN == 256 ? 4 : BN == 128 ? 6 : 8;
   static constexpr int A_BYTES = BM * BK * 2;      // 16 KB
   static constexpr int B_BYTES = BN * BK * 2;      // 32 KB
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -90,11 +91,11 @@ __device__ __forceinline__ void gemm_tile_coords(int tile, int tiles_m, int tile
 // tile to bf16 into a swizzled staging buffer, and one thread (warp 3) adds it into the copy of C of the rank that
 // owns those rows with a TMA reduce-add -- whole 128-byte lines, over NVLink when the owner is a peer -- while the
 // tensor core is already on the next tile.
-template <int LAYOUT, bool QKV = false, bool RS = false>
+template <int LAYOUT, bool QKV = false, bool RS = false, int BN = 256>
 __global__ void __launch_bounds__(256, 1)
 gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                        const GemmParams prm, const __grid_constant__ GemmScatterMaps rs_maps) {
-  using T = GemmTraits;
+  using T = GemmTraits<BN>;
   using namespace ptx;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + T::SMEM_BAR);
@@ -139,6 +140,8 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dep_wait();     // operands may be what the kernel in front wrote, and the output what it still reads
+  grid_dep_launch();
   const uint32_t tmem_base = *tmem_slot;
   const bool run = (*abort_flag == 0) && n_kb > 0;
 
@@ -171,9 +174,9 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           }
           if (LAYOUT == 0) {   // B [N,K]: 256 rows of 64 K
             tma_load_4d(sb, &tmap_b, &full[st], k0, n0, 0, 0);
-          } else {             // B [K,N]: 64 K-rows of N, four 64-wide N blocks
+          } else {             // B [K,N]: 64 K-rows of N, 64-wide N blocks
 #pragma unroll
-            for (int b = 0; b < 4; ++b) tma_load_4d(sb + b * (T::B_BYTES / 4), &tmap_b, &full[st], n0 + b * 64, k0, 0, 0);
+            for (int b = 0; b < BN / 64; ++b) tma_load_4d(sb + b * (64 * T::BK * 2), &tmap_b, &full[st], n0 + b * 64, k0, 0, 0);
           }
         }
         if (!ok) break;
@@ -198,7 +201,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           // K-major: 8-row groups 1024 bytes apart, a K step of 16 is 32 bytes along the row.
           // MN-major: the next 64 M/N elements one block further, a K step of 16 rows is 2048 bytes.
           const uint64_t da = (LAYOUT == 2) ? make_sdesc(a_addr, T::A_BYTES / 2, 1024) : make_sdesc(a_addr, 16, 1024);
-          const uint64_t db = (LAYOUT == 0) ? make_sdesc(b_addr, 16, 1024) : make_sdesc(b_addr, T::B_BYTES / 4, 1024);
+          const uint64_t db = (LAYOUT == 0) ? make_sdesc(b_addr, 16, 1024) : make_sdesc(b_addr, 64 * T::BK * 2, 1024);
 #pragma unroll
           for (int kk = 0; kk < T::BK / 16; ++kk)
             umma_ss(tmem_base + buf * T::BN, sdesc_advance(da, (LAYOUT == 2) ? kk * 2048 : kk * 32),

@@ -489,13 +489,30 @@ int tensor_clear(PyObject* o) {
   Py_CLEAR(reinterpret_cast<TensorObject*>(o)->lse);
   return 0;
 }
-PyObject* tensor_set(PyObject* o, PyObject* t) {   // the torch tensor of the logical shape
-  if (!THPVariable_Check(t)) {
-    PyErr_SetString(PyExc_TypeError, "a torch tensor is needed");
+bool read_shape(PyObject* shape, c10::SmallVector<int64_t, 6>* dims, int64_t* numel) {
+  PyObject* seq = PySequence_Fast(shape, "a shape is a sequence of numbers");
+  if (seq == nullptr) return false;
+  *numel = 1;
+  for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq); ++i) {
+    dims->push_back(PyLong_AsLongLong(PySequence_Fast_GET_ITEM(seq, i)));
+    *numel *= dims->back();
+  }
+  Py_DECREF(seq);
+  return !PyErr_Occurred();
+}
+PyObject* tensor_set(PyObject* o, PyObject* const* a, Py_ssize_t nargs) {   // torch tensor, logical shape
+  if (nargs != 2 || !THPVariable_Check(a[0])) {
+    PyErr_SetString(PyExc_TypeError, "a torch tensor and a shape are needed");
     return nullptr;
   }
-  ten(o) = THPVariable_Unpack(t);
-  Py_RETURN_NONE;
+  return guard([&]() -> PyObject* {
+    c10::SmallVector<int64_t, 6> dims;
+    int64_t numel;
+    if (!read_shape(a[1], &dims, &numel)) return nullptr;
+    const at::Tensor& t = THPVariable_Unpack(a[0]);
+    ten(o) = t.sizes() == at::IntArrayRef(dims) ? t : t.view(dims);
+    Py_RETURN_NONE;
+  });
 }
 PyObject* tensor_torch(PyObject* o, PyObject*) { return THPVariable_Wrap(ten(o)); }
 PyObject* tensor_shape(PyObject* o, PyObject*) {
@@ -511,24 +528,16 @@ PyObject* tensor_data_ptr(PyObject* o, PyObject*) {
 }
 PyObject* tensor_reshaped(PyObject* o, PyObject* shape) {   // the same memory under another shape; None if the sizes differ
   return guard([&]() -> PyObject* {
-    PyObject* seq = PySequence_Fast(shape, "a shape is a sequence of numbers");
-    if (seq == nullptr) return nullptr;
-    const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
     c10::SmallVector<int64_t, 6> dims;
-    int64_t numel = 1;
-    for (Py_ssize_t i = 0; i < n; ++i) {
-      dims.push_back(PyLong_AsLongLong(PySequence_Fast_GET_ITEM(seq, i)));
-      numel *= dims.back();
-    }
-    Py_DECREF(seq);
-    if (PyErr_Occurred()) return nullptr;
+    int64_t numel;
+    if (!read_shape(shape, &dims, &numel)) return nullptr;
     if (numel != ten(o).numel()) Py_RETURN_NONE;
     return wrap(ten(o).view(dims));
   });
 }
 
 PyMethodDef tensor_methods[] = {
-    {"_set", tensor_set, METH_O, nullptr},
+    {"_set", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(tensor_set)), METH_FASTCALL, nullptr},
     {"torch", tensor_torch, METH_NOARGS, "The torch tensor behind it, in the logical shape."},
     {"shape", tensor_shape, METH_NOARGS, "The shape, as a list."},
     {"precision", tensor_precision, METH_NOARGS, "Precision.FP32 or Precision.BF16."},

@@ -27,6 +27,7 @@
 #include "fa_fwd_f32_sm100.cuh"
 #include "fa_bwd_f32_sm100.cuh"
 #include "gemm_sm100.cuh"
+#include "gemm_skinny.cuh"
 #include "fa_generic.cuh"
 #include "selftest_sm100.cuh"
 
@@ -593,11 +594,11 @@ struct ScatterEpilogue {
   int world, rows_per_rank;
 };
 
-template <int LAYOUT, bool QKV = false, bool RS = false>
-it_status launch_gemm(it_ctx* ctx, cudaStream_t s, int M, int N, int K, const void* a, long long lda, const void* b,
-                      long long ldb, void* c, long long ldc, bool c_is_f32, const QkvEpilogue* epi = nullptr,
-                      const ScatterEpilogue* rs = nullptr) {
-  using T = it::GemmTraits;
+template <int LAYOUT, bool QKV, bool RS, int BN>
+it_status launch_gemm_tiles(it_ctx* ctx, cudaStream_t s, int M, int N, int K, const void* a, long long lda, const void* b,
+                      long long ldb, void* c, long long ldc, bool c_is_f32, const QkvEpilogue* epi,
+                      const ScatterEpilogue* rs) {
+  using T = it::GemmTraits<BN>;
   CUtensorMap ma, mb;
   it_status st;
   const int a_rows = (LAYOUT == 2) ? K : M, a_cols = (LAYOUT == 2) ? M : K;
@@ -607,7 +608,7 @@ it_status launch_gemm(it_ctx* ctx, cudaStream_t s, int M, int N, int K, const vo
   if ((st = make_tmap(ctx, &mb, b, 1, 1, b_rows, b_cols, sb, (LAYOUT == 0) ? T::BN : T::BK)) != IT_OK) return st;
   static std::atomic<bool> attr_set[16];   // zero-initialised; setting an attribute twice is harmless
   if (!attr_set[ctx->device & 15]) {
-    IT_CUDA(cudaFuncSetAttribute(it::gemm_bf16_sm100_kernel<LAYOUT, QKV, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    IT_CUDA(cudaFuncSetAttribute(it::gemm_bf16_sm100_kernel<LAYOUT, QKV, RS, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  T::SMEM_BYTES));
     attr_set[ctx->device & 15] = true;
   }
@@ -649,9 +650,46 @@ it_status launch_gemm(it_ctx* ctx, cudaStream_t s, int M, int N, int K, const vo
   }
   const int n_tiles = ((M + T::BM - 1) / T::BM) * ((N + T::BN - 1) / T::BN);
   const int grid = std::min(n_tiles, ctx->sm_count);
-  it::gemm_bf16_sm100_kernel<LAYOUT, QKV, RS><<<grid, T::THREADS, T::SMEM_BYTES, s>>>(ma, mb, p, RS ? rs_maps : no_maps);
+  IT_CUDA(launch_dependent(it::gemm_bf16_sm100_kernel<LAYOUT, QKV, RS, BN>, grid, T::THREADS, T::SMEM_BYTES, s, ma, mb, p, RS ? rs_maps : no_maps));
   ctx->launches += 1;
   IT_CUDA(cudaGetLastError());
+  return IT_OK;
+}
+
+// Tile width: the one with the smallest (waves of tiles over the SMs) x (cost of a tile).  A 64-column tile costs 0.42 and a
+// 128-column one 0.575 of a 256-column tile (8192 x 2048 -> 6144: 282, 199 and 175 us): a stage's operands are 24, 32 and 48 KB
+// of shared-memory reads at 128 B per cycle against 128, 256 and 512 cycles of MMA.
+template <int LAYOUT, bool QKV = false, bool RS = false>
+it_status launch_gemm(it_ctx* ctx, cudaStream_t s, int M, int N, int K, const void* a, long long lda, const void* b,
+                      long long ldb, void* c, long long ldc, bool c_is_f32, const QkvEpilogue* epi = nullptr,
+                      const ScatterEpilogue* rs = nullptr) {
+  auto cost = [&](int bn, double tile) {
+    const long long tiles = static_cast<long long>((M + 127) / 128) * ((N + bn - 1) / bn);
+    return static_cast<double>((tiles + ctx->sm_count - 1) / ctx->sm_count) * tile;
+  };
+  int bn = 256;
+  if (!RS) {
+    const double c256 = cost(256, 1.0), c128 = cost(128, 0.575), c64 = cost(64, 0.42);
+    bn = c64 < c128 && c64 < c256 ? 64 : c128 < c256 ? 128 : 256;
+  }
+  if constexpr (!RS) {
+    if (bn == 64) return launch_gemm_tiles<LAYOUT, QKV, RS, 64>(ctx, s, M, N, K, a, lda, b, ldb, c, ldc, c_is_f32, epi, rs);
+    if (bn == 128) return launch_gemm_tiles<LAYOUT, QKV, RS, 128>(ctx, s, M, N, K, a, lda, b, ldb, c, ldc, c_is_f32, epi, rs);
+  }
+  return launch_gemm_tiles<LAYOUT, QKV, RS, 256>(ctx, s, M, N, K, a, lda, b, ldb, c, ldc, c_is_f32, epi, rs);
+}
+
+// A handful of tokens (gemm_skinny.cuh).  The kernel reads every token once per 16 rows of weights, so the more tokens, the
+// smaller the weights up to which it beats the tcgen05 tiles: measured over 512 -> 512 to 4096 -> 12288, at 16 tokens up to
+// 2048 -> 6144 (8.0 against 8.3 us; 4096 -> 6144: 20 against 15), at 32 up to 2048 -> 3072 (7.4 against 7.7; 2048 -> 6144: 11 against 8).
+bool use_skinny(int64_t n, int64_t K, int64_t N) {
+  return n <= 8 || (n <= 16 && K * N <= 2048LL * 6144) || (n <= 32 && K * N <= 2048LL * 3072);
+}
+
+it_status launch_skinny(it_ctx* ctx, cudaStream_t s, const it::SkinnyParams& p, const it::RopeFreqs& rf) {
+  const auto kernel = p.n <= 8 ? it::gemm_skinny_kernel<1> : p.n <= 16 ? it::gemm_skinny_kernel<2> : it::gemm_skinny_kernel<4>;
+  IT_CUDA(launch_dependent(kernel, static_cast<unsigned>((p.N + 15) / 16), 256, 0, s, p, rf));
+  ctx->launches += 1;
   return IT_OK;
 }
 
@@ -1246,6 +1284,16 @@ it_status it_linear_fwd(it_ctx* ctx, it_stream* stream, int32_t n, int32_t in_di
     return IT_OK;
   }
   IT_CUDA(cudaSetDevice(ctx->device));
+  if (use_skinny(n, in_dim, out_dim)) {
+    it::SkinnyParams p{};
+    p.x = static_cast<const __nv_bfloat16*>(x);
+    p.w = static_cast<const __nv_bfloat16*>(w);
+    p.y = static_cast<__nv_bfloat16*>(y);
+    p.n = n;
+    p.K = in_dim;
+    p.N = out_dim;
+    return launch_skinny(ctx, stream->s, p, make_rope_freqs(0, 1.f, 0, false));
+  }
   return launch_gemm<0>(ctx, stream->s, n, out_dim, in_dim, x, in_dim, w, in_dim, y, out_dim, false);
 }
 
@@ -1304,6 +1352,32 @@ it_status it_qkv_rope_fwd(it_ctx* ctx, it_stream* stream, int32_t B, int32_t S, 
   if (!aligned16(x) || !aligned16(w_qkv) || !aligned16(q_out) || !aligned16(k_out) || !aligned16(v_out))
     return fail(IT_ERR_ALIGNMENT, "tensors must be 16-byte aligned");
   IT_CUDA(cudaSetDevice(ctx->device));
+  const int out_dim = (H + 2 * Hkv) * D;
+  QkvEpilogue epi{q_out, k_out, v_out, S, H, Hkv, D, nullptr, static_cast<long long>(H) * D, static_cast<long long>(Hkv) * D};
+  if (packed) {
+    __nv_bfloat16* base = static_cast<__nv_bfloat16*>(q_out);
+    epi.k = base + static_cast<long long>(H) * D;
+    epi.v = base + (static_cast<long long>(H) + Hkv) * D;
+    epi.ld_q = epi.ld_kv = out_dim;
+  }
+  if (use_skinny(n, hidden, out_dim)) {
+    it::SkinnyParams p{};
+    p.x = static_cast<const __nv_bfloat16*>(x);
+    p.w = static_cast<const __nv_bfloat16*>(w_qkv);
+    p.n = static_cast<int>(n);
+    p.K = hidden;
+    p.N = out_dim;
+    p.q = static_cast<__nv_bfloat16*>(epi.q);
+    p.k = static_cast<__nv_bfloat16*>(epi.k);
+    p.v = static_cast<__nv_bfloat16*>(epi.v);
+    p.seq = S;
+    p.heads = H;
+    p.kv_heads = Hkv;
+    p.head_dim = D;
+    p.ld_q = epi.ld_q;
+    p.ld_kv = epi.ld_kv;
+    return launch_skinny(ctx, stream->s, p, make_rope_freqs(D, rope_base == 0.f ? 1.f : rope_base, position_offset, rope_base != 0.f));
+  }
   const float2* table = nullptr;
   if (rope_base != 0.f) {
     size_t need = 0;
@@ -1312,19 +1386,12 @@ it_status it_qkv_rope_fwd(it_ctx* ctx, it_stream* stream, int32_t B, int32_t S, 
       return fail(IT_ERR_INVALID_ARG, "workspace of %zu bytes needed, %zu given", need, workspace_bytes);
     if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return fail(IT_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
     const int cells = S * (D / 2);
-    it::rope_table_kernel<<<(cells + 255) / 256, 256, 0, stream->s>>>(static_cast<float2*>(workspace), S, D / 2,
-                                                                      make_rope_freqs(D, rope_base, position_offset, true));
+    IT_CUDA(launch_dependent(it::rope_table_kernel, (cells + 255) / 256, 256, 0, stream->s, static_cast<float2*>(workspace), S, D / 2,
+                             make_rope_freqs(D, rope_base, position_offset, true)));
     ctx->launches += 1;
     table = static_cast<const float2*>(workspace);
   }
-  const int out_dim = (H + 2 * Hkv) * D;
-  QkvEpilogue epi{q_out, k_out, v_out, S, H, Hkv, D, table, static_cast<long long>(H) * D, static_cast<long long>(Hkv) * D};
-  if (packed) {
-    __nv_bfloat16* base = static_cast<__nv_bfloat16*>(q_out);
-    epi.k = base + static_cast<long long>(H) * D;
-    epi.v = base + (static_cast<long long>(H) + Hkv) * D;
-    epi.ld_q = epi.ld_kv = out_dim;
-  }
+  epi.rope_table = table;
   return launch_gemm<0, true>(ctx, stream->s, static_cast<int>(n), out_dim, hidden, x, hidden, w_qkv, hidden, nullptr, 0,
                               false, &epi);
 }

@@ -19,6 +19,8 @@
 
 #include <cstdint>
 
+#include "sm100_ptx.cuh"
+
 namespace it {
 
 struct RopeFreqs {
@@ -78,6 +80,8 @@ __device__ __forceinline__ void rope_fill_table(float2* table, int S, int half, 
   }
 }
 __global__ void rope_table_kernel(float2* __restrict__ table, int S, int half, const __grid_constant__ RopeFreqs freqs) {
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
   rope_fill_table(table, S, half, freqs, static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x,
                   static_cast<long long>(gridDim.x) * blockDim.x);
 }

@@ -181,7 +181,7 @@ class Tensor(_host_ops.TensorBase):
     (src/tensor.rs:136-148); here it synchronises the stream and copies device -> host."""
 
     def __init__(self, data, shape, precision):
-        self._set(data.view(list(shape)))    # `data`: a torch CUDA tensor of that many elements
+        self._set(data, shape)    # `data`: a torch CUDA tensor of that many elements
 
     @property
     def _data(self):

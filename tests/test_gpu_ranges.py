@@ -116,3 +116,46 @@ def test_fp32_backward_on_the_tensor_cores(it_ctx, B, S, H, Hkv, D, causal, rope
         assert not np.isnan(g).any()
         assert np.abs(g - want).max() <= 1e-4, f"{name}: {np.abs(g - want).max():.2e}"
         assert np.linalg.norm(g - want) <= 1e-5 * np.linalg.norm(want), name
+
+
+# The skinny kernel's token groups of 8, its 16-row tiles and 32-wide K steps, and the three tile widths of the tcgen05 GEMM
+# (chosen by how many tiles the product has), each with remainders in every dimension.
+@pytest.mark.parametrize("n,k,out", [(1, 8, 8), (3, 40, 24), (8, 264, 120), (9, 2048, 200), (16, 72, 1000), (17, 520, 40), (32, 2048, 3064),
+                                     (33, 136, 200), (64, 4104, 520), (130, 264, 9480), (700, 200, 5000), (2500, 136, 3080)])
+def test_projection_of_any_number_of_tokens(it_ctx, n, k, out):
+    """linear_forward against an fp32 product of the same bf16 operands: error of the bf16 result, 2^-9 / sqrt(3) relative per
+    element plus fp32 sums (1.7e-3 in L2)."""
+    from irontensor_b200 import Tensor, linear_forward
+    x = synth.round_bf16(synth.normal(180, synth.TENSOR_Q, 0, n * k, 1.0)).reshape(n, k)
+    w = synth.round_bf16(synth.normal(181, synth.TENSOR_K, 0, out * k, k ** -0.5)).reshape(out, k)
+    y = linear_forward(Tensor.from_f32_as_bf16(x.reshape(-1), [n, k]), Tensor.from_f32_as_bf16(w.reshape(-1), [out, k]))
+    assert it_ctx.poll_status() == 0
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    got = y.to_f32_host()
+    assert np.linalg.norm(got - want) <= 2.0e-3 * np.linalg.norm(want)
+    assert np.all(np.abs(got - want) <= 2.0 ** -8 * np.abs(want) + 1e-4)
+
+
+@pytest.mark.parametrize("B,S,hidden,H,Hkv,D,base,packed", [(4, 1, 256, 4, 2, 64, 10000.0, False), (1, 20, 512, 8, 8, 128, 10000.0, True),
+                                                            (3, 5, 72, 2, 1, 96, 500.0, False), (9, 1, 128, 4, 1, 32, None, True)])
+def test_qkv_projection_of_a_few_tokens(it_ctx, B, S, hidden, H, Hkv, D, base, packed):
+    """The skinny kernel's Q/K/V epilogue (rotation evaluated in place, separate and packed outputs)."""
+    from irontensor_b200 import Tensor, qkv_rope_forward
+    n, width, pos = B * S, (H + 2 * Hkv) * D, 11
+    x = synth.round_bf16(synth.normal(190, synth.TENSOR_Q, 0, n * hidden, 1.0)).reshape(n, hidden)
+    w = synth.round_bf16(synth.normal(191, synth.TENSOR_K, 0, width * hidden, hidden ** -0.5)).reshape(width, hidden)
+    out = qkv_rope_forward(Tensor.from_f32_as_bf16(x.reshape(-1), [B, S, hidden]), Tensor.from_f32_as_bf16(w.reshape(-1), [width, hidden]),
+                           H, Hkv, D, base, pos, packed=packed)
+    assert it_ctx.poll_status() == 0
+    y = (x.astype(np.float64) @ w.astype(np.float64).T).astype(np.float32).reshape(B, S, width)
+    q, k, v = y[..., :H * D].reshape(B, S, H, D), y[..., H * D:(H + Hkv) * D].reshape(B, S, Hkv, D), y[..., (H + Hkv) * D:].reshape(B, S, Hkv, D)
+    if base is not None:
+        q, k = ol.rope(np.ascontiguousarray(q), base, pos), ol.rope(np.ascontiguousarray(k), base, pos)
+    if packed:
+        got = out.to_f32_host()
+        got = (got[..., :H * D].reshape(q.shape), got[..., H * D:(H + Hkv) * D].reshape(k.shape), got[..., (H + Hkv) * D:].reshape(v.shape))
+    else:
+        got = [t.to_f32_host() for t in out]
+    for g, want in zip(got, (q, k, v)):
+        # a bf16 rounding step of the result, and sines and products in fp32
+        assert np.all(np.abs(g - want) <= 2.0 ** -8 * np.abs(want) + 1e-4)
