@@ -32,6 +32,8 @@
 // TMEM columns (512 allocated): S buffers [0,128) [128,256), O [256,256+D), P [256+D,256+D+64) and
 // Q [256+D+64,256+D+64+D/2) as packed bf16.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "fa_fwd_sm100.cuh"   // FwdParams
 #include "sm100_ptx.cuh"
 
@@ -64,9 +66,10 @@ struct FwdPPTraits {
 // DECODE = true is the same pipeline for one new token per sequence against a key/value cache
 // (fa_decode.cuh describes the op): the rows of the query tile are the query HEADS of one K/V head's
 // group (rows past the group are zero-filled by TMA and never stored), prm.S is the number of valid
-// cache positions, a CTA takes one split of the key tiles of one (batch, K/V head) and leaves either
-// the final output (one split) or an unnormalised partial output with its reference maximum and row
-// sum for fa_decode_merge_kernel.  The cache is streamed by TMA through the same K and V rings, so
+// cache positions, a CTA takes one split of the key tiles of one (batch, K/V head).  Up to 8 splits of a
+// (batch, K/V head) are a thread-block cluster that merges its outputs through distributed shared memory;
+// more splits leave unnormalised partial outputs with their reference maxima and row sums for
+// fa_decode_merge_kernel.  The cache is streamed by TMA through the same K and V rings, so
 // the op runs at the rate the memory system delivers tiles, not at the rate CUDA cores can issue loads.
 template <int D, bool DECODE = false>
 __global__ void __launch_bounds__(384, 1)
@@ -463,6 +466,16 @@ fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
               *reinterpret_cast<uint4*>(orow + v * 8) = o4;
             }
             if (w == 0 && prm.lse != nullptr) prm.lse[slice] = (m_fin + lg2(l_tot)) * 0.6931471805599453f;
+          } else if (prm.dec_clustered) {
+            // the K ring is free (the last S is complete): rows of D + 4 floats, then (maximum, sum) per row
+            float* srow = reinterpret_cast<float*>(smem + T::SMEM_K) + row * (D + 4) + w * HC;
+#pragma unroll
+            for (int v = 0; v < HC / 4; ++v)
+              *reinterpret_cast<uint4*>(srow + v * 4) = make_uint4(r[v * 4], r[v * 4 + 1], r[v * 4 + 2], r[v * 4 + 3]);
+            if (w == 0) {
+              m_ref[row] = m_fin;
+              l_part[row] = l_tot;
+            }
           } else {
             const int sp = static_cast<int>(blockIdx.x) % prm.dec_n_splits;
             float* prow = prm.dec_part_o + (slice * prm.dec_n_splits + sp) * D + w * HC;
@@ -499,6 +512,47 @@ fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             prm.lse[static_cast<size_t>(bh) * S + q_row] = (m_fin + lg2(l_tot)) * 0.6931471805599453f;
         }
       }
+    }
+  }
+
+  if constexpr (DECODE) {
+    if (prm.dec_clustered) {
+      // Every thread of every CTA passes both cluster barriers, whatever happened to it before (a CTA that gave up leaves
+      // garbage behind, as any launch does then).  CTA `rank` finishes every n-th element of the group's rows.
+      namespace cg = cooperative_groups;
+      cg::cluster_group cluster = cg::this_cluster();
+      __syncwarp();
+      cluster.sync();
+      const int n = prm.dec_n_splits, rank = static_cast<int>(blockIdx.x) % n;
+      for (int i = rank * 384 + static_cast<int>(threadIdx.x); i < prm.kv_group * (D / 2); i += 384 * n) {
+        const int row = i / (D / 2), d = 2 * (i % (D / 2));
+        float mx = -INFINITY, ms[8], ls[8];
+        float2 a[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          ms[c] = -INFINITY;
+          if (c < n) {
+            ms[c] = *cluster.map_shared_rank(m_ref + row, c);
+            ls[c] = *cluster.map_shared_rank(l_part + row, c);
+            a[c] = *cluster.map_shared_rank(reinterpret_cast<float2*>(reinterpret_cast<float*>(smem + T::SMEM_K) + row * (D + 4) + d), c);
+          }
+          mx = fmaxf(mx, ms[c]);
+        }
+        float sum = 0.f;
+        float2 o2 = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+          if (c < n) {
+            const float f = ex2(ms[c] - mx);
+            sum = fmaf(f, ls[c], sum);
+            o2.x = fmaf(f, a[c].x, o2.x);
+            o2.y = fmaf(f, a[c].y, o2.y);
+          }
+        const float inv = 1.0f / sum;
+        *reinterpret_cast<uint32_t*>(prm.o + (static_cast<size_t>(bh) + row) * D + d) = pack_bf16(o2.x * inv, o2.y * inv);
+        if (d == 0 && prm.lse != nullptr) prm.lse[static_cast<size_t>(bh) + row] = (mx + lg2(sum)) * 0.6931471805599453f;
+      }
+      cluster.sync();   // nobody's shared memory goes away while it is read
     }
   }
 

@@ -61,6 +61,7 @@ struct FwdParams {
   // decode instantiation of the long-sequence kernel only (one new token against a key/value cache):
   int dec_tiles_per_split;   // key tiles per CTA
   int dec_n_splits;
+  int dec_clustered;         // the splits of a (batch, K/V head) are one cluster and merge in the launch
   float* dec_part_o;    // [B*H, n_splits, D] unnormalised partial outputs (n_splits > 1)
   float* dec_part_ml;   // [B*H, n_splits, 2] reference maximum (log2 domain) and row sum of each split
 };

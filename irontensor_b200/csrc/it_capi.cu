@@ -199,19 +199,27 @@ it_status check_common(it_ctx* ctx, it_stream* stream, it_dtype dtype, int32_t B
 
 // Launch with the programmatic-stream-serialization attribute: the kernel may be set up while the kernel in front of it
 // in the stream still runs, and waits in griddepcontrol.wait for that kernel's completion before it touches its results.
+// launch_cluster: in clusters of `cluster` CTAs along x (1: no clusters).
 template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+cudaError_t launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, int cluster, Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(std::forward<Args>(args))...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+  return launch_cluster(kernel, grid, block, smem, s, 1, std::forward<Args>(args)...);
 }
 
 // The tensor-core kernels take bf16 tensors whose rows TMA can address (a multiple of 8 columns = 16 bytes); rows past the
@@ -427,6 +435,7 @@ it_status launch_fwd_sm100(it_ctx* ctx, it_stream* stream, int B, int H, int S, 
   }
   p.dec_tiles_per_split = 0;
   p.dec_n_splits = 1;
+  p.dec_clustered = 0;
   p.dec_part_o = nullptr;
   p.dec_part_ml = nullptr;
   const int n_ctas_per_slice = (S + T::BM * T::QT_PER_CTA - 1) / (T::BM * T::QT_PER_CTA);
@@ -579,7 +588,7 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
   return IT_OK;
 }
 
-constexpr int kDecodeMaxSplits = 64;
+constexpr int kDecodeMaxSplits = it::DEC_MAX_SPLITS;
 
 // C[M,N] = op(A) op(B) in bf16 with fp32 accumulation.  layout 0: A [M,K], B [N,K]; 1: A [M,K], B [K,N];
 // 2: A [K,M], B [K,N].  Row-major, pitches in elements.
@@ -701,6 +710,33 @@ it_status check_linear(it_ctx* ctx, it_stream* stream, int32_t n, int32_t in_dim
   return IT_OK;
 }
 
+// How many clusters of `size` CTAs of the decode pipeline are resident at once (asked once per device and size).
+template <int D>
+int max_clusters(it_ctx* ctx, int size) {
+  static std::atomic<int> known[16][9];   // 0: not asked yet
+  std::atomic<int>& k = known[ctx->device & 15][size];
+  if (k == 0) {
+    using T = it::FwdPPTraits<D>;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(T::THREADS);
+    cfg.dynamicSmemBytes = T::SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(size);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, it::fa_fwd_pp_sm100_kernel<D, true>, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = 1;
+    }
+    k = n;
+  }
+  return k;
+}
+
 // Decode on the tensor-core pipeline (bf16, head_dim 64 or 128): the group's query heads are the rows of
 // one query tile, the cache is streamed by TMA.  See fa_fwd_pp_sm100.cuh, DECODE.
 template <int D>
@@ -710,11 +746,30 @@ it_status launch_decode_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int Hkv
   const int G = H / Hkv;
   const int n_tiles = (kv_len + T::BN - 1) / T::BN;
   const long long base_ctas = static_cast<long long>(B) * Hkv;
-  // one CTA per SM runs at a time: split the keys until the GPU is covered, but keep at least four tiles per CTA
-  long long want = (ctx->sm_count + base_ctas - 1) / base_ctas;
-  want = std::max(1LL, std::min<long long>({want, std::max(1, n_tiles / 4), kDecodeMaxSplits}));
-  const int tiles_per_split = static_cast<int>((n_tiles + want - 1) / want);
-  const int n_splits = (n_tiles + tiles_per_split - 1) / tiles_per_split;
+  auto kernel = it::fa_fwd_pp_sm100_kernel<D, true>;
+  static std::atomic<bool> attr_set[16];   // zero-initialised; setting an attribute twice is harmless
+  if (!attr_set[ctx->device & 15]) {
+    IT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES));
+    attr_set[ctx->device & 15] = true;
+  }
+  // One CTA per SM runs at a time: split the keys until the GPU is covered.  Up to 8 splits (2, 4 or 8, down to one tile each:
+  // a tile costs a CTA 0.6 us, its start and end 5) are a cluster and merge in the launch; where 8 leave SMs idle and a split
+  // still has four tiles, more splits and a merge launch (2 us).
+  const long long fill = std::max<long long>(1, ctx->sm_count / base_ctas);
+  int n_splits, tiles_per_split;
+  if (fill > 8 && n_tiles > 4 * 8) {
+    const long long want = std::min<long long>({(ctx->sm_count + base_ctas - 1) / base_ctas, n_tiles / 4, kDecodeMaxSplits});
+    tiles_per_split = static_cast<int>((n_tiles + want - 1) / want);
+  } else {
+    const long long want = std::min<long long>(fill, n_tiles);
+    int c = want >= 8 ? 8 : want >= 4 ? 4 : want >= 2 ? 2 : 1;
+    // clusters that are all resident at once: one of 8 needs 8 free SMs in one GPC, and a second wave doubles the launch
+    // (16 clusters of 8: 15.6 us for 1000 positions, 16 of 4: 9)
+    while (c > 2 && base_ctas > max_clusters<D>(ctx, c)) c /= 2;
+    tiles_per_split = (n_tiles + c - 1) / c;
+  }
+  n_splits = (n_tiles + tiles_per_split - 1) / tiles_per_split;
+  const bool clustered = n_splits > 1 && n_splits <= 8;
   CUtensorMap mq, mk, mv;
   it_status st;
   const it::TensorStrides sq{D, static_cast<long long>(G) * D, static_cast<long long>(H) * D, Hkv};
@@ -722,12 +777,6 @@ it_status launch_decode_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int Hkv
   if ((st = make_tmap(ctx, &mq, q, B, Hkv, G, D, sq, 128)) != IT_OK) return st;
   if ((st = make_tmap(ctx, &mk, kc, B, Hkv, kv_len, D, sc, 128)) != IT_OK) return st;
   if ((st = make_tmap(ctx, &mv, vc, B, Hkv, kv_len, D, sc, 128)) != IT_OK) return st;
-  auto kernel = it::fa_fwd_pp_sm100_kernel<D, true>;
-  static std::atomic<bool> attr_set[16];   // zero-initialised; setting an attribute twice is harmless
-  if (!attr_set[ctx->device & 15]) {
-    IT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES));
-    attr_set[ctx->device & 15] = true;
-  }
   it::FwdParams p;
   p.st = it::TensorStrides{D, D, static_cast<long long>(H) * D, H};
   p.o = static_cast<__nv_bfloat16*>(o);
@@ -743,11 +792,13 @@ it_status launch_decode_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int Hkv
   p.work_counter = nullptr;
   p.dec_tiles_per_split = tiles_per_split;
   p.dec_n_splits = n_splits;
+  p.dec_clustered = clustered;
   p.dec_part_o = ws;
   p.dec_part_ml = ws + static_cast<size_t>(B) * H * n_splits * D;
-  IT_CUDA(launch_dependent(kernel, static_cast<unsigned>(base_ctas * n_splits), T::THREADS, T::SMEM_BYTES, s, mq, mk, mv, p));
+  IT_CUDA(launch_cluster(kernel, static_cast<unsigned>(base_ctas * n_splits), T::THREADS, T::SMEM_BYTES, s, clustered ? n_splits : 1, mq,
+                         mk, mv, p));
   ctx->launches += 1;
-  if (n_splits > 1) {
+  if (n_splits > 1 && !clustered) {
     IT_CUDA(launch_dependent(it::fa_decode_merge_kernel<__nv_bfloat16>, static_cast<unsigned>(B * H), 128, 0, s,
                              static_cast<const float*>(p.dec_part_o), static_cast<const float*>(p.dec_part_ml),
                              static_cast<__nv_bfloat16*>(o), lse, n_splits, D));
@@ -757,47 +808,63 @@ it_status launch_decode_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int Hkv
   return IT_OK;
 }
 
+template <typename ST, int LK, int GC>
+it_status launch_decode_kernel(it_ctx* ctx, cudaStream_t s, const ST* q, const ST* kc, const ST* vc, ST* o, float* lse, float* part_o,
+                               float* part_ml, const it::DecodeParams& p, int B, int chunks) {
+  IT_CUDA(launch_cluster(it::fa_decode_kernel<ST, LK, GC>, dim3(p.n_splits, B * p.Hkv, chunks), 32 * it::DEC_WARPS, 0, s,
+                         p.clustered ? p.n_splits : 1, q, kc, vc, o, lse, part_o, part_ml, p));
+  ctx->launches += 1;
+  return IT_OK;
+}
+
 template <typename ST>
 it_status launch_decode(it_ctx* ctx, cudaStream_t s, int B, int H, int Hkv, int D, int kv_len, int max_len,
                                const void* q, const void* kc, const void* vc, void* o, float* lse, float* ws) {
   const int G = H / Hkv;
-  const int chunks = (G + it::DEC_GC - 1) / it::DEC_GC;
+  const int GC = G >= 5 ? 8 : G >= 3 ? 4 : G;     // query heads per CTA
+  const int chunks = (G + GC - 1) / GC;
   const long long base_ctas = static_cast<long long>(B) * Hkv * chunks;
-  // enough CTAs for about four per SM, no split shorter than 256 keys, at most kDecodeMaxSplits
-  long long want = (4LL * ctx->sm_count + base_ctas - 1) / base_ctas;
-  want = std::max(1LL, std::min<long long>({want, (kv_len + 255) / 256, kDecodeMaxSplits}));
-  int split_len = static_cast<int>((kv_len + want - 1) / want);
-  split_len = (split_len + it::DEC_TK - 1) / it::DEC_TK * it::DEC_TK;
-  const int n_splits = (kv_len + split_len - 1) / split_len;
+  constexpr int VN = it::DecVec<ST>::N;
+  const int LK = D <= 8 * VN ? 8 : D <= 16 * VN ? 16 : 32;
+  // Keys a CTA takes in one round of loads (8 warps x 32 / LK keys x 4 groups in flight, 2 with four or eight heads): no split is shorter
+  // than half of that.  Splits up to two CTAs per SM; up to 8 of them merge inside the launch.
+  const int round = it::DEC_WARPS * (32 / LK) * (GC >= 4 ? 2 : 4);
+  long long want = (2LL * ctx->sm_count + base_ctas - 1) / base_ctas;
+  want = std::max(1LL, std::min<long long>({want, (kv_len + round / 2 - 1) / (round / 2), kDecodeMaxSplits}));
+  if (want > it::DEC_MAX_CLUSTER && kv_len <= 8 * it::DEC_MAX_CLUSTER * round) want = it::DEC_MAX_CLUSTER;   // a merge launch costs more than 8 rounds
+  int n_splits = static_cast<int>(want);
+  if (n_splits > 1 && n_splits <= it::DEC_MAX_CLUSTER) n_splits = n_splits >= 8 ? 8 : n_splits >= 4 ? 4 : 2;   // cluster sizes
   it::DecodeParams p;
+  p.split_len = (kv_len + n_splits - 1) / n_splits;
+  n_splits = (kv_len + p.split_len - 1) / p.split_len;   // every split has a key
   p.H = H;
   p.Hkv = Hkv;
   p.D = D;
   p.kv_len = kv_len;
   p.cache_batch_stride = static_cast<long long>(max_len) * Hkv * D;
   p.n_splits = n_splits;
-  p.split_len = split_len;
+  p.clustered = n_splits > 1 && n_splits <= it::DEC_MAX_CLUSTER;
   p.scale_log2 = (1.0f / sqrtf(static_cast<float>(D))) * 1.4426950408889634f;
-  const int pad = 16 / static_cast<int>(sizeof(ST));
-  const size_t smem = static_cast<size_t>(it::DEC_GC) * D * 4 + 2ull * it::DEC_TK * (D + pad) * sizeof(ST) +
-                      static_cast<size_t>(it::DEC_GC) * it::DEC_TK * 4 + 3 * it::DEC_GC * 4;
-  static std::atomic<bool> attr_set[16];   // zero-initialised; setting an attribute twice is harmless
-  if (!attr_set[ctx->device & 15]) {
-    IT_CUDA(cudaFuncSetAttribute(it::fa_decode_split_kernel<ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024));
-    attr_set[ctx->device & 15] = true;
-  }
   float* part_o = ws;
   float* part_ml = ws + static_cast<size_t>(B) * H * n_splits * D;
-  const dim3 grid(n_splits, B * Hkv, chunks);
-  it::fa_decode_split_kernel<ST><<<grid, it::DEC_THREADS, smem, s>>>(
-      static_cast<const ST*>(q), static_cast<const ST*>(kc), static_cast<const ST*>(vc), static_cast<ST*>(o), lse, part_o,
-      part_ml, p);
-  ctx->launches += 1;
-  if (n_splits > 1) {
-    it::fa_decode_merge_kernel<ST><<<B * H, 128, 0, s>>>(part_o, part_ml, static_cast<ST*>(o), lse, n_splits, D);
+  const ST *qq = static_cast<const ST*>(q), *kk = static_cast<const ST*>(kc), *vv = static_cast<const ST*>(vc);
+  auto by_heads = [&](auto lk) -> it_status {
+    constexpr int L = decltype(lk)::value;
+    auto launch = GC == 8 ? launch_decode_kernel<ST, L, 8> : GC == 4 ? launch_decode_kernel<ST, L, 4>
+                  : GC == 2 ? launch_decode_kernel<ST, L, 2> : launch_decode_kernel<ST, L, 1>;
+    return launch(ctx, s, qq, kk, vv, static_cast<ST*>(o), lse, part_o, part_ml, p, B, chunks);
+  };
+  it_status st;
+  if (LK == 8) st = by_heads(std::integral_constant<int, 8>{});
+  else if (LK == 16) st = by_heads(std::integral_constant<int, 16>{});
+  else if constexpr (VN == 4) st = by_heads(std::integral_constant<int, 32>{});
+  else st = IT_ERR_UNSUPPORTED_SHAPE;   // not reached: 16 lanes cover 128 bf16
+  if (st != IT_OK) return st;
+  if (n_splits > 1 && !p.clustered) {
+    IT_CUDA(launch_dependent(it::fa_decode_merge_kernel<ST>, static_cast<unsigned>(B * H), 128, 0, s, static_cast<const float*>(part_o),
+                             static_cast<const float*>(part_ml), static_cast<ST*>(o), lse, n_splits, D));
     ctx->launches += 1;
   }
-  IT_CUDA(cudaGetLastError());
   return IT_OK;
 }
 
@@ -1264,7 +1331,15 @@ it_status it_attention_decode(it_ctx* ctx, it_stream* stream, it_dtype dtype, in
   if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return fail(IT_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
   IT_CUDA(cudaSetDevice(ctx->device));
   float* ws = static_cast<float*>(workspace);
-  if (dtype == IT_BF16 && (D == 64 || D == 128) && H / Hkv <= 128 && kv_len >= 256)
+  // The tensor-core pipeline reads long caches at the HBM rate whatever the group; the CUDA-core kernel starts 1 to 2 us
+  // sooner and its cost per byte grows with the group.  Measured (us, tensor / CUDA cores) at head_dim 128: B16 16 heads of one
+  // query head each, 512 positions 19.4 / 17.3, 1000: 27.2 / 28.5; groups of four, B4 with 4 K/V heads, 512 positions: 7.5 / 7.3,
+  // B8 with 8, 512: 8.7 / 9.2; head_dim 64: one query head 206 / 179 at 16000 positions, groups of four, B8 with 8, 1000: 9.9 / 8.6.
+  const int G = H / Hkv;
+  const long long bytes = 4LL * B * Hkv * kv_len * D;   // both caches, bf16
+  const bool short_cache = kv_len < 64 || (G == 1 && (D == 64 || bytes <= 100LL << 20)) ||
+                           (G <= 4 && kv_len <= (D == 64 ? 2500 : 1200) && bytes <= (D == 64 ? 16LL : 5LL) << 20);
+  if (dtype == IT_BF16 && (D == 64 || D == 128) && G <= 128 && !short_cache)
     return D == 128 ? launch_decode_sm100<128>(ctx, stream->s, B, H, Hkv, kv_len, max_len, q, k_cache, v_cache, o, lse, ws)
                     : launch_decode_sm100<64>(ctx, stream->s, B, H, Hkv, kv_len, max_len, q, k_cache, v_cache, o, lse, ws);
   return dtype == IT_F32 ? launch_decode<float>(ctx, stream->s, B, H, Hkv, D, kv_len, max_len, q, k_cache, v_cache, o, lse, ws)

@@ -159,3 +159,31 @@ def test_qkv_projection_of_a_few_tokens(it_ctx, B, S, hidden, H, Hkv, D, base, p
     for g, want in zip(got, (q, k, v)):
         # a bf16 rounding step of the result, and sines and products in fp32
         assert np.all(np.abs(g - want) <= 2.0 ** -8 * np.abs(want) + 1e-4)
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("B,H,Hkv,D,kv_len,max_len", [
+    (1, 4, 4, 64, 1, 1), (1, 1, 1, 8, 2, 5), (2, 4, 4, 64, 65, 128), (1, 8, 4, 40, 129, 129), (3, 6, 2, 96, 33, 64),   # one split
+    (1, 4, 2, 128, 300, 512), (2, 8, 2, 64, 1111, 2000), (1, 5, 1, 128, 700, 701), (1, 9, 1, 64, 150, 150),            # clusters of 2 to 8
+    (1, 4, 4, 64, 16500, 16500), (4, 16, 4, 128, 1000, 1024), (1, 32, 4, 128, 9000, 9000), (48, 8, 4, 128, 520, 600),  # merge launch, tensor cores
+])
+def test_decode_over_its_ranges(it_ctx, B, H, Hkv, D, kv_len, max_len, bf16):
+    """Splits of one, clusters merging through distributed shared memory, merge launches; every head grouping.  Bounds: fp32
+    sums of up to 16500 terms (1e-6 relative each way, 1e-5 in L2); bf16 the output's rounding and P's (2.5e-3, as O elsewhere)."""
+    from irontensor_b200 import Tensor, attention_decode
+    f = synth.round_bf16 if bf16 else (lambda a: a)
+    q = f(synth.normal(200 + kv_len, synth.TENSOR_Q, 0, B * H * D)).reshape(B, H, D)
+    k = f(synth.normal(200 + kv_len, synth.TENSOR_K, 0, B * max_len * Hkv * D)).reshape(B, max_len, Hkv, D)
+    v = f(synth.normal(200 + kv_len, synth.TENSOR_V, 0, B * max_len * Hkv * D)).reshape(B, max_len, Hkv, D)
+    mk = Tensor.from_f32_as_bf16 if bf16 else Tensor.from_f32_slice
+    o = attention_decode(*(mk(t.reshape(-1), list(t.shape)) for t in (q, k, v)), kv_len)
+    assert it_ctx.poll_status() == 0
+    kk, vv = (t[:, :kv_len].astype(np.float64).repeat(H // Hkv, axis=2) for t in (k, v))
+    s = np.einsum("bhd,blhd->bhl", q.astype(np.float64), kk) / math.sqrt(D)
+    mx = s.max(-1, keepdims=True)
+    p = np.exp(s - mx)
+    want = np.einsum("bhl,blhd->bhd", p, vv) / p.sum(-1)[..., None]
+    lse = (mx[..., 0] + np.log(p.sum(-1)))
+    got = o.to_f32_host()
+    assert np.abs(o.lse.to_f32_host() - lse).max() <= 1e-4
+    assert np.linalg.norm(got - want) <= (2.5e-3 if bf16 else 1e-5) * np.linalg.norm(want)
