@@ -8,7 +8,8 @@
 //   dQ CTA (one 128-row query tile)      : stationary X0 = Q, X1 = dO;  streamed Y0 = K, Y1 = V
 //   dK/dV CTA (one 128-row key tile)     : stationary X0 = K, X1 = V;   streamed Y0 = Q, Y1 = dO
 // With T0 = X0 Y0^T (the scores, or their transpose) and T1 = X1 Y1^T (dP, or its transpose) both kinds do the same:
-//   P = 2^(T0 c - LSE log2e),  dS = P o (T1 - delta),  acc0 += dS Y0  (dQ, or dK),  acc1 += P Y1  (dV; dK/dV CTA only).
+//   P = 2^(T0 c - LSE log2e),  dS = P o (T1 - delta),  acc0 = dS Y0  (dQ, or dK),  acc1 = P Y1  (dV; dK/dV CTA only).
+// The accumulators are those of one tile; the math warps add them up in the output rows (see `drain`).
 // The scores are computed twice, seven contractions in place of five; in exchange dS is only ever an A operand in the
 // orientation it is produced in, so it goes registers -> tensor memory -> MMA and never through shared memory (which the
 // twelve operand planes fill), and dQ needs neither an fp32 accumulator in memory nor its clearing and read-back.
@@ -39,7 +40,7 @@ struct BwdF32Traits {
   static constexpr int SMEM_X1 = SMEM_X0 + 3 * PLANE_BYTES;
   static constexpr int SMEM_Y0 = SMEM_X1 + 3 * PLANE_BYTES;
   static constexpr int SMEM_Y1 = SMEM_Y0 + 3 * PLANE_BYTES;
-  static constexpr int SMEM_ROW = SMEM_Y1 + 3 * PLANE_BYTES;   // [2 tiles][128] LSE*log2e, [2 tiles][128] delta of the streamed rows
+  static constexpr int SMEM_ROW = SMEM_Y1 + 3 * PLANE_BYTES;   // [2 tiles][128] -LSE*log2e, [2 tiles][128] -delta of the streamed rows
   static constexpr int SMEM_BAR = SMEM_ROW + 4 * 512;
   static constexpr int NUM_BARS = 11;
   static constexpr int SMEM_MISC = SMEM_BAR + NUM_BARS * 8;
@@ -173,18 +174,18 @@ __device__ __forceinline__ void fa_bwd_f32_body(const BwdF32Params& prm, uint8_t
     // let go of Y1's planes, then fetch Y0(n+1) under acc0(n) and store it behind it.
     const int t = threadIdx.x - 256;
     float4 r[16];
-    float lse2 = INFINITY, dl = 0.f;
+    float lse2 = -INFINITY, dl = 0.f;   // negated, as the packed operations of the math warps want them
     auto y0_of = [&](int n) { return (KV ? prm.q + prm.st.slice(bh0 + n / per_head) : prm.k + prm.st_kv.slice(bh0)); };
     auto y1_of = [&](int n) { return (KV ? prm.d_o + prm.st.slice(bh0 + n / per_head) : prm.v + prm.st_kv.slice(bh0)); };
     auto tile_of = [&](int n) { return j_lo + n % per_head; };
     auto fetch_rows = [&](int n) {   // LSE and delta of streamed row t; rows past S never contribute (P = 2^-inf)
       const int s = tile_of(n) * T::BM + t;
-      lse2 = INFINITY;
+      lse2 = -INFINITY;
       dl = 0.f;
       if (s < S) {
         const size_t i = static_cast<size_t>(bh0 + n / per_head) * S + s;
-        lse2 = prm.lse[i] * 1.4426950408889634f;
-        dl = prm.delta[i];
+        lse2 = prm.lse[i] * -1.4426950408889634f;
+        dl = -prm.delta[i];
       }
     };
     auto store_rows = [&](int n) {   // two buffers: read by the math groups of tile n, rewritten for n + 2
@@ -242,14 +243,14 @@ __device__ __forceinline__ void fa_bwd_f32_body(const BwdF32Params& prm, uint8_t
               umma_ss(tmem_base + col, sdesc_advance(da, kk * 32), sdesc_advance(db, kk * 32), IDESC_T, (term > 0 || kk > 0) ? 1u : 0u);
         }
       };
-      auto issue_acc = [&](uint32_t t_col, uint32_t e_col, uint32_t ya, uint32_t acc, bool first) {   // acc += (P or dS) Y
+      auto issue_acc = [&](uint32_t t_col, uint32_t e_col, uint32_t ya, uint32_t acc) {   // acc = (P or dS) Y
 #pragma unroll
         for (int term = 0; term < 6; ++term) {
           const uint64_t db = make_sdesc(ya + TB[term] * T::PLANE_BYTES, T::PLANE_BYTES, 1024);
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {   // 16 columns of the streamed tile each: math group kk >> 2
             const uint32_t a = (TA[term] == 2 ? e_col + (kk >> 2) * 32 : t_col + (kk >> 2) * 64 + TA[term] * 32) + (kk & 3) * 8;
-            umma_ts(tmem_base + acc, tmem_base + a, sdesc_advance(db, kk * 2048), IDESC_ACC, (!first || term > 0 || kk > 0) ? 1u : 0u);
+            umma_ts(tmem_base + acc, tmem_base + a, sdesc_advance(db, kk * 2048), IDESC_ACC, (term > 0 || kk > 0) ? 1u : 0u);
           }
         }
       };
@@ -272,13 +273,13 @@ __device__ __forceinline__ void fa_bwd_f32_body(const BwdF32Params& prm, uint8_t
         if (!ok) break;
         if (KV) {
           tc_fence_after();
-          issue_acc(T::COL_T0, T::COL_E0, y1_a, T::COL_ACC1, n == 0);
+          issue_acc(T::COL_T0, T::COL_E0, y1_a, T::COL_ACC1);
           umma_commit(y1_free);
         }
         ok = mbar_wait(ds_full, par, abort_flag, prm.status, DEV_ERR_TIMEOUT_SOFTMAX);
         if (!ok) break;
         tc_fence_after();
-        issue_acc(T::COL_T1, T::COL_E1, y0_a, T::COL_ACC0, n == 0);
+        issue_acc(T::COL_T1, T::COL_E1, y0_a, T::COL_ACC0);
         umma_commit(y0_free);
       }
     }
@@ -296,10 +297,10 @@ __device__ __forceinline__ void fa_bwd_f32_body(const BwdF32Params& prm, uint8_t
       f32_tile_store(smem + (g ? T::SMEM_X1 : T::SMEM_X0), threadIdx.x & 127, x);
       mbar_arrive(g ? x1_full : x0_full);
     }
-    float row_lse2 = INFINITY, row_dl = 0.f;    // dQ: this thread's query row
+    float row_lse2 = -INFINITY, row_dl = 0.f;    // dQ: this thread's query row, negated
     if (!KV && x_idx < S) {
-      row_lse2 = prm.lse[static_cast<size_t>(bh0) * S + x_idx] * 1.4426950408889634f;
-      row_dl = prm.delta[static_cast<size_t>(bh0) * S + x_idx];
+      row_lse2 = prm.lse[static_cast<size_t>(bh0) * S + x_idx] * -1.4426950408889634f;
+      row_dl = -prm.delta[static_cast<size_t>(bh0) * S + x_idx];
     }
     bool ok = true;
     uint32_t p[64];   // this thread's T0, then P, then dS (fp32 bits)
@@ -317,7 +318,53 @@ __device__ __forceinline__ void fa_bwd_f32_body(const BwdF32Params& prm, uint8_t
       }
       tmem_wait_st();
     };
+    // The tile's accumulators into the output rows (group 0 its row of dK, group 1 of dV; dQ: a half of the row each), which
+    // hold the sum of the tiles before; with the last tile's go scale and rotation.  The tensor core truncates when it adds
+    // into fp32, so a sum left in tensor memory over all tiles drifts with their number: dK of 1024 rows was 7.0e-6 off 64
+    // bits (the CUDA-core kernel 1.3e-6); added up here, rounding to nearest, it is 0.8e-6 at any length.  Runs while Y0 is
+    // replaced and the next T0 computed.
+    auto drain = [&](int n, bool last) -> bool {
+      constexpr int NC = KV ? 2 : 1;
+      float* out = KV ? (g ? prm.dv : prm.dk) + prm.st_kv.slice(bh0) + static_cast<long long>(x_idx) * prm.st_kv.row
+                      : prm.dq + prm.st.slice(bh0) + static_cast<long long>(x_idx) * prm.st.row + g * 32;
+      const int width = KV ? D : D - g * 32;   // columns of this thread's part (may be <= 0)
+      float4 prev[NC * 8];
+#pragma unroll
+      for (int i = 0; i < NC * 8; ++i) {
+        prev[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (n > 0 && x_idx < S && 4 * i < width) prev[i] = reinterpret_cast<const float4*>(out)[i];
+      }
+      bool got = mbar_wait(y0_free, n & 1, abort_flag, prm.status, DEV_ERR_TIMEOUT_MMA);   // the tile's MMAs are complete
+      got = __all_sync(0xffffffffu, got);
+      if (!got) return false;
+      tc_fence_after();
+      const float f = !last || (KV && g) ? 1.0f : prm.scale;
+      const bool rotate = last && prm.rope_table != nullptr && !(KV && g);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        uint32_t a[32];
+        tmem_ld_x32(t_lane + ((KV && g) ? T::COL_ACC1 : T::COL_ACC0) + (KV ? c * 32 : g * 32), a);
+        tmem_wait_ld();
+        if (x_idx < S) {
+          const float2* tab = prm.rope_table + static_cast<size_t>(x_idx) * (D >> 1) + (KV ? c * 16 : g * 16);
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            if (c * 32 + i >= width) break;
+            const float4 pv = prev[c * 8 + (i >> 2)];
+            float4 w = make_float4((__uint_as_float(a[i]) + pv.x) * f, (__uint_as_float(a[i + 1]) + pv.y) * f,
+                                   (__uint_as_float(a[i + 2]) + pv.z) * f, (__uint_as_float(a[i + 3]) + pv.w) * f);
+            if (rotate) {
+              const float4 cs = *reinterpret_cast<const float4*>(tab + (i >> 1));   // (cos, sin) of two pairs
+              w = make_float4(w.x * cs.x + w.y * cs.y, w.y * cs.x - w.x * cs.y, w.z * cs.z + w.w * cs.w, w.w * cs.z - w.z * cs.w);
+            }
+            *reinterpret_cast<float4*>(out + c * 32 + i) = w;
+          }
+        }
+      }
+      return true;
+    };
     for (int n = 0; n < n_iter; ++n) {
+      if (n > 0 && !(ok = drain(n - 1, false))) break;
       const uint32_t par = n & 1;
       const int jt = j_lo + n % per_head;
       const float* rows = reinterpret_cast<const float*>(smem + T::SMEM_ROW) + (n & 1) * 128 + g * 64;
@@ -335,10 +382,12 @@ __device__ __forceinline__ void fa_bwd_f32_body(const BwdF32Params& prm, uint8_t
       for (int i = 0; i < 64; i += 4) {
         float4 l4 = make_float4(row_lse2, row_lse2, row_lse2, row_lse2);
         if (KV) l4 = *reinterpret_cast<const float4*>(rows + i);
-        p[i + 0] = __float_as_uint(ex2(fmaf(__uint_as_float(p[i + 0]), sl2, -l4.x)));
-        p[i + 1] = __float_as_uint(ex2(fmaf(__uint_as_float(p[i + 1]), sl2, -l4.y)));
-        p[i + 2] = __float_as_uint(ex2(fmaf(__uint_as_float(p[i + 2]), sl2, -l4.z)));
-        p[i + 3] = __float_as_uint(ex2(fmaf(__uint_as_float(p[i + 3]), sl2, -l4.w)));
+        const float2 x01 = fma2(bits2(p[i + 0], p[i + 1]), make_float2(sl2, sl2), make_float2(l4.x, l4.y));
+        const float2 x23 = fma2(bits2(p[i + 2], p[i + 3]), make_float2(sl2, sl2), make_float2(l4.z, l4.w));
+        p[i + 0] = __float_as_uint(ex2(x01.x));
+        p[i + 1] = __float_as_uint(ex2(x01.y));
+        p[i + 2] = __float_as_uint(ex2(x23.x));
+        p[i + 3] = __float_as_uint(ex2(x23.y));
       }
       if (prm.causal && jt == tile) {   // the diagonal tile: keys after the query are masked
 #pragma unroll
@@ -366,50 +415,20 @@ __device__ __forceinline__ void fa_bwd_f32_body(const BwdF32Params& prm, uint8_t
         for (int i = 0; i < 32; i += 4) {
           float4 d4 = make_float4(row_dl, row_dl, row_dl, row_dl);
           if (KV) d4 = *reinterpret_cast<const float4*>(rows + 256 + c * 32 + i);
-          const float dd[4] = {d4.x, d4.y, d4.z, d4.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            p[c * 32 + i + e] = __float_as_uint(__uint_as_float(p[c * 32 + i + e]) * (__uint_as_float(d[i + e]) - dd[e]));
+          uint32_t* pp = &p[c * 32 + i];
+          const float2 s01 = mul2(bits2(pp[0], pp[1]), add2(bits2(d[i + 0], d[i + 1]), make_float2(d4.x, d4.y)));
+          const float2 s23 = mul2(bits2(pp[2], pp[3]), add2(bits2(d[i + 2], d[i + 3]), make_float2(d4.z, d4.w)));
+          pp[0] = __float_as_uint(s01.x);
+          pp[1] = __float_as_uint(s01.y);
+          pp[2] = __float_as_uint(s23.x);
+          pp[3] = __float_as_uint(s23.y);
         }
       }
       put_planes(T::COL_T1, T::COL_E1);
       tc_fence_before();
       mbar_arrive(ds_full);
     }
-    if (ok) {
-      ok = mbar_wait(y0_free, (n_iter - 1) & 1, abort_flag, prm.status, DEV_ERR_TIMEOUT_MMA);   // the last acc0 is complete
-      ok = __all_sync(0xffffffffu, ok);
-    }
-    if (ok) {
-      // dK/dV: group 0 writes its row of dK, group 1 of dV; dQ: a half of the row each
-      tc_fence_after();
-      const int n_c = KV ? 2 : 1;
-      float* out = KV ? (g ? prm.dv : prm.dk) + prm.st_kv.slice(bh0) + static_cast<long long>(x_idx) * prm.st_kv.row
-                      : prm.dq + prm.st.slice(bh0) + static_cast<long long>(x_idx) * prm.st.row;
-      const float f = (KV && g) ? 1.0f : prm.scale;
-      const bool rotate = prm.rope_table != nullptr && !(KV && g);
-#pragma unroll 1
-      for (int c = 0; c < n_c; ++c) {
-        const int d0 = KV ? c * 32 : g * 32;
-        uint32_t a[32];
-        tmem_ld_x32(t_lane + ((KV && g) ? T::COL_ACC1 : T::COL_ACC0) + d0, a);
-        tmem_wait_ld();
-        if (x_idx < S) {
-          const float2* tab = prm.rope_table + static_cast<size_t>(x_idx) * (D >> 1) + (d0 >> 1);
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            if (d0 + i >= D) break;
-            float4 w = make_float4(__uint_as_float(a[i]) * f, __uint_as_float(a[i + 1]) * f, __uint_as_float(a[i + 2]) * f,
-                                   __uint_as_float(a[i + 3]) * f);
-            if (rotate) {
-              const float4 cs = *reinterpret_cast<const float4*>(tab + (i >> 1));   // (cos, sin) of two pairs
-              w = make_float4(w.x * cs.x + w.y * cs.y, w.y * cs.x - w.x * cs.y, w.z * cs.z + w.w * cs.w, w.w * cs.z - w.z * cs.w);
-            }
-            *reinterpret_cast<float4*>(out + d0 + i) = w;
-          }
-        }
-      }
-    }
+    if (ok) drain(n_iter - 1, true);
   }
 }
 

@@ -57,12 +57,12 @@ struct FwdF32Params {
 // The three bf16 terms of two fp32 values, each packed (first value in the low half).
 __device__ __forceinline__ void split3_bf16x2(float a, float b, uint32_t* hi, uint32_t* mid, uint32_t* lo) {
   const uint32_t h = ptx::pack_bf16(a, b);
-  const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xFFFF0000u);
-  const uint32_t m = ptx::pack_bf16(ra, rb);
-  const float sa = ra - __uint_as_float(m << 16), sb = rb - __uint_as_float(m & 0xFFFF0000u);
+  const float2 r = ptx::fma2(ptx::bits2(h << 16, h & 0xFFFF0000u), make_float2(-1.f, -1.f), make_float2(a, b));
+  const uint32_t m = ptx::pack_bf16(r.x, r.y);
+  const float2 s = ptx::fma2(ptx::bits2(m << 16, m & 0xFFFF0000u), make_float2(-1.f, -1.f), r);
   *hi = h;
   *mid = m;
-  *lo = ptx::pack_bf16(sa, sb);
+  *lo = ptx::pack_bf16(s.x, s.y);
 }
 
 __global__ void __launch_bounds__(288, 1) fa_fwd_f32_sm100_kernel(const FwdF32Params prm) {
@@ -293,8 +293,8 @@ __global__ void __launch_bounds__(288, 1) fa_fwd_f32_sm100_kernel(const FwdF32Pa
         tmem_wait_ld();
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          float p0 = ex2(fmaf(__uint_as_float(r[i]), sl2, neg_m));
-          float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), sl2, neg_m));
+          const float2 x = fma2(bits2(r[i], r[i + 1]), make_float2(sl2, sl2), make_float2(neg_m, neg_m));
+          float p0 = ex2(x.x), p1 = ex2(x.y);
           if (c * 32 + i > vis) p0 = 0.f;
           if (c * 32 + i + 1 > vis) p1 = 0.f;
           l0 += p0;

@@ -187,3 +187,24 @@ def test_decode_over_its_ranges(it_ctx, B, H, Hkv, D, kv_len, max_len, bf16):
     got = o.to_f32_host()
     assert np.abs(o.lse.to_f32_host() - lse).max() <= 1e-4
     assert np.linalg.norm(got - want) <= (2.5e-3 if bf16 else 1e-5) * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("S,D", [(640, 64), (1024, 64), (777, 32)])
+def test_fp32_backward_keeps_its_precision_over_many_tiles(it_ctx, S, D):
+    """Gradients of long sequences against 64 bits.  fp32 sums of S terms, rounded to nearest, are off by about
+    sqrt(S) * 2^-25 relative to the terms (1e-6 at 1024), the operands' 24 bits by less: 2e-6.  (Sums that stay in tensor memory
+    over all tiles are truncated at every addition and drift to 7e-6.)"""
+    import torch
+    q, k, v, d_o = [torch.from_numpy(t.reshape(1, 2, S, D)).cuda() for t in synth.attention_inputs(960 + S, 1, 2, S, D)]
+    from irontensor_b200 import Tensor, attention_backward_recompute, flash_attention
+    from irontensor_b200 import Precision
+    tq, tk, tv, tdo = (Tensor(t.reshape(-1), [1, 2, S, D], Precision.FP32) for t in (q, k, v, d_o))
+    o = flash_attention(tq, tk, tv, True)
+    got = attention_backward_recompute(tdo, tq, tk, tv, o, o.lse)
+    q, k, v, d_o = (t.double() for t in (q, k, v, d_o))
+    s = (q @ k.mT / math.sqrt(D)).masked_fill(~torch.ones(S, S, dtype=torch.bool, device="cuda").tril(), -math.inf)
+    p = torch.softmax(s, -1)
+    ds = p * (d_o @ v.mT - (d_o * (p @ v)).sum(-1, keepdim=True))
+    want = (ds @ k / math.sqrt(D), ds.mT @ q / math.sqrt(D), p.mT @ d_o)
+    for g, w, name in zip(got, want, ("dQ", "dK", "dV")):
+        assert (g.torch().reshape(w.shape).double() - w).norm() <= 2e-6 * w.norm(), name
