@@ -16,6 +16,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <new>
@@ -171,11 +172,11 @@ bool as_bool(PyObject* o, int32_t* v) {
     return nullptr;                                                                                   \
   }
 template <typename F>
-PyObject* guard(F&& f) {   // C++ exceptions (out of memory, mostly) as Python's
+PyObject* guard(F&& f) {   // C++ exceptions as Python's
   try {
     return f();
-  } catch (const std::exception& e) {
-    if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
+  } catch (...) {   // as torch's own functions report them: torch.OutOfMemoryError from the allocator, RuntimeError, ...
+    if (!PyErr_Occurred()) torch::translate_exception_to_python(std::current_exception());
     return nullptr;
   }
 }

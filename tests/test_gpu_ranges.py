@@ -208,3 +208,20 @@ def test_fp32_backward_keeps_its_precision_over_many_tiles(it_ctx, S, D):
     want = (ds @ k / math.sqrt(D), ds.mT @ q / math.sqrt(D), p.mT @ d_o)
     for g, w, name in zip(got, want, ("dQ", "dK", "dV")):
         assert (g.torch().reshape(w.shape).double() - w).norm() <= 2e-6 * w.norm(), name
+
+
+def test_out_of_memory_keeps_its_type(it_ctx):
+    """An allocation that cannot succeed raises what torch raises for it, and the context stays usable."""
+    import torch
+    from irontensor_b200 import Precision, Tensor, flash_attention
+    t = Tensor(torch.zeros(8 * 4 * 64 * 64, device="cuda"), [8, 4, 64, 64], Precision.FP32)
+    keep = []
+    torch.cuda.empty_cache()
+    torch.cuda.memory.set_per_process_memory_fraction(1e-9)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            for _ in range(1000):   # until the allocator's cached blocks are used up
+                keep.append(flash_attention(t, t, t, True))
+    finally:
+        torch.cuda.memory.set_per_process_memory_fraction(1.0)
+    assert np.isfinite(flash_attention(t, t, t, True).to_f32_host()).all()
