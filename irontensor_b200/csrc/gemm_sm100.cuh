@@ -8,7 +8,8 @@
 //   LAYOUT 0 (NT): A [M,K], B [N,K]   -> both K-major           y  = x W^T
 //   LAYOUT 1 (NN): A [M,K], B [K,N]   -> A K-major, B N-major   dx = dy W
 //   LAYOUT 2 (TN): A [K,M], B [K,N]   -> A M-major, B N-major   dW = dy^T x
-// Persistent kernel, one CTA per SM, tiles of 128 x 256 (or 128, or 64 columns, where those fill the GPU better) handed out round-robin in an order that keeps the
+// Persistent kernel, one CTA per SM, tiles of 128 x 256 (or 128, or 64 columns, where those fill the GPU better; or of 256 x 256
+// on pairs of CTAs) handed out round-robin in an order that keeps the
 // tiles of the CTAs running at one time close together (gemm_tile_coords):
 //   warp 0     : TMA producer, a ring of four (six, eight) stages of (A 128x64, B 256x64) blocks, 128-byte swizzle
 //   warp 1     : MMA issuer, tcgen05.mma 128x256x16, two accumulators of 256 TMEM columns each so that the
@@ -23,11 +24,14 @@
 
 namespace it {
 
-template <int BN_ = 256>
+// CG: CTAs per tile (2: a pair of CTAs, one tile of 256 rows).
+template <int BN_ = 256, int CG = 1>
 struct GemmTraits {
-  static constexpr int BM = 128, BN = BN_, BK = 64, STAGES = BN == 256 ? 4 : BN == 128 ? 6 : 8;
-  static constexpr int A_BYTES = BM * BK * 2;      // 16 KB
-  static constexpr int B_BYTES = BN * BK * 2;      // 32 KB
+  static constexpr int BM = 128, BN = BN_, BK = 64;   // rows per CTA, columns per tile
+  static constexpr int B_ROWS = BN / CG;              // columns of C whose B a CTA loads
+  static constexpr int STAGES = B_ROWS == 256 ? 4 : B_ROWS == 128 ? 6 : 8;
+  static constexpr int A_BYTES = BM * BK * 2;         // 16 KB
+  static constexpr int B_BYTES = B_ROWS * BK * 2;     // 32, 16 or 8 KB
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int OUT_BYTES = BM * 128;       // reduce-scatter epilogue: staging of 128 rows x 64 bf16 columns, two of them
   static constexpr int SMEM_OUT = STAGES * STAGE_BYTES;
@@ -91,11 +95,18 @@ __device__ __forceinline__ void gemm_tile_coords(int tile, int tiles_m, int tile
 // tile to bf16 into a swizzled staging buffer, and one thread (warp 3) adds it into the copy of C of the rank that
 // owns those rows with a TMA reduce-add -- whole 128-byte lines, over NVLink when the owner is a peer -- while the
 // tensor core is already on the next tile.
-template <int LAYOUT, bool QKV = false, bool RS = false, int BN = 256>
+// CG = 2: a cluster of two CTAs (one TPC) works on one tile of 256 x 256.  Each CTA loads its 128 rows of A and half of the
+// tile's B, and the even CTA's MMA thread issues 256x256x16 MMAs that read both CTAs' shared memory and accumulate each
+// CTA's rows in its own TMEM.  Per 64 columns of K an SM then moves 32 KB into and 32 KB out of shared memory, 512 cycles at
+// 128 B per cycle, which is what the MMAs take; a 128 x 256 tile of one CTA moves 48 + 48 KB, 768 cycles.  All loads signal
+// the even CTA's `full` barrier; `empty` and `acc_full` are committed to both CTAs.  8192 x 2048 -> 6144: 159 -> 136 us
+// (1.30 -> 1.52 PFLOP/s).
+template <int LAYOUT, bool QKV = false, bool RS = false, int BN = 256, int CG = 1>
 __global__ void __launch_bounds__(256, 1)
 gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                        const GemmParams prm, const __grid_constant__ GemmScatterMaps rs_maps) {
-  using T = GemmTraits<BN>;
+  using T = GemmTraits<BN, CG>;
+  static_assert(CG == 1 || !RS, "the reduce-scatter epilogue runs on tiles of one CTA");
   using namespace ptx;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + T::SMEM_BAR);
@@ -109,7 +120,9 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + T::SMEM_MISC + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (prm.M + T::BM - 1) / T::BM, tiles_n = (prm.N + T::BN - 1) / T::BN;
+  const int rank = CG == 2 ? static_cast<int>(blockIdx.x) & 1 : 0;   // in the pair
+  const int first_tile = static_cast<int>(blockIdx.x) / CG, tile_step = static_cast<int>(gridDim.x) / CG;
+  const int tiles_m = (prm.M + CG * T::BM - 1) / (CG * T::BM), tiles_n = (prm.N + T::BN - 1) / T::BN;
   const int n_tiles = tiles_m * tiles_n;
   const int n_kb = (prm.K + T::BK - 1) / T::BK;
 
@@ -126,7 +139,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&acc_full[i], 1);
-      mbar_init(&acc_empty[i], 128);
+      mbar_init(&acc_empty[i], CG == 2 ? 8 : 128);   // a pair: one arrival per epilogue warp of both CTAs
       mbar_init(&out_full[i], 128);
       mbar_init(&out_free[i], 1);
     }
@@ -134,11 +147,17 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     fence_proxy_async_smem();
   }
   if (warp == 2) {
-    tmem_alloc(tmem_slot, T::TMEM_COLS);
-    tmem_relinquish();
+    if (CG == 2) {
+      tmem_alloc_2cta(tmem_slot, T::TMEM_COLS);
+      tmem_relinquish_2cta();
+    } else {
+      tmem_alloc(tmem_slot, T::TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (CG == 2) cluster_sync_all();   // both CTAs' barriers are initialised and both have their tensor memory
   tc_fence_after();
   grid_dep_wait();     // operands may be what the kernel in front wrote, and the output what it still reads
   grid_dep_launch();
@@ -152,10 +171,10 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       prefetch_tensormap(&tmap_a);
       prefetch_tensormap(&tmap_b);
       int it = 0;   // stage use counter
-      for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+      for (int tile = first_tile; tile < n_tiles; tile += tile_step) {
         int tm, tn;
         gemm_tile_coords(tile, tiles_m, tiles_n, &tm, &tn);
-        const int m0 = tm * T::BM, n0 = tn * T::BN;
+        const int m0 = (tm * CG + rank) * T::BM, n0 = tn * T::BN + rank * T::B_ROWS;
         bool ok = true;
         for (int kb = 0; kb < n_kb; ++kb, ++it) {
           const int st = it % T::STAGES;
@@ -164,8 +183,26 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           if (!ok) break;
           uint8_t* sa = smem + st * T::STAGE_BYTES;
           uint8_t* sb = sa + T::A_BYTES;
-          mbar_arrive_expect_tx(&full[st], T::STAGE_BYTES);
           const int k0 = kb * T::BK;
+          if (CG == 2) {
+            // the even CTA expects both CTAs' bytes (the other's may land first: the phase still lacks this arrival)
+            if (rank == 0) mbar_arrive_expect_tx(&full[st], 2 * T::STAGE_BYTES);
+            const uint32_t bar = cluster_addr(&full[st], 0);
+            if (LAYOUT == 2) {
+              tma_load_4d_2cta(sa, &tmap_a, bar, m0, k0, 0, 0);
+              tma_load_4d_2cta(sa + T::A_BYTES / 2, &tmap_a, bar, m0 + 64, k0, 0, 0);
+            } else {
+              tma_load_4d_2cta(sa, &tmap_a, bar, k0, m0, 0, 0);
+            }
+            if (LAYOUT == 0) {
+              tma_load_4d_2cta(sb, &tmap_b, bar, k0, n0, 0, 0);
+            } else {
+#pragma unroll
+              for (int b = 0; b < T::B_ROWS / 64; ++b) tma_load_4d_2cta(sb + b * (64 * T::BK * 2), &tmap_b, bar, n0 + b * 64, k0, 0, 0);
+            }
+            continue;
+          }
+          mbar_arrive_expect_tx(&full[st], T::STAGE_BYTES);
           if (LAYOUT == 2) {   // A [K,M]: 64 K-rows of M, two 64-wide M blocks
             tma_load_4d(sa, &tmap_a, &full[st], m0, k0, 0, 0);
             tma_load_4d(sa + T::A_BYTES / 2, &tmap_a, &full[st], m0 + 64, k0, 0, 0);
@@ -183,11 +220,11 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       }
     }
   } else if (warp == 1) {
-    if (elect_one()) {
-      constexpr uint32_t IDESC = make_idesc(T::BM, T::BN, LAYOUT == 2, LAYOUT != 0);
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t IDESC = make_idesc(CG * T::BM, T::BN, LAYOUT == 2, LAYOUT != 0);
       int it = 0, t = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++t) {
+      for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step, ++t) {
         const int buf = t & 1;
         ok = mbar_wait(&acc_empty[buf], ((t >> 1) & 1) ^ 1, abort_flag, prm.status, DEV_ERR_TIMEOUT_SOFTMAX);
         if (!ok) break;
@@ -203,12 +240,25 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           const uint64_t da = (LAYOUT == 2) ? make_sdesc(a_addr, T::A_BYTES / 2, 1024) : make_sdesc(a_addr, 16, 1024);
           const uint64_t db = (LAYOUT == 0) ? make_sdesc(b_addr, 16, 1024) : make_sdesc(b_addr, 64 * T::BK * 2, 1024);
 #pragma unroll
-          for (int kk = 0; kk < T::BK / 16; ++kk)
-            umma_ss(tmem_base + buf * T::BN, sdesc_advance(da, (LAYOUT == 2) ? kk * 2048 : kk * 32),
-                    sdesc_advance(db, (LAYOUT == 0) ? kk * 32 : kk * 2048), IDESC, (kb > 0 || kk > 0) ? 1u : 0u);
-          umma_commit(&empty[st]);
+          for (int kk = 0; kk < T::BK / 16; ++kk) {
+            const uint64_t dak = sdesc_advance(da, (LAYOUT == 2) ? kk * 2048 : kk * 32);
+            const uint64_t dbk = sdesc_advance(db, (LAYOUT == 0) ? kk * 32 : kk * 2048);
+            if (CG == 2)
+              umma_ss_2cta(tmem_base + buf * T::BN, dak, dbk, IDESC, (kb > 0 || kk > 0) ? 1u : 0u);
+            else
+              umma_ss(tmem_base + buf * T::BN, dak, dbk, IDESC, (kb > 0 || kk > 0) ? 1u : 0u);
+          }
+          if (CG == 2)
+            umma_commit_2cta(&empty[st]);
+          else
+            umma_commit(&empty[st]);
         }
-        if (ok) umma_commit(&acc_full[buf]);
+        if (ok) {
+          if (CG == 2)
+            umma_commit_2cta(&acc_full[buf]);
+          else
+            umma_commit(&acc_full[buf]);
+        }
       }
     }
   } else if (warp == 3) {
@@ -216,7 +266,7 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       // reduce-add issuer: pieces in the order the epilogue produces them
       int g = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+      for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step) {
         int tm, tn;
         gemm_tile_coords(tile, tiles_m, tiles_n, &tm, &tn);
         const int m0 = tm * T::BM, n0 = tn * T::BN;
@@ -244,11 +294,11 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     int rs_g = 0;   // staged pieces so far (reduce-scatter epilogue)
     bool ok = true;
     uint32_t r[32];
-    for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++t) {
+    for (int tile = first_tile; tile < n_tiles && ok; tile += tile_step, ++t) {
       const int buf = t & 1;
       int tm, tn;
       gemm_tile_coords(tile, tiles_m, tiles_n, &tm, &tn);
-      const int m0 = tm * T::BM, n0 = tn * T::BN;
+      const int m0 = (tm * CG + rank) * T::BM, n0 = tn * T::BN;
       ok = mbar_wait(&acc_full[buf], (t >> 1) & 1, abort_flag, prm.status, DEV_ERR_TIMEOUT_MMA);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
@@ -369,14 +419,29 @@ gemm_bf16_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       }
       }
       tc_fence_before();
-      mbar_arrive(&acc_empty[buf]);
+      if (CG == 2) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0));
+      } else {
+        mbar_arrive(&acc_empty[buf]);
+      }
     }
   }
 
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (warp == 2) {
+  if (CG == 2) {
+    // a CTA that gave up lets what it has in flight land in its pair's memory before either goes away
+    if (*abort_flag)
+      for (int i = 0; i < 50; ++i) __nanosleep(20000);
+    __syncwarp();
+    cluster_sync_all();
+    if (warp == 2) {
+      tc_fence_after();
+      tmem_dealloc_2cta(tmem_base, T::TMEM_COLS);
+    }
+  } else if (warp == 2) {
     if (*abort_flag)
       for (int i = 0; i < 50; ++i) __nanosleep(20000);
     tc_fence_after();

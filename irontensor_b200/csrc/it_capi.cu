@@ -603,21 +603,21 @@ struct ScatterEpilogue {
   int world, rows_per_rank;
 };
 
-template <int LAYOUT, bool QKV, bool RS, int BN>
+template <int LAYOUT, bool QKV, bool RS, int BN, int CG = 1>
 it_status launch_gemm_tiles(it_ctx* ctx, cudaStream_t s, int M, int N, int K, const void* a, long long lda, const void* b,
                       long long ldb, void* c, long long ldc, bool c_is_f32, const QkvEpilogue* epi,
                       const ScatterEpilogue* rs) {
-  using T = it::GemmTraits<BN>;
+  using T = it::GemmTraits<BN, CG>;
   CUtensorMap ma, mb;
   it_status st;
   const int a_rows = (LAYOUT == 2) ? K : M, a_cols = (LAYOUT == 2) ? M : K;
   const int b_rows = (LAYOUT == 0) ? N : K, b_cols = (LAYOUT == 0) ? K : N;
   const it::TensorStrides sa{lda, lda * a_rows, lda * a_rows, 1}, sb{ldb, ldb * b_rows, ldb * b_rows, 1};
   if ((st = make_tmap(ctx, &ma, a, 1, 1, a_rows, a_cols, sa, (LAYOUT == 2) ? T::BK : T::BM)) != IT_OK) return st;
-  if ((st = make_tmap(ctx, &mb, b, 1, 1, b_rows, b_cols, sb, (LAYOUT == 0) ? T::BN : T::BK)) != IT_OK) return st;
+  if ((st = make_tmap(ctx, &mb, b, 1, 1, b_rows, b_cols, sb, (LAYOUT == 0) ? T::B_ROWS : T::BK)) != IT_OK) return st;
   static std::atomic<bool> attr_set[16];   // zero-initialised; setting an attribute twice is harmless
   if (!attr_set[ctx->device & 15]) {
-    IT_CUDA(cudaFuncSetAttribute(it::gemm_bf16_sm100_kernel<LAYOUT, QKV, RS, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    IT_CUDA(cudaFuncSetAttribute(it::gemm_bf16_sm100_kernel<LAYOUT, QKV, RS, BN, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  T::SMEM_BYTES));
     attr_set[ctx->device & 15] = true;
   }
@@ -657,9 +657,10 @@ it_status launch_gemm_tiles(it_ctx* ctx, cudaStream_t s, int M, int N, int K, co
     p.ld_q = epi->ld_q;
     p.ld_kv = epi->ld_kv;
   }
-  const int n_tiles = ((M + T::BM - 1) / T::BM) * ((N + T::BN - 1) / T::BN);
-  const int grid = std::min(n_tiles, ctx->sm_count);
-  IT_CUDA(launch_dependent(it::gemm_bf16_sm100_kernel<LAYOUT, QKV, RS, BN>, grid, T::THREADS, T::SMEM_BYTES, s, ma, mb, p, RS ? rs_maps : no_maps));
+  const long long n_tiles = static_cast<long long>((M + CG * T::BM - 1) / (CG * T::BM)) * ((N + T::BN - 1) / T::BN);
+  const int grid = static_cast<int>(std::min<long long>(n_tiles, ctx->sm_count / CG)) * CG;
+  IT_CUDA(launch_cluster(it::gemm_bf16_sm100_kernel<LAYOUT, QKV, RS, BN, CG>, grid, T::THREADS, T::SMEM_BYTES, s, CG, ma, mb, p,
+                         RS ? rs_maps : no_maps));
   ctx->launches += 1;
   IT_CUDA(cudaGetLastError());
   return IT_OK;
@@ -667,7 +668,10 @@ it_status launch_gemm_tiles(it_ctx* ctx, cudaStream_t s, int M, int N, int K, co
 
 // Tile width: the one with the smallest (waves of tiles over the SMs) x (cost of a tile).  A 64-column tile costs 0.42 and a
 // 128-column one 0.575 of a 256-column tile (8192 x 2048 -> 6144: 282, 199 and 175 us): a stage's operands are 24, 32 and 48 KB
-// of shared-memory reads at 128 B per cycle against 128, 256 and 512 cycles of MMA.
+// of shared-memory reads at 128 B per cycle against 128, 256 and 512 cycles of MMA.  A 256 x 256 tile of a pair of CTAs costs
+// 0.89 (y = x W^T, dy W and dy^T x of 8192 x 2048 -> 6144: 209, 174 and 201 us in 256-column tiles, 184, 160 and 189 on pairs;
+// 2999 x 2048 -> 3072: 49, 50, 59 and 44, 45, 52) where K is long enough to hide what a pair starts with: at K = 512 it is
+// slower (6000 x 512 -> 1536: 20.2 and 22.8 us), at 1024 even.  IT_GEMM_TILE=64, 128, 256 or 512 (a pair) overrides the choice.
 template <int LAYOUT, bool QKV = false, bool RS = false>
 it_status launch_gemm(it_ctx* ctx, cudaStream_t s, int M, int N, int K, const void* a, long long lda, const void* b,
                       long long ldb, void* c, long long ldc, bool c_is_f32, const QkvEpilogue* epi = nullptr,
@@ -680,8 +684,13 @@ it_status launch_gemm(it_ctx* ctx, cudaStream_t s, int M, int N, int K, const vo
   if (!RS) {
     const double c256 = cost(256, 1.0), c128 = cost(128, 0.575), c64 = cost(64, 0.42);
     bn = c64 < c128 && c64 < c256 ? 64 : c128 < c256 ? 128 : 256;
+    const long long pair_tiles = static_cast<long long>((M + 255) / 256) * ((N + 255) / 256), pairs = std::max(1, ctx->sm_count / 2);
+    const double c_pair = static_cast<double>((pair_tiles + pairs - 1) / pairs) * 0.89;
+    if (K >= 1024 && c_pair < std::min(c256, std::min(c128, c64))) bn = 512;
+    if (const char* e = getenv("IT_GEMM_TILE")) bn = atoi(e);
   }
   if constexpr (!RS) {
+    if (bn == 512) return launch_gemm_tiles<LAYOUT, QKV, RS, 256, 2>(ctx, s, M, N, K, a, lda, b, ldb, c, ldc, c_is_f32, epi, rs);
     if (bn == 64) return launch_gemm_tiles<LAYOUT, QKV, RS, 64>(ctx, s, M, N, K, a, lda, b, ldb, c, ldc, c_is_f32, epi, rs);
     if (bn == 128) return launch_gemm_tiles<LAYOUT, QKV, RS, 128>(ctx, s, M, N, K, a, lda, b, ldb, c, ldc, c_is_f32, epi, rs);
   }

@@ -225,3 +225,20 @@ def test_out_of_memory_keeps_its_type(it_ctx):
     finally:
         torch.cuda.memory.set_per_process_memory_fraction(1.0)
     assert np.isfinite(flash_attention(t, t, t, True).to_f32_host()).all()
+
+
+# pairs of CTAs on a tile of 256 x 256: remainders of rows (a whole CTA's rows missing), columns and K, several tiles per pair
+@pytest.mark.parametrize("n,k,out", [(33, 72, 264), (130, 136, 200), (300, 264, 520), (257, 64, 256), (5000, 520, 5000)])
+def test_projection_on_pairs_of_ctas(it_ctx, monkeypatch, n, k, out):
+    """All three transposition cases, 1.7e-3 in L2 (2^-9 / sqrt(3) per bf16 element) for y and dx, fp32 sums for dW."""
+    import torch
+    from irontensor_b200 import Precision, Tensor, linear_backward, linear_forward
+    monkeypatch.setenv("IT_GEMM_TILE", "512")
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    x, w, dy = (torch.randn(s, generator=gen, device="cuda").to(torch.bfloat16) for s in ((n, k), (out, k), (n, out)))
+    tx, tw, tdy = (Tensor(t.reshape(-1), list(t.shape), Precision.BF16) for t in (x, w, dy))
+    y, (dx, dw) = linear_forward(tx, tw), linear_backward(tdy, tx, tw)
+    assert it_ctx.poll_status() == 0
+    x, w, dy = x.double(), w.double(), dy.double()
+    for got, want, bound in ((y, x @ w.T, 2e-3), (dx, dy @ w, 2e-3), (dw, dy.T @ x, 1e-5)):
+        assert (got.torch().reshape(want.shape).double() - want).norm() <= bound * want.norm()
