@@ -242,3 +242,16 @@ def test_projection_on_pairs_of_ctas(it_ctx, monkeypatch, n, k, out):
     x, w, dy = x.double(), w.double(), dy.double()
     for got, want, bound in ((y, x @ w.T, 2e-3), (dx, dy @ w, 2e-3), (dw, dy.T @ x, 1e-5)):
         assert (got.torch().reshape(want.shape).double() - want).norm() <= bound * want.norm()
+
+
+@pytest.mark.parametrize("D,kernel", [(64, "pp"), (128, "pp"), (64, "two"), (128, "two")])
+@pytest.mark.parametrize("S,causal", [(128, True), (129, False), (300, True), (520, False)])
+def test_bf16_forward_kernels_at_short_lengths(it_ctx, monkeypatch, D, kernel, S, causal):
+    """Either forward kernel may get any full-width launch, by how it fills the GPU: both, from one key tile on."""
+    monkeypatch.setenv("IT_FWD_KERNEL", kernel)
+    H = 6
+    q, k, v, d_o = seeded(970 + S + D, 1, H, S, D, bf16=True)
+    o, lse, _, _, _ = gu.run_fwd_bwd(it_ctx, q, k, v, d_o, causal, bf16=True)
+    ro, rlse = ol.fwd(q, k, v, causal)
+    assert np.abs(lse - rlse).max() <= 1e-4
+    check_bf16(o, ro, f"{(S, D, kernel)} O")
