@@ -1316,6 +1316,26 @@ it_status it_rope_qk(it_ctx* ctx, it_stream* stream, it_dtype dtype, int32_t B, 
   const int threads = half * std::max(1, std::min(n_heads, 256 / half));
   const unsigned grid = static_cast<unsigned>(static_cast<int64_t>(B) * S);
   const void* kin = Hkv > 0 ? k_in : nullptr;
+  const int row_bytes = D * (dtype == IT_F32 ? 4 : 2);
+  if ((row_bytes & 15) == 0 && aligned16(q_in) && aligned16(q_out) && aligned16(k_in) && aligned16(k_out)) {
+    // as many positions per CTA as have one sine per thread, as long as that leaves four CTAs per SM
+    const int64_t rows = static_cast<int64_t>(B) * S;
+    const int n_pos = static_cast<int>(std::clamp<int64_t>(rows / (4LL * ctx->sm_count), 1, 256 / half));
+    const unsigned ctas = static_cast<unsigned>((rows + n_pos - 1) / n_pos);
+#define IT_ROPE_CHUNKS(ST, INV)                                                                                               \
+  IT_CUDA(launch_dependent(it::rope_qk_chunks_kernel<ST, INV>, ctas, 256, 0, stream->s, static_cast<const ST*>(q_in),         \
+                           static_cast<const ST*>(k_in), static_cast<ST*>(q_out), static_cast<ST*>(k_out), rows, n_pos, S, H, Hkv, D, rf))
+    if (dtype == IT_F32) {
+      if (inverse) IT_ROPE_CHUNKS(float, true);
+      else IT_ROPE_CHUNKS(float, false);
+    } else {
+      if (inverse) IT_ROPE_CHUNKS(__nv_bfloat16, true);
+      else IT_ROPE_CHUNKS(__nv_bfloat16, false);
+    }
+#undef IT_ROPE_CHUNKS
+    ctx->launches += 1;
+    return IT_OK;
+  }
 #define IT_ROPE_LAUNCH(ST, INV)                                                                                   \
   it::rope_qk_kernel<ST, INV><<<grid, threads, 0, stream->s>>>(static_cast<const ST*>(q_in), static_cast<const ST*>(kin), \
                                                                static_cast<ST*>(q_out), static_cast<ST*>(k_out), S, H, Hkv, D, rf)

@@ -67,6 +67,78 @@ rope_qk_kernel(const ST* __restrict__ q_in, const ST* __restrict__ k_in, ST* __r
   }
 }
 
+// The same for rows of whole 16-byte chunks (head_dim a multiple of 8 in bf16, of 4 in fp32): a CTA owns `n_pos` positions,
+// evaluates their sines and cosines once, at most one per thread, into shared memory, and streams the heads of Q and K in
+// 16-byte chunks, four loads of a thread in flight and issued in front of the sines.  The kernel above evaluates them in
+// every thread and moves 4 bytes per thread and head.  Bound: memory latency at the sizes of one layer (2 x 1003 positions, 16 + 4
+// heads of 96 columns, bf16, inside a training step of attention: 118.5 -> 116.0 us for the step).
+template <typename ST, bool INVERSE>
+__global__ void __launch_bounds__(256)
+rope_qk_chunks_kernel(const ST* q_in, const ST* k_in, ST* q_out, ST* k_out, long long rows, int n_pos, int S, int H, int Hkv, int D,
+                      const __grid_constant__ RopeFreqs freqs) {
+  constexpr int VEC = 16 / sizeof(ST);
+  __shared__ float2 tab[256];
+  const int half = D >> 1, per_head = D / VEC;
+  const int n_heads = H + Hkv;
+  const long long row0 = static_cast<long long>(blockIdx.x) * n_pos;
+  const int n_rows = static_cast<int>(min(static_cast<long long>(n_pos), rows - row0));
+  const int n_chunks = n_rows * n_heads * per_head;
+  ptx::grid_dep_wait();
+  ptx::grid_dep_launch();
+  // chunk index -> element offset in Q (or, past H heads, in K), local row and first column
+  auto locate = [&](int i, bool* is_q, long long* off, int* r, int* d) {
+    const int head_row = i / per_head;
+    *d = (i - head_row * per_head) * VEC;
+    *r = head_row / n_heads;
+    const int hh = head_row - *r * n_heads;
+    *is_q = hh < H;
+    *off = (*is_q ? (row0 + *r) * H + hh : (row0 + *r) * Hkv + (hh - H)) * D + *d;
+  };
+  bool first = true;
+  for (int base = static_cast<int>(threadIdx.x); first || base < n_chunks; base += 4 * 256) {
+    uint4 x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = base + u * 256;
+      if (i < n_chunks) {
+        bool is_q;
+        long long off;
+        int r, d;
+        locate(i, &is_q, &off, &r, &d);
+        x[u] = *reinterpret_cast<const uint4*>((is_q ? q_in : k_in) + off);
+      }
+    }
+    if (first) {   // every thread passes here once
+      for (int t = static_cast<int>(threadIdx.x); t < n_rows * half; t += 256) {
+        const int r = t / half;
+        float c, s;
+        rope_sincos(freqs, static_cast<int>((row0 + r) % S) + freqs.position_offset, t - r * half, &c, &s);
+        tab[t] = make_float2(c, INVERSE ? -s : s);
+      }
+      __syncthreads();
+      first = false;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = base + u * 256;
+      if (i >= n_chunks) break;
+      bool is_q;
+      long long off;
+      int r, d;
+      locate(i, &is_q, &off, &r, &d);
+      const float2* cs = &tab[r * half + (d >> 1)];
+      ST* e = reinterpret_cast<ST*>(&x[u]);
+#pragma unroll
+      for (int p = 0; p < VEC / 2; ++p) {
+        const float x0 = rope_ld(e + 2 * p), x1 = rope_ld(e + 2 * p + 1);
+        rope_st(e + 2 * p, x0 * cs[p].x - x1 * cs[p].y);
+        rope_st(e + 2 * p + 1, x0 * cs[p].y + x1 * cs[p].x);
+      }
+      *reinterpret_cast<uint4*>((is_q ? q_out : k_out) + off) = x[u];
+    }
+  }
+}
+
 // (cos, sin) of every (sequence index, dimension pair): [S][D/2] float2.  Built once per call for kernels that would
 // otherwise evaluate the same sine and cosine once per head (the attention backward) or per column tile (the fused QKV
 // projection).  `first` and `stride` number the threads that share the work.

@@ -255,3 +255,19 @@ def test_bf16_forward_kernels_at_short_lengths(it_ctx, monkeypatch, D, kernel, S
     ro, rlse = ol.fwd(q, k, v, causal)
     assert np.abs(lse - rlse).max() <= 1e-4
     check_bf16(o, ro, f"{(S, D, kernel)} O")
+
+
+# rows of whole 16-byte chunks and others, one position per CTA and several with a remainder, heads of Q and K apart and alike
+@pytest.mark.parametrize("B,S,H,Hkv,D,bf16", [(1, 1, 3, 1, 8, True), (2, 1003, 4, 2, 96, True), (3, 700, 2, 2, 128, True), (1, 2500, 1, 1, 4, False),
+                                              (2, 333, 3, 1, 64, False), (1, 77, 2, 1, 20, True), (1, 50, 2, 2, 6, False)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_rope_of_any_row_width(it_ctx, B, S, H, Hkv, D, bf16, inverse):
+    from irontensor_b200 import Tensor, rope_qk
+    q, k = (synth.normal(995, t, 0, B * S * h * D, 1.0).reshape(B, S, h, D) for t, h in ((synth.TENSOR_Q, H), (synth.TENSOR_K, Hkv)))
+    if bf16:
+        q, k = synth.round_bf16(q), synth.round_bf16(k)
+    make = Tensor.from_f32_as_bf16 if bf16 else Tensor.from_f32_slice
+    got = rope_qk(make(q.reshape(-1), list(q.shape)), make(k.reshape(-1), list(k.shape)), 10000.0, 11, inverse=inverse)
+    for g, x in zip(got, (q, k)):
+        want = ol.rope(x, 10000.0, 11, inverse=inverse)
+        assert np.abs(g.to_f32_host() - want).max() <= (2.0 ** -8 * np.abs(want).max() if bf16 else 1e-5)
