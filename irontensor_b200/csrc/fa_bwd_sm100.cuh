@@ -28,6 +28,8 @@
 // [64,96): each math group overwrites only columns it has already read), dP^T and dQ (aliased) [128,256),
 // dV [256,256+D), dK [384,384+D).
 #pragma once
+#include <cooperative_groups.h>
+
 #include "rope.cuh"
 #include "sm100_ptx.cuh"
 
@@ -75,6 +77,7 @@ struct BwdParams {
   int BH;
   int causal;
   int head_dim;            // columns of the tensors: D, or fewer in the PAD instantiations
+  int n_split;             // SPLIT instantiations: CTAs (one cluster) per key tile
   float scale;             // 1/sqrt(head_dim)
   float scale_log2;        // scale * log2(e)
 };
@@ -206,7 +209,11 @@ __global__ void fa_bwd_finish_kernel(const float* __restrict__ dq_accum, __nv_bf
 // ------------------------------------------------------------------ (2) main kernel
 // PAD: tensors with fewer columns than D (see fa_fwd_sm100.cuh): zero-filled on load, the contractions over the head
 // dimension and the widths of dV, dK and dQ stop at the last 16-column step that holds data.
-template <int D, int KT = 1, bool PAD = false>
+// SPLIT: the iterations (query head of the group, query tile) of a key tile are shared out among the CTAs of a cluster, in
+// equal contiguous parts; the parts of dK and dV meet through distributed shared memory in the epilogue (summed in rank
+// order).  For launches whose longest CTA is what everybody waits for: a key tile of a K/V head shared by four query heads
+// takes four times as long, and there are a quarter as many (the launcher has the rule and the figures).
+template <int D, int KT = 1, bool PAD = false, bool SPLIT = false>
 __global__ void __launch_bounds__(512, 1)
 fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
@@ -250,7 +257,11 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   // half as many start-ups and epilogues, for the same work -- at a thousand keys those are half of a CTA's life.
   const int n_kp = (n_k_tiles + KT - 1) / KT;
   int bhk, ktp;   // batch * kv_heads + kv_head, index of the CTA's key tiles
-  grouped_tile_order(static_cast<int>(blockIdx.x), n_kp, static_cast<int>(gridDim.x) / n_kp, &bhk, &ktp);
+  static_assert(!SPLIT || KT == 1, "a split key tile is the CTA's only one");
+  const int n_split = SPLIT ? prm.n_split : 1;
+  const int rank = SPLIT ? static_cast<int>(blockIdx.x) % n_split : 0;
+  const int cta = SPLIT ? static_cast<int>(blockIdx.x) / n_split : static_cast<int>(blockIdx.x);
+  grouped_tile_order(cta, n_kp, static_cast<int>(gridDim.x) / (n_kp * n_split), &bhk, &ktp);
   const int kt = ktp * KT;                                    // first key tile
   const int nk_cta = min(KT, n_k_tiles - kt);                 // key tiles this CTA owns
   const int hkv = bhk % kv_heads, bt = bhk / kv_heads;        // TMA coordinates of the K/V slice
@@ -259,8 +270,10 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   // An iteration = (query head of the group, query tile, one of the CTA's key tiles), in that nesting; under the causal
   // mask key tile kt + t takes part from query tile kt + t on.
   const int per_head = prm.causal ? (n_q_tiles - kt) * nk_cta - (nk_cta * (nk_cta - 1)) / 2 : n_q_tiles * nk_cta;
-  const int n_iter = per_head * G;
-  // (g, qi, t) of the next iteration; every role walks the same sequence, starting at (0, i0, 0)
+  const int it_lo = SPLIT ? per_head * G * rank / n_split : 0;   // a cluster's CTA takes iterations [it_lo, it_lo + n_iter)
+  const int n_iter = SPLIT ? per_head * G * (rank + 1) / n_split - it_lo : per_head * G;
+  const int g0 = SPLIT ? it_lo / per_head : 0, q0 = SPLIT ? i0 + it_lo % per_head : i0;
+  // (g, qi, t) of the next iteration; every role walks the same sequence, starting at (g0, q0, 0)
   auto advance = [&](int& g_, int& qi_, int& t_) {
     ++t_;
     if (t_ >= nk_cta || (prm.causal && qi_ < kt + t_)) {
@@ -345,7 +358,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         tma_load_4d(smem + T::SMEM_K + t * T::TILE_BYTES + b * T::BLOCK_BYTES, &tmap_k, kv_full, b * 64, (kt + t) * T::BM, hkv, bt);
         tma_load_4d(smem + T::SMEM_V + t * T::TILE_BYTES + b * T::BLOCK_BYTES, &tmap_v, kv_full, b * 64, (kt + t) * T::BM, hkv, bt);
       }
-    load_q_do(0, i0, 0);
+    load_q_do(0, q0, g0);
   }
   if (warp == 2) {
     tmem_alloc(tmem_slot, T::TMEM_COLS);
@@ -372,7 +385,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       // ------------------------------------------------------------ TMA producer
       // (K, V and the first query tile's loads were issued by this thread before the CTA-wide set-up barrier.)
       if (elect_one()) {
-        int g = 0, qi = i0, t = 0;   // iteration 0
+        int g = g0, qi = q0, t = 0;   // iteration 0
         for (int n = 1; n < n_iter; ++n) {
           advance(g, qi, t);
           if (!load_q_do(n, qi, g)) break;   // (with two key tiles a query tile is fetched once per key tile; the second comes from L2)
@@ -457,7 +470,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           issue_st(0, 0, none);
         }
         bool r_do = false, r_dq = false, r_p = false, r_q = false, r_ds = false;   // answers of the early probes
-        int g_c = 0, qi_c = i0, t_c = 0;     // this iteration's query head, query tile and key tile
+        int g_c = g0, qi_c = q0, t_c = 0;     // this iteration's query head, query tile and key tile
         bool started[KT] = {};               // has the key tile's dV / dK accumulation begun?
         for (int n = 0; n < n_iter && ok; ++n) {
           const int t = t_c;
@@ -508,7 +521,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       if (elect_one()) {
         bool ok = true;
         int g = 0;
-        int g_q = 0, qi = i0, t_q = 0;
+        int g_q = g0, qi = q0, t_q = 0;
         for (int n = 0; n < n_iter && ok; ++n, advance(g_q, qi, t_q)) {
           const int bh_q = bh0 + g_q;
 #pragma unroll
@@ -545,7 +558,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       bool ok = true;
       uint32_t ra[16], rb[16];
       uint32_t p_keep[32];   // this thread's 64 P^T values, packed bf16, kept between the two phases
-      int g_m = 0, qi = i0, t_m = 0;
+      int g_m = g0, qi = q0, t_m = 0;
       for (int n = 0; n < n_iter; ++n, advance(g_m, qi, t_m)) {
         const int st = n & 1;
         const bool diag = prm.causal && (qi == kt + t_m);   // the key tile's own query tile: keys after the query are masked
@@ -637,6 +650,21 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         // each math group writes one half of the head dimension of its key row's dV and dK
         tc_fence_after();
         constexpr int HC = D / 2;
+        if constexpr (SPLIT) {
+          // this CTA's part, fp32, over the operand tiles (every MMA that read them is complete): rows of D + 4 floats
+#pragma unroll 1
+          for (int which = 0; which < 2; ++which) {
+            float* srow = reinterpret_cast<float*>(smem) + (which * T::BM + k_local) * (D + 4) + half * HC;
+#pragma unroll 1
+            for (int c = 0; c < HC / 16; ++c) {
+              tmem_ld_x16(t_lane + (which ? T::COL_DK : T::COL_DV) + half * HC + c * 16, ra);
+              tmem_wait_ld();
+#pragma unroll
+              for (int v4 = 0; v4 < 4; ++v4)
+                *reinterpret_cast<uint4*>(srow + c * 16 + v4 * 4) = make_uint4(ra[v4 * 4], ra[v4 * 4 + 1], ra[v4 * 4 + 2], ra[v4 * 4 + 3]);
+            }
+          }
+        } else
 #pragma unroll 1
         for (int tw = 0; tw < 2 * nk_cta; ++tw) {   // dV then dK of each of the CTA's key tiles
           const int t = tw >> 1, which = tw & 1;
@@ -727,6 +755,56 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         }
       }
     }
+  }
+
+  if constexpr (SPLIT) {
+    static_assert(2 * T::BM * (D + 4) * 4 <= T::SMEM_DQS, "the parts of dK and dV reach into the dQ staging buffers");
+    // Every thread of every CTA passes both cluster barriers, whatever happened to it before (a CTA that gave up leaves
+    // garbage behind, as any launch does then).
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __syncwarp();
+    cluster.sync();
+    if (warp >= 4 && warp < 12) {
+      // CTA `rank` finishes every n_split-th float4 of the dV and dK tiles, four at a time so that their loads are in flight
+      // together.  A part with no iterations left nothing to add.
+      constexpr int N4 = 2 * T::BM * (D / 4);
+      const int total = per_head * G, step = 256 * n_split;
+      for (int first = rank * 256 + static_cast<int>(threadIdx.x) - 128; first < N4; first += 4 * step) {
+        float4 a[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) a[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int c = 0; c < n_split; ++c) {
+          if (total * c / n_split == total * (c + 1) / n_split) continue;
+          const float* part = cluster.map_shared_rank(reinterpret_cast<float*>(smem), c);
+          float4 x[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int i = min(first + u * step, N4 - 1);
+            x[u] = *reinterpret_cast<const float4*>(part + (i / (D / 4)) * (D + 4) + (i % (D / 4)) * 4);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) a[u] = make_float4(a[u].x + x[u].x, a[u].y + x[u].y, a[u].z + x[u].z, a[u].w + x[u].w);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = first + u * step;
+          const int which = i / (T::BM * (D / 4)), row = (i / (D / 4)) % T::BM, d = (i % (D / 4)) * 4;
+          const int k_row = kt * T::BM + row;
+          if (i >= N4 || k_row >= S || (PAD && d >= prm.head_dim)) continue;
+          float4 g = a[u];
+          if (which && prm.rope_table != nullptr) {   // dK leaves through the inverse rotary rotation of its key position
+            const float4 cs = *reinterpret_cast<const float4*>(
+                prm.rope_table + static_cast<size_t>(k_row) * ((PAD ? prm.head_dim : D) >> 1) + (d >> 1));
+            g = make_float4(g.x * cs.x + g.y * cs.y, g.y * cs.x - g.x * cs.y, g.z * cs.z + g.w * cs.w, g.w * cs.z - g.z * cs.w);
+          }
+          const float f = which ? prm.scale : 1.0f;
+          __nv_bfloat16* out = (which ? prm.dk : prm.dv) + prm.st_kv.slice(bh0) + static_cast<long long>(k_row) * prm.st_kv.row + d;
+          *reinterpret_cast<uint2*>(out) = make_uint2(pack_bf16(g.x * f, g.y * f), pack_bf16(g.z * f, g.w * f));
+        }
+      }
+    }
+    cluster.sync();   // nobody's shared memory goes away while it is read
   }
 
   // ------------------------------------------------------------------ teardown

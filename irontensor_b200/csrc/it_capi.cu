@@ -508,6 +508,25 @@ BwdWorkspace bwd_workspace_layout(it_dtype dtype, int64_t BH, int64_t S, int64_t
   return w;
 }
 
+// CTAs per key tile of the bf16 backward (one cluster; 1: no split).  The longest CTA walks group * n_kt (query head, query
+// tile) pairs; a launch cannot be quicker than that, nor than its pairs shared out evenly over the SMs.  Estimate of both, in
+// pairs, with what a CTA costs besides (set-up, epilogue, and the merge of a cluster); clusters of four do not find room on
+// every SM.  Fitted to 403 shapes (head_dim 64, 96 and 128, groups of 1, 2 and 4) timed with 1, 2 and 4 CTAs per tile: the
+// choice is nowhere more than 2.5 % behind no split.  Below 8 pairs the merge costs what the split gains.  Backward, us, with
+// 1, 2, 4: B1 S1003 H8 Hkv2 D64 61, 40, 28; B2 S2048 H16 Hkv4 D64 126, 85, 113; B1 S2500 H8 Hkv2 D96 286, 163, 94.
+// IT_BWD_SPLIT=1, 2 or 4 in the environment overrides the choice.
+int bwd_splits(int sm_count, int n_kt, long long kv_slices, int group, int causal) {
+  if (const char* e = getenv("IT_BWD_SPLIT")) return e[0] == '4' ? 4 : e[0] == '2' ? 2 : 1;
+  const long long longest = static_cast<long long>(group) * n_kt, ctas = kv_slices * n_kt;
+  if (longest < 8) return 1;
+  const double pairs = static_cast<double>(kv_slices) * group * (causal ? 0.5 * n_kt * (n_kt + 1) : static_cast<double>(n_kt) * n_kt);
+  auto estimate = [&](int c, double per_cta, double sms) {
+    return std::max(static_cast<double>((longest + c - 1) / c) + per_cta, (pairs + per_cta * static_cast<double>(ctas) * c) / sms);
+  };
+  const double one = estimate(1, 4, sm_count), two = estimate(2, 6, 0.88 * sm_count), four = estimate(4, 5, 0.81 * sm_count);
+  return one <= two && one <= four ? 1 : two <= four ? 2 : 4;
+}
+
 template <int D, bool PAD = false>
 it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int head_dim, int causal, const void* q, const void* k,
                            const void* v, const void* o, const void* d_o, const float* lse, void* dq, void* dk,
@@ -537,6 +556,8 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
   static std::atomic<bool> attr_set[16];   // zero-initialised; setting an attribute twice is harmless
   if (!attr_set[ctx->device & 15]) {
     IT_CUDA(cudaFuncSetAttribute(it::fa_bwd_sm100_kernel<D, 1, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 it::BwdTraits<D, 1>::SMEM_BYTES));
+    IT_CUDA(cudaFuncSetAttribute(it::fa_bwd_sm100_kernel<D, 1, PAD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  it::BwdTraits<D, 1>::SMEM_BYTES));
     if constexpr (D == 64)
       IT_CUDA(cudaFuncSetAttribute(it::fa_bwd_sm100_kernel<D, 2, PAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -578,6 +599,7 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
   const char* force = getenv("IT_BWD_KEY_TILES");
   const bool two_tiles = (D == 64) && n_kt >= 2 &&
                          (force != nullptr ? force[0] == '2' : static_cast<long long>(n_kt) * B * Hkv > 2LL * ctx->sm_count);
+  p.n_split = two_tiles ? 1 : bwd_splits(ctx->sm_count, n_kt, static_cast<long long>(B) * Hkv, skv.group, causal);
   if (ctx->timing >= 3) {
     IT_CUDA(cudaEventRecord(ctx->ev[2][1], s));
     ctx->ev_valid[2] = true;
@@ -588,7 +610,10 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
       IT_CUDA(launch_dependent(it::fa_bwd_sm100_kernel<D, 2, PAD>, static_cast<unsigned>((n_kt + 1) / 2) * B * Hkv, T::THREADS,
                                it::BwdTraits<D, 2>::SMEM_BYTES, s, mq, mk, mv, mdo, mdq, p));
   }
-  if (!two_tiles)
+  if (p.n_split > 1)
+    IT_CUDA(launch_cluster(it::fa_bwd_sm100_kernel<D, 1, PAD, true>, static_cast<unsigned>(n_kt) * B * Hkv * p.n_split, T::THREADS,
+                           T::SMEM_BYTES, s, p.n_split, mq, mk, mv, mdo, mdq, p));
+  else if (!two_tiles)
     IT_CUDA(launch_dependent(it::fa_bwd_sm100_kernel<D, 1, PAD>, static_cast<unsigned>(n_kt) * B * Hkv, T::THREADS, T::SMEM_BYTES, s,
                              mq, mk, mv, mdo, mdq, p));
   if (ctx->timing) {

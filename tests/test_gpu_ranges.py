@@ -271,3 +271,27 @@ def test_rope_of_any_row_width(it_ctx, B, S, H, Hkv, D, bf16, inverse):
     for g, x in zip(got, (q, k)):
         want = ol.rope(x, 10000.0, 11, inverse=inverse)
         assert np.abs(g.to_f32_host() - want).max() <= (2.0 ** -8 * np.abs(want).max() if bf16 else 1e-5)
+
+
+@pytest.mark.parametrize("split", ["2", "4"])
+@pytest.mark.parametrize("B,S,H,Hkv,D,causal,rope", [
+    (1, 100, 4, 1, 64, True, False),     # one query tile per head: parts of one iteration
+    (2, 128, 2, 2, 128, True, True),     # one iteration in all: parts without any
+    (1, 300, 6, 2, 128, False, True), (2, 385, 4, 1, 64, True, True), (1, 640, 8, 2, 96, True, True), (1, 257, 3, 3, 40, True, False),
+])
+def test_bf16_backward_split_over_a_cluster(it_ctx, monkeypatch, split, B, S, H, Hkv, D, causal, rope):
+    from irontensor_b200 import Tensor, attention_gqa, attention_gqa_backward
+    q, _, _, d_o = [np.ascontiguousarray(t.transpose(0, 2, 1, 3)) for t in seeded(980 + S, B, H, S, D, bf16=True)]
+    _, k, v, _ = [np.ascontiguousarray(t.transpose(0, 2, 1, 3)) for t in seeded(981 + S, B, Hkv, S, D, bf16=True)]
+    tq, tk, tv, tdo = (Tensor.from_f32_as_bf16(t.reshape(-1), list(t.shape)) for t in (q, k, v, d_o))
+    o = attention_gqa(tq, tk, tv, causal)
+    monkeypatch.setenv("IT_BWD_SPLIT", split)
+    monkeypatch.setenv("IT_BWD_KEY_TILES", "1")
+    dq, dk, dv = attention_gqa_backward(tdo, tq, tk, tv, o, causal, rope_base=10000.0 if rope else None, position_offset=3)
+    assert it_ctx.poll_status() == 0
+    rdq, rdk, rdv = ol.gqa_bwd(q, k, v, d_o, causal)
+    if rope:
+        rdq, rdk = ol.rope(rdq, 10000.0, 3, inverse=True), ol.rope(rdk, 10000.0, 3, inverse=True)
+    for got, want, name in ((dq, rdq, "dQ"), (dk, rdk, "dK"), (dv, rdv, "dV")):
+        scale = math.sqrt(H // Hkv) if name in ("dK", "dV") else 1.0   # sums over the group's heads
+        check_bf16(got.to_f32_host() / scale, want / scale, f"{(B, S, H, Hkv, D)} {name}")
