@@ -208,7 +208,10 @@ __global__ void fa_bwd_finish_kernel(const float* __restrict__ dq_accum, __nv_bf
 
 // ------------------------------------------------------------------ (2) main kernel
 // PAD: tensors with fewer columns than D (see fa_fwd_sm100.cuh): zero-filled on load, the contractions over the head
-// dimension and the widths of dV, dK and dQ stop at the last 16-column step that holds data.
+// dimension and the widths of dV, dK and dQ stop at the last 16-column step that holds data.  As in the forward these
+// instantiations keep P, and dS too, in two bf16 terms: one term would put dQ and dK 3.0e-3 off 64 bits, where the CUDA-core
+// kernels that had these shapes before were 1.8e-3 off.  P^T takes the whole of its math group's columns of S^T; the low
+// term of dS^T waits in registers until dK and dQ have read the high one from shared memory, then takes its place there.
 // SPLIT: the iterations (query head of the group, query tile) of a key tile are shared out among the CTAs of a cluster, in
 // equal contiguous parts; the parts of dK and dV meet through distributed shared memory in the epilogue (summed in rank
 // order).  For launches whose longest CTA is what everybody waits for: a key tile of a K/V head shared by four query heads
@@ -227,6 +230,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   uint64_t* q_full = bars + 1;     // [2]
   uint64_t* q_empty = bars + 3;    // [2]
   uint64_t* do_full = bars + 5;
+  uint64_t* hi_done = bars + 6;    // PAD: dK and dQ have read the high term of dS
   uint64_t* do_empty = bars + 7;
   uint64_t* st_full = bars + 9;
   uint64_t* dpt_full = bars + 10;
@@ -305,6 +309,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     mbar_init(dpt_full, 1);
     mbar_init(p_full, 256);
     mbar_init(ds_full, 256);
+    mbar_init(hi_done, 1);
     mbar_init(dq_full, 1);
     mbar_init(dq_empty, 128);
     mbar_init(dkv_done, 1);
@@ -441,6 +446,12 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             umma_ts(tmem_base + T::COL_DV + t * D, tmem_base + T::COL_ST + (kk >> 2) * 64 + (kk & 3) * 8,
                     sdesc_advance(db, kk * 2048), IDESC_ND, (!first || kk > 0) ? 1u : 0u);
           }
+          if (PAD) {   // the low terms of P^T
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+              umma_ts(tmem_base + T::COL_DV + t * D, tmem_base + T::COL_ST + (kk >> 2) * 64 + 32 + (kk & 3) * 8,
+                      sdesc_advance(db, kk * 2048), IDESC_ND, 1u);
+          }
         };
         auto issue_dk = [&](int st, int t, bool first, auto mid) {   // dK += dS^T * Q   (A = dS^T K-major, B = Q N-major)
           const uint64_t da = make_sdesc(ds_addr, 16, 1024);
@@ -452,13 +463,13 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     (!first || kk > 0) ? 1u : 0u);
           }
         };
-        auto issue_dq = [&](int t) {   // dQ = dS * K   (A = dS M-major from the same buffer, B = K N-major)
+        auto issue_dq = [&](int t, bool first) {   // dQ = dS * K   (A = dS M-major from the same buffer, B = K N-major)
           const uint64_t da = make_sdesc(ds_addr, T::BLOCK_BYTES, 1024);
           const uint64_t db = make_sdesc(k_addr + t * T::TILE_BYTES, T::BLOCK_BYTES, 1024);
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
             umma_ss(tmem_base + T::COL_DQ, sdesc_advance(da, kk * 2048), sdesc_advance(db, kk * 2048), IDESC_DQ,
-                    kk > 0);
+                    (!first || kk > 0) ? 1u : 0u);
         };
         auto need = [&](bool ready, uint64_t* bar, uint32_t parity, int code) {
           return ready || mbar_wait_parked(bar, parity, abort_flag, prm.status, code);
@@ -498,14 +509,22 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             ok = need(r_q, &q_full[st_n], ph_n, DEV_ERR_TIMEOUT_LOAD);
             if (!ok) break;
             tc_fence_after();
-            issue_st(st_n, t_c, [&] { r_ds = mbar_test_wait(ds_full, par); });
+            issue_st(st_n, t_c, [&] { r_ds = mbar_test_wait(ds_full, PAD ? 0u : par); });
           }
-          ok = need(r_ds, ds_full, par, DEV_ERR_TIMEOUT_SOFTMAX);
+          ok = need(r_ds, ds_full, PAD ? 0u : par, DEV_ERR_TIMEOUT_SOFTMAX);
           if (!ok) break;
           tc_fence_after();
-          issue_dq(t);
+          if (PAD) {   // ds_full completes twice per iteration: high terms, low terms
+            issue_dk(st, t, first, none);
+            issue_dq(t, true);
+            umma_commit(hi_done);
+            ok = mbar_wait_parked(ds_full, 1, abort_flag, prm.status, DEV_ERR_TIMEOUT_SOFTMAX);
+            if (!ok) break;
+            tc_fence_after();
+          }
+          issue_dq(t, !PAD);
           umma_commit(dq_full);
-          issue_dk(st, t, first, [&] {
+          issue_dk(st, t, first && !PAD, [&] {
             r_do = more && mbar_test_wait(do_full, par ^ 1);
             r_dq = more && mbar_test_wait(dq_empty, par);
           });
@@ -558,6 +577,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       bool ok = true;
       uint32_t ra[16], rb[16];
       uint32_t p_keep[32];   // this thread's 64 P^T values, packed bf16, kept between the two phases
+      uint32_t p_low[PAD ? 32 : 1];   // PAD: their second terms; then those of dS^T
       int g_m = g0, qi = q0, t_m = 0;
       for (int n = 0; n < n_iter; ++n, advance(g_m, qi, t_m)) {
         const int st = n & 1;
@@ -588,6 +608,10 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             }
             p_keep[c * 8 + (i >> 1)] = pack_bf16(p0, p1);
             p_keep[c * 8 + (i >> 1) + 1] = pack_bf16(p2, p3);
+            if constexpr (PAD) {
+              p_low[c * 8 + (i >> 1)] = pack_bf16_rest(p_keep[c * 8 + (i >> 1)], p0, p1);
+              p_low[c * 8 + (i >> 1) + 1] = pack_bf16_rest(p_keep[c * 8 + (i >> 1) + 1], p2, p3);
+            }
           }
         };
         tmem_ld_x16(t_st, ra);
@@ -602,6 +626,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         phase_a(ra, 2);
         tmem_wait_ld();
         phase_a(rb, 3);
+        if constexpr (PAD) tmem_st_x32(t_st + 32, p_low);
         tmem_st_x32(t_st, p_keep);   // 64 queries -> 32 packed columns at the start of this group's own range
         tmem_wait_st();
         tc_fence_before();
@@ -617,10 +642,21 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           for (int i = 0; i < 16; i += 4) {
             const float4 d4 = *reinterpret_cast<const float4*>(dl_s + c * 16 + i);
             const uint32_t pa = p_keep[c * 8 + (i >> 1)], pb = p_keep[c * 8 + (i >> 1) + 1];
-            const float p0 = __uint_as_float(pa << 16), p1 = __uint_as_float(pa & 0xFFFF0000u);
-            const float p2 = __uint_as_float(pb << 16), p3 = __uint_as_float(pb & 0xFFFF0000u);
-            dsp[i >> 1] = pack_bf16(p0 * (__uint_as_float(r[i + 0]) - d4.x), p1 * (__uint_as_float(r[i + 1]) - d4.y));
-            dsp[(i >> 1) + 1] = pack_bf16(p2 * (__uint_as_float(r[i + 2]) - d4.z), p3 * (__uint_as_float(r[i + 3]) - d4.w));
+            float p0 = __uint_as_float(pa << 16), p1 = __uint_as_float(pa & 0xFFFF0000u);
+            float p2 = __uint_as_float(pb << 16), p3 = __uint_as_float(pb & 0xFFFF0000u);
+            if constexpr (PAD) {
+              const uint32_t la = p_low[c * 8 + (i >> 1)], lb = p_low[c * 8 + (i >> 1) + 1];
+              p0 += __uint_as_float(la << 16), p1 += __uint_as_float(la & 0xFFFF0000u);
+              p2 += __uint_as_float(lb << 16), p3 += __uint_as_float(lb & 0xFFFF0000u);
+            }
+            const float s0 = p0 * (__uint_as_float(r[i + 0]) - d4.x), s1 = p1 * (__uint_as_float(r[i + 1]) - d4.y);
+            const float s2 = p2 * (__uint_as_float(r[i + 2]) - d4.z), s3 = p3 * (__uint_as_float(r[i + 3]) - d4.w);
+            dsp[i >> 1] = pack_bf16(s0, s1);
+            dsp[(i >> 1) + 1] = pack_bf16(s2, s3);
+            if constexpr (PAD) {
+              p_low[c * 8 + (i >> 1)] = pack_bf16_rest(dsp[i >> 1], s0, s1);
+              p_low[c * 8 + (i >> 1) + 1] = pack_bf16_rest(dsp[(i >> 1) + 1], s2, s3);
+            }
           }
           // 16 query columns = two 16-byte chunks of this key row
           *reinterpret_cast<uint4*>(ds_row + (((2 * c) ^ swz) << 4)) = make_uint4(dsp[0], dsp[1], dsp[2], dsp[3]);
@@ -641,6 +677,18 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         tc_fence_before();
         fence_proxy_async_smem();
         mbar_arrive(ds_full);
+        if constexpr (PAD) {
+          ok = mbar_wait_parked(hi_done, n & 1, abort_flag, prm.status, DEV_ERR_TIMEOUT_MMA);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            *reinterpret_cast<uint4*>(ds_row + ((c ^ swz) << 4)) = make_uint4(p_low[c * 4], p_low[c * 4 + 1], p_low[c * 4 + 2], p_low[c * 4 + 3]);
+          tc_fence_before();
+          fence_proxy_async_smem();
+          mbar_arrive(ds_full);
+        }
       }
       if (ok) {
         ok = mbar_wait_parked(dkv_done, 0, abort_flag, prm.status, DEV_ERR_TIMEOUT_MMA);

@@ -69,6 +69,9 @@ struct FwdParams {
 // PAD: tensors with fewer columns than D (any multiple of 8).  TMA fills the missing columns of every tile with zeros, so
 // the shared-memory image is that of a D-column tensor; the MMAs run over the 16-column steps that hold data and the store
 // stops at the last real column.  Instantiations of their own, so that the loops of the full-width kernels stay compile-time.
+// They also take full-width tensors of fewer than 128 rows.  The probabilities of these shapes are kept to 16 bits of
+// mantissa, as two bf16 terms in the 128 columns that S leaves (P V is two products): the CUDA-core kernels that had these
+// shapes before computed P in fp32, and one bf16 term would put O 2.0e-3 off 64 bits where the rounding of O itself is 1.6e-3.
 template <int D, bool PAD = false>
 __global__ void __launch_bounds__(384, 1)
 fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -276,6 +279,11 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           for (int kk = 0; kk < T::BN / 16; ++kk)
             umma_ts(tmem_base + 256 + t * D, tmem_base + t * 128 + kk * 8, sdesc_advance(dv, kk * 2048), IDESC_PV,
                     (!first || kk > 0) ? 1u : 0u);
+          if (PAD) {   // the low terms of P
+#pragma unroll
+            for (int kk = 0; kk < T::BN / 16; ++kk)
+              umma_ts(tmem_base + 256 + t * D, tmem_base + t * 128 + 64 + kk * 8, sdesc_advance(dv, kk * 2048), IDESC_PV, 1u);
+          }
         };
         bool ok = true;
         uint32_t g0 = 0;               // ring slot counter of the current item's key tile 0
@@ -438,7 +446,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          uint32_t pk[16];
+          uint32_t pk[16], pl[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             const float p0 = ex2(fmaf(__uint_as_float(r[c * 32 + i + 0]), sl2, neg_m));
@@ -451,8 +459,13 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             l3 += p3;
             pk[(i >> 1)] = pack_bf16(p0, p1);
             pk[(i >> 1) + 1] = pack_bf16(p2, p3);
+            if (PAD) {
+              pl[(i >> 1)] = pack_bf16_rest(pk[(i >> 1)], p0, p1);
+              pl[(i >> 1) + 1] = pack_bf16_rest(pk[(i >> 1) + 1], p2, p3);
+            }
           }
           tmem_st_x16(t_s + c * 16, pk);
+          if (PAD) tmem_st_x16(t_s + 64 + c * 16, pl);
         }
         l_sum += (l0 + l1) + (l2 + l3);
         tmem_wait_st();

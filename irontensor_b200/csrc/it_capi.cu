@@ -1146,8 +1146,8 @@ static it_status attention_fwd_impl(it_ctx* ctx, it_stream* stream, it_dtype dty
   it::TensorStrides skv = strides_kv(bshd, H, Hkv, S, D);
   it::TensorStrides sq = sv;
   if (qkv_row != 0) {   // q, k and v are column ranges of one [batch, seq, qkv_row] buffer
-    if (!use_sm100_path(dtype, S, D))
-      return fail(IT_ERR_UNSUPPORTED_SHAPE, "the packed layout needs bf16, a head_dim that is a multiple of 8 from 16 on, and seq >= 48");
+    if (dtype != IT_BF16 || (D != 64 && D != 128) || S < 128)
+      return fail(IT_ERR_UNSUPPORTED_SHAPE, "the packed layout needs bf16, head_dim 64 or 128 and seq >= 128");
     sq.row = skv.row = qkv_row;
     sq.batch = skv.batch = qkv_row * S;
   }
@@ -1155,8 +1155,9 @@ static it_status attention_fwd_impl(it_ctx* ctx, it_stream* stream, it_dtype dty
     // IT_FWD_KERNEL=pp|two in the environment overrides the choice (A/B runs).
     const char* force = getenv("IT_FWD_KERNEL");
     const bool pp = (force != nullptr) ? (force[0] == 'p') : fwd_one_tile(ctx->sm_count, D, BH, S, causal);
-    auto launch = D == 128 ? (pp ? launch_fwd_sm100<128, true> : launch_fwd_sm100<128, false>)
-                  : D == 64 ? (pp ? launch_fwd_sm100<64, true> : launch_fwd_sm100<64, false>)
+    const bool full = (D == 128 || D == 64) && S >= 128;   // else the PAD instantiations
+    auto launch = full && D == 128 ? (pp ? launch_fwd_sm100<128, true> : launch_fwd_sm100<128, false>)
+                  : full ? (pp ? launch_fwd_sm100<64, true> : launch_fwd_sm100<64, false>)
                   : D > 64 ? launch_fwd_sm100<128, false, true> : launch_fwd_sm100<64, false, true>;
     return launch(ctx, stream, B, H, S, D, causal != 0, q, k, v, o, lse, sv, skv, sq);
   }
@@ -1236,13 +1237,14 @@ static it_status attention_bwd_impl(it_ctx* ctx, it_stream* stream, it_dtype dty
   it::TensorStrides skv = strides_kv(bshd, H, Hkv, S, D);
   it::TensorStrides sq = sv;
   if (qkv_row != 0) {   // q, k, v (and dq, dk, dv) are column ranges of one [batch, seq, qkv_row] buffer each
-    if (!use_sm100_path(dtype, S, D))
-      return fail(IT_ERR_UNSUPPORTED_SHAPE, "the packed layout needs bf16, a head_dim that is a multiple of 8 from 16 on, and seq >= 48");
+    if (dtype != IT_BF16 || (D != 64 && D != 128) || S < 128)
+      return fail(IT_ERR_UNSUPPORTED_SHAPE, "the packed layout needs bf16, head_dim 64 or 128 and seq >= 128");
     sq.row = skv.row = qkv_row;
     sq.batch = skv.batch = qkv_row * S;
   }
   if (!cuda_cores && use_sm100_path(dtype, S, D)) {
-    auto launch = D == 128 ? launch_bwd_sm100<128> : D == 64 ? launch_bwd_sm100<64>
+    const bool full = (D == 128 || D == 64) && S >= 128;   // else the PAD instantiations
+    auto launch = full && D == 128 ? launch_bwd_sm100<128> : full ? launch_bwd_sm100<64>
                   : D > 64 ? launch_bwd_sm100<128, true> : launch_bwd_sm100<64, true>;
     return launch(ctx, stream->s, B, H, S, D, causal != 0, q, k, v, o, d_o, lse, dq, dk, dv, ws, w, sv, skv, rf, sq);
   }

@@ -401,6 +401,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
+// What rounding to bf16 took from lo and hi, packed the same way: the second of two bf16 terms.
+__device__ __forceinline__ uint32_t pack_bf16_rest(uint32_t packed, float lo, float hi) {
+  return pack_bf16(lo - __uint_as_float(packed << 16), hi - __uint_as_float(packed & 0xFFFF0000u));
+}
 // Byte offset of element (row, col) in a [rows x 64] bf16 block stored with the 128-byte swizzle
 // (the layout TMA writes and the UMMA descriptors above read); the block base is 1024-byte aligned.
 __device__ __forceinline__ uint32_t swz128_offset(int row, int col) {

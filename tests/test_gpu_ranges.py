@@ -295,3 +295,31 @@ def test_bf16_backward_split_over_a_cluster(it_ctx, monkeypatch, split, B, S, H,
     for got, want, name in ((dq, rdq, "dQ"), (dk, rdk, "dK"), (dv, rdv, "dV")):
         scale = math.sqrt(H // Hkv) if name in ("dK", "dV") else 1.0   # sums over the group's heads
         check_bf16(got.to_f32_host() / scale, want / scale, f"{(B, S, H, Hkv, D)} {name}")
+
+
+@pytest.mark.parametrize("S,D", [(100, 64), (127, 128), (300, 96), (200, 32), (260, 40)])
+def test_bf16_padded_shapes_keep_fp32_probabilities(it_ctx, S, D):
+    """Shapes of the padded tiles against 64 bits.  Rounding a result to bf16 costs 1.66e-3 of its norm (2^-9 of each element,
+    uniform over the binades); delta, computed from the rounded O, adds to dQ and dK (1.9e-3 in all).  One bf16 term for P and
+    dS would add as much again (2.0e-3, 2.3e-3 and 3.0e-3)."""
+    import torch
+    from irontensor_b200 import Precision, Tensor, attention_backward_recompute, flash_attention
+    q, k, v, d_o = [torch.from_numpy(t.reshape(2, 8, S, D)).cuda() for t in synth.attention_inputs(990 + S, 2, 8, S, D, bf16=True)]
+    tq, tk, tv, tdo = (Tensor(t.to(torch.bfloat16).reshape(-1), [2, 8, S, D], Precision.BF16) for t in (q, k, v, d_o))
+    o = flash_attention(tq, tk, tv, True)
+    got = (o,) + tuple(attention_backward_recompute(tdo, tq, tk, tv, o, o.lse))
+    q, k, v, d_o = (t.double() for t in (q, k, v, d_o))
+    s = (q @ k.mT / math.sqrt(D)).masked_fill(~torch.ones(S, S, dtype=torch.bool, device="cuda").tril(), -math.inf)
+    p = torch.softmax(s, -1)
+    ds = p * (d_o @ v.mT - (d_o * (p @ v)).sum(-1, keepdim=True))
+    want = (p @ v, ds @ k / math.sqrt(D), ds.mT @ q / math.sqrt(D), p.mT @ d_o)
+    for g, w, name, bound in zip(got, want, ("O", "dQ", "dK", "dV"), (1.75e-3, 2.1e-3, 2.1e-3, 1.75e-3)):
+        err = ((g.torch().reshape(w.shape).double() - w).norm() / w.norm()).item()
+        assert err <= bound, f"{name}: {err:.2e}"
+
+
+def test_packed_layout_refuses_other_shapes(it_ctx):
+    from irontensor_b200 import Tensor, attention_packed
+    for S, D in ((100, 64), (200, 96)):
+        with pytest.raises(_lib.ITError, match="head_dim 64 or 128 and seq >= 128"):
+            attention_packed(Tensor.from_f32_as_bf16(np.zeros(S * 6 * D, np.float32), [1, S, 6 * D]), 2, 2, D, True)
