@@ -1,10 +1,10 @@
-// Causal / full scaled-dot-product attention forward for bf16 inputs on sm_100a, long sequences:
+// Causal / full scaled-dot-product attention forward for bf16 inputs on sm_100a:
 // one query tile per CTA, the two softmax groups alternating over KEY tiles.
 //
 // Replaces, for bf16 tensors, the reference project's forward kernels
 // (src/shaders/flash_attention.metal:45-163 online softmax; :167-223 exact softmax) and adds the
-// per-row log-sum-exp output the fused backward needs.  The launcher picks this kernel for head_dim 128
-// and 5120 keys or more; fa_fwd_sm100.cuh (two query tiles per CTA) covers the rest.
+// per-row log-sum-exp output the fused backward needs.  The launcher picks between this kernel and
+// fa_fwd_sm100.cuh (two query tiles per CTA) by how the launch fills the GPU (fwd_one_tile in it_capi.cu).
 //
 // One CTA owns one 128-row query tile of one (batch, head) slice and walks its key tiles once:
 //   warp 0      : TMA producer  - the Q tile once, then a ring of K tiles (128-byte swizzle)

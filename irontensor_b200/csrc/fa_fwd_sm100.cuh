@@ -1,6 +1,6 @@
 // Causal / full scaled-dot-product attention forward for bf16 inputs on sm_100a: two query tiles per
-// CTA sharing each K/V tile.  The launcher uses it for head_dim 64 and for sequences below 5120 keys
-// (fa_fwd_pp_sm100.cuh takes head_dim 128 from 5120 keys on).
+// CTA sharing each K/V tile.  The launcher picks between it and fa_fwd_pp_sm100.cuh (one
+// query tile per CTA) by how the launch fills the GPU (fwd_one_tile in it_capi.cu).
 //
 // Replaces, for bf16 tensors (head_dim 64 or 128, and any other multiple of 8 up to 128 zero-padded to those), the reference project's forward kernels
 // (src/shaders/flash_attention.metal:45-163 online softmax; :167-223 exact softmax) and adds the

@@ -71,8 +71,9 @@ struct it_ctx {
   std::atomic<uint64_t> launches{0};
   // Work-item counters of the forward kernel that walks its items in a loop: one int per live stream object (launches
   // on one stream run one after the other, so a stream needs one counter), handed out from a pool allocated with the
-  // context so that wrapping a stream calls nothing a stream capture forbids.
-  static constexpr int WORK_SLOTS = 4096;
+  // context so that wrapping a stream calls nothing a stream capture forbids; and behind those one per captured launch.
+  static constexpr int WORK_SLOTS = 4096, CAPTURE_SLOTS = 61440;
+  std::atomic<int> captured{0};
   int* d_work_pool = nullptr;
   std::mutex work_mutex;
   std::vector<int> work_free;
@@ -94,6 +95,11 @@ int* take_work_slot(it_ctx* ctx) {
     return ctx->d_work_pool + i;
   }
   return ctx->work_next < it_ctx::WORK_SLOTS ? ctx->d_work_pool + ctx->work_next++ : nullptr;
+}
+int* take_capture_slot(it_ctx* ctx) {
+  if (ctx->d_work_pool == nullptr || ctx->captured >= it_ctx::CAPTURE_SLOTS) return nullptr;
+  const int i = ctx->captured++;
+  return i < it_ctx::CAPTURE_SLOTS ? ctx->d_work_pool + it_ctx::WORK_SLOTS + i : nullptr;
 }
 void give_work_slot(it_ctx* ctx, it_stream* stream) {
   if (ctx == nullptr || stream->d_work == nullptr) return;
@@ -444,10 +450,18 @@ it_status launch_fwd_sm100(it_ctx* ctx, it_stream* stream, int B, int H, int S, 
   if (!PP && grid > ctx->sm_count) {
     // One CTA per SM; each draws its next work item from a counter (one per stream: launches on a stream run one
     // after the other), which the launch leaves at zero.  IT_FWD_ONE_ITEM_PER_CTA=1 launches one CTA per item instead.
+    // A captured launch gets a counter of its own, for good: its graph may be replayed on any stream, beside eager launches of
+    // the capturing stream object or other graphs captured through it.
     const char* one = getenv("IT_FWD_ONE_ITEM_PER_CTA");
-    if (stream->d_work != nullptr && (one == nullptr || one[0] != '1')) {
-      stream->work_used = true;
-      p.work_counter = stream->d_work;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) {   // the legacy stream beside a capture: not captured itself
+      cudaGetLastError();
+      capture = cudaStreamCaptureStatusNone;
+    }
+    int* counter = capture == cudaStreamCaptureStatusNone ? stream->d_work : take_capture_slot(ctx);
+    if (counter != nullptr && (one == nullptr || one[0] != '1')) {
+      if (counter == stream->d_work) stream->work_used = true;
+      p.work_counter = counter;
       grid = ctx->sm_count;
     }
   }
@@ -953,8 +967,8 @@ it_status it_ctx_create(int device, it_ctx** out) {
   }
   c->encode = reinterpret_cast<EncodeTiledFn>(fn);
   if (cudaMalloc(&c->d_status, sizeof(int)) != cudaSuccess || cudaMemset(c->d_status, 0, sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&c->d_work_pool, it_ctx::WORK_SLOTS * sizeof(int)) != cudaSuccess ||
-      cudaMemset(c->d_work_pool, 0, it_ctx::WORK_SLOTS * sizeof(int)) != cudaSuccess ||
+      cudaMalloc(&c->d_work_pool, (it_ctx::WORK_SLOTS + it_ctx::CAPTURE_SLOTS) * sizeof(int)) != cudaSuccess ||
+      cudaMemset(c->d_work_pool, 0, (it_ctx::WORK_SLOTS + it_ctx::CAPTURE_SLOTS) * sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&c->h_status, sizeof(int)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->status_stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete c;
@@ -1731,7 +1745,7 @@ it_status it_attention_status_poll(it_ctx* ctx, it_stream* stream, int32_t* devi
   *device_status = word;
   if (*device_status != 0) {
     // a launch that gave up may not have made all its draws: the work-item counters start over as well
-    IT_CUDA(cudaMemsetAsync(ctx->d_work_pool, 0, it_ctx::WORK_SLOTS * sizeof(int), stream->s));
+    IT_CUDA(cudaMemsetAsync(ctx->d_work_pool, 0, (it_ctx::WORK_SLOTS + it_ctx::CAPTURE_SLOTS) * sizeof(int), stream->s));
     IT_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), stream->s));
     IT_CUDA(cudaStreamSynchronize(stream->s));
     return fail(IT_ERR_TIMEOUT, "a bounded wait inside a kernel ran out (device status %d)", *device_status);

@@ -323,3 +323,31 @@ def test_packed_layout_refuses_other_shapes(it_ctx):
     for S, D in ((100, 64), (200, 96)):
         with pytest.raises(_lib.ITError, match="head_dim 64 or 128 and seq >= 128"):
             attention_packed(Tensor.from_f32_as_bf16(np.zeros(S * 6 * D, np.float32), [1, S, 6 * D]), 2, 2, D, True)
+
+
+def test_captured_forwards_replay_on_any_stream(it_ctx):
+    """Two graphs captured through one stream, replayed side by side on two others and beside eager launches: a captured launch
+    has a work-item counter of its own."""
+    import torch
+    from irontensor_b200 import Precision, Tensor, flash_attention
+    B, H, S, D = 8, 16, 1024, 64   # 512 work items: more than SMs, so the launch draws from a counter
+    ts = [Tensor(torch.randn(B * H * S * D, device="cuda").to(torch.bfloat16), [B, H, S, D], Precision.BF16) for _ in range(6)]
+    want = [flash_attention(*ts[i:i + 3], True).torch().clone() for i in (0, 3)]
+    side, graphs, outs = torch.cuda.Stream(), [], []
+    for i in (0, 3):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            outs.append(flash_attention(*ts[i:i + 3], True))
+        graphs.append(g)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for _ in range(50):
+        for g, s in zip(graphs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+        with torch.cuda.stream(side):
+            eager = flash_attention(*ts[:3], True)
+    torch.cuda.synchronize()
+    assert it_ctx.poll_status() == 0
+    for o, w in zip(outs + [eager], want + want[:1]):
+        assert torch.equal(o.torch(), w)
