@@ -834,6 +834,12 @@ it_status launch_decode_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int Hkv
     // clusters that are all resident at once: one of 8 needs 8 free SMs in one GPC, and a second wave doubles the launch
     // (16 clusters of 8: 15.6 us for 1000 positions, 16 of 4: 9)
     while (c > 2 && base_ctas > max_clusters<D>(ctx, c)) c /= 2;
+    // Two waves of CTAs of which the second is less than half full: half as long CTAs run in three.  A wave costs 10 us besides, so
+    // from 64 tiles on: 160 (batch, K/V head) pairs of 8190 positions 106 -> 95 us at head_dim 64, 133 -> 123 at 128; 16000
+    // positions 196 -> 162 (64); 200 pairs 106 -> 97 and 137 -> 135.  4000 positions: 58 and 59, 72 and 73.  216 pairs at
+    // head_dim 128, where a CTA's share of the memory rate is the limit sooner: 142 and 148, so it ends at 200 there.  Fuller second
+    // waves and more of them lose (256 pairs, 8190 positions: 107 -> 127, 158 -> 173).
+    if (c == 1 && base_ctas > ctx->sm_count && 200 * base_ctas <= (D == 64 ? 300LL : 272LL) * ctx->sm_count && n_tiles >= 64) c = 2;
     tiles_per_split = (n_tiles + c - 1) / c;
   }
   n_splits = (n_tiles + tiles_per_split - 1) / tiles_per_split;

@@ -351,3 +351,20 @@ def test_captured_forwards_replay_on_any_stream(it_ctx):
     assert it_ctx.poll_status() == 0
     for o, w in zip(outs + [eager], want + want[:1]):
         assert torch.equal(o.torch(), w)
+
+
+@pytest.mark.parametrize("B,Hkv,kv_len,D", [(19, 8, 8150, 128), (37, 4, 8064, 64), (37, 6, 8190, 64)])
+def test_decode_of_a_second_wave_less_than_half_full(it_ctx, B, Hkv, kv_len, D):
+    """Long caches of 149 to 222 (batch, K/V head) pairs are split over clusters of two; against fp32 of the same bf16 values."""
+    import torch
+    from irontensor_b200 import Precision, Tensor, attention_decode
+    G, L = 2, 8192
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(s, generator=gen, device="cuda").to(torch.bfloat16) for s in ((B, Hkv * G, D), (B, L, Hkv, D), (B, L, Hkv, D)))
+    got = attention_decode(*(Tensor(t.reshape(-1), list(t.shape), Precision.BF16) for t in (q, k, v)), kv_len)
+    assert it_ctx.poll_status() == 0
+    for b in (0, B - 1):
+        s = torch.einsum("hgd,lhd->hgl", q[b].float().reshape(Hkv, G, D), k[b, :kv_len].float()) / math.sqrt(D)
+        want = torch.einsum("hgl,lhd->hgd", torch.softmax(s, -1), v[b, :kv_len].float()).reshape(Hkv * G, D)
+        o = got.torch().reshape(B, Hkv * G, D)[b].float()
+        assert (o - want).norm() <= 4e-3 * want.norm()   # bf16 output (1.7e-3) and bf16 probabilities (2e-3)
