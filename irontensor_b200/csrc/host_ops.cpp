@@ -4,7 +4,7 @@
 //
 // TensorBase is the storage behind irontensor_b200.Tensor: one torch tensor of the logical shape (device memory comes from
 // torch's caching allocator, on the current stream) and the optional `lse` side output.  Every op function here takes the plain
-// case -- tensors on the current device, shapes and precisions that fit together, nothing empty -- and returns None otherwise:
+// case -- packed tensors on the current device, shapes and precisions that fit together, nothing empty -- and returns None otherwise:
 // the Python function of the same name then raises the reference's assertion, or handles the case.
 // Workspaces are allocated per call (stream-ordered reuse is the allocator's), so calls on different streams or threads share
 // nothing.  The GIL is released around the C-ABI calls.
@@ -144,7 +144,7 @@ bool call(F&& f) {
 bool plain(PyObject* o, int64_t dim) {
   if (!is_tensor(o)) return false;
   const at::Tensor& t = ten(o);
-  return t.dim() == dim && t.is_cuda() && t.numel() > 0 && t.is_contiguous() &&
+  return (is_bf16(t) || t.scalar_type() == at::kFloat) && t.dim() == dim && t.is_cuda() && t.numel() > 0 && t.is_contiguous() &&
          t.get_device() == c10::cuda::current_device();
 }
 bool same(const at::Tensor& a, const at::Tensor& b) { return a.sizes() == b.sizes() && a.scalar_type() == b.scalar_type(); }
@@ -501,16 +501,33 @@ bool read_shape(PyObject* shape, c10::SmallVector<int64_t, 6>* dims, int64_t* nu
   Py_DECREF(seq);
   return !PyErr_Occurred();
 }
-PyObject* tensor_set(PyObject* o, PyObject* const* a, Py_ssize_t nargs) {   // torch tensor, logical shape
-  if (nargs != 2 || !THPVariable_Check(a[0])) {
-    PyErr_SetString(PyExc_TypeError, "a torch tensor and a shape are needed");
+// `t` as the declared precision's values: a tensor of that type itself, or integers of its width, or bytes, that carry its
+// bits.  Anything else would be read at a wrong width or as other numbers: undefined, with an exception set.
+at::Tensor as_declared(const at::Tensor& t, PyObject* precision) {
+  if (precision != g_fp32 && precision != g_bf16) {
+    PyErr_SetString(PyExc_TypeError, "the precision is Precision.FP32 or Precision.BF16");
+    return {};
+  }
+  const at::ScalarType want = precision == g_bf16 ? at::kBFloat16 : at::kFloat, have = t.scalar_type();
+  if (have == want) return t;
+  const bool bits = c10::isIntegralType(have, /*includeBool=*/false) && (t.itemsize() == 1 || t.itemsize() == (want == at::kFloat ? 4 : 2));
+  if (!bits) {
+    PyErr_Format(PyExc_TypeError, "a torch tensor of type %s does not hold %s values", c10::toString(have), precision == g_bf16 ? "BF16" : "FP32");
+    return {};
+  }
+  return t.view(want);
+}
+PyObject* tensor_set(PyObject* o, PyObject* const* a, Py_ssize_t nargs) {   // torch tensor, logical shape, precision
+  if (nargs != 3 || !THPVariable_Check(a[0])) {
+    PyErr_SetString(PyExc_TypeError, "a torch tensor, a shape and a precision are needed");
     return nullptr;
   }
   return guard([&]() -> PyObject* {
     c10::SmallVector<int64_t, 6> dims;
     int64_t numel;
     if (!read_shape(a[1], &dims, &numel)) return nullptr;
-    const at::Tensor& t = THPVariable_Unpack(a[0]);
+    const at::Tensor t = as_declared(THPVariable_Unpack(a[0]), a[2]);
+    if (!t.defined()) return nullptr;
     ten(o) = t.sizes() == at::IntArrayRef(dims) ? t : t.view(dims);
     Py_RETURN_NONE;
   });
@@ -525,7 +542,13 @@ PyObject* tensor_shape(PyObject* o, PyObject*) {
 PyObject* tensor_precision(PyObject* o, PyObject*) { return Py_NewRef(is_bf16(ten(o)) ? g_bf16 : g_fp32); }
 PyObject* tensor_numel(PyObject* o, PyObject*) { return PyLong_FromLongLong(ten(o).numel()); }
 PyObject* tensor_data_ptr(PyObject* o, PyObject*) {
-  return guard([&] { return PyLong_FromVoidPtr(ten(o).data_ptr()); });
+  return guard([&]() -> PyObject* {
+    if (!ten(o).is_contiguous()) {   // the kernels take packed rows, and an address does not tell
+      PyErr_SetString(PyExc_ValueError, "the tensor's storage is not contiguous");
+      return nullptr;
+    }
+    return PyLong_FromVoidPtr(ten(o).data_ptr());
+  });
 }
 PyObject* tensor_reshaped(PyObject* o, PyObject* shape) {   // the same memory under another shape; None if the sizes differ
   return guard([&]() -> PyObject* {

@@ -181,11 +181,12 @@ class Tensor(_host_ops.TensorBase):
     (src/tensor.rs:136-148); here it synchronises the stream and copies device -> host."""
 
     def __init__(self, data, shape, precision):
-        self._set(data, shape)    # `data`: a torch CUDA tensor of that many elements
+        # `data`: a torch CUDA tensor of that many elements, in the type of the precision or as integers or bytes with its bits
+        self._set(data, shape, precision)
 
     @property
     def _data(self):
-        return self.torch().view(-1)
+        return self.torch().reshape(-1)
 
     # -- constructors (src/tensor.rs:63-118, 205-240)
     @staticmethod

@@ -1,0 +1,45 @@
+"""The Tensor object itself, on CPU: what it takes for its storage, and what it hands out.  (The ops need a GPU; the object does
+not, as long as the native host side is built.)"""
+import pytest
+import torch
+
+from irontensor_b200 import Precision, Tensor, _lib
+
+pytestmark = pytest.mark.skipif(isinstance(_lib.host_ops(), _lib._Missing), reason="_host_ops.so is not built")
+FP32, BF16 = Precision.FP32, Precision.BF16
+
+
+# The declared precision decides what the bits are; integers of the same width, or bytes, carry them.
+@pytest.mark.parametrize("stored,precision,held", [
+    (torch.float32, FP32, torch.float32), (torch.int32, FP32, torch.float32), (torch.uint32, FP32, torch.float32),
+    (torch.bfloat16, BF16, torch.bfloat16), (torch.int16, BF16, torch.bfloat16), (torch.uint16, BF16, torch.bfloat16),
+])
+def test_bits_of_the_declared_precision(stored, precision, held):
+    values = torch.arange(12, dtype=torch.float32).to(held)
+    t = Tensor(values.view(stored), [3, 4], precision)
+    assert t.precision() is precision and t.byte_size() == 12 * precision.byte_size()
+    assert t.torch().dtype == held and torch.equal(t.torch(), values.view(3, 4))
+    assert t.data_ptr() % 4 == 0 and t.shape() == [3, 4]
+    b = Tensor(values.view(torch.uint8), [3, 4], precision)
+    assert b.precision() is precision and torch.equal(b.torch(), values.view(3, 4))
+
+
+@pytest.mark.parametrize("stored,precision", [
+    (torch.float16, FP32), (torch.float16, BF16), (torch.float64, FP32), (torch.float32, BF16), (torch.bfloat16, FP32),
+    (torch.int16, FP32), (torch.int32, BF16), (torch.int64, FP32), (torch.bool, FP32), (torch.complex64, FP32),
+])
+def test_other_types_are_refused(stored, precision):
+    with pytest.raises(TypeError):
+        Tensor(torch.zeros(4, dtype=stored), [4], precision)
+    with pytest.raises(TypeError):
+        Tensor(torch.zeros(4), [4], None)
+
+
+def test_storage_that_is_not_packed_has_no_address():
+    """The kernels know packed rows only: a strided view may be held and read back, but no op gets its address."""
+    x = torch.arange(12, dtype=torch.float32).view(3, 4)
+    t = Tensor(x[:, :2], [3, 2], FP32)
+    assert torch.equal(t.torch(), x[:, :2])
+    assert torch.equal(t._data, x[:, :2].reshape(-1))
+    with pytest.raises(ValueError):
+        t.data_ptr()
