@@ -43,3 +43,24 @@ def test_storage_that_is_not_packed_has_no_address():
     assert torch.equal(t._data, x[:, :2].reshape(-1))
     with pytest.raises(ValueError):
         t.data_ptr()
+
+
+def test_torch_views_do_not_share_their_form():
+    """What torch() hands out, and what the constructor was given, share memory with the object and nothing else: changing their
+    shape or strides in place leaves the object as it was."""
+    x = torch.arange(6, dtype=torch.float32).view(2, 3)
+    t = Tensor(x, [2, 3], FP32)
+    x.t_()
+    assert t.shape() == [2, 3] and t.torch().stride() == (3, 1)
+    y = t.torch()
+    y.t_()
+    y[0, 1] = 40.0
+    assert t.shape() == [2, 3] and t.torch().is_contiguous() and t.torch()[1, 0] == 40.0 and x[0, 1] == 40.0
+    t.torch().unsqueeze_(0)
+    assert t.shape() == [2, 3]
+    w = torch.ones(4, requires_grad=True)      # a view in autograd's sense too
+    Tensor(w, [4], FP32).torch().sum().backward()
+    assert torch.equal(w.grad, torch.ones(4))
+    v = t.torch()._version
+    t.torch().add_(1.0)
+    assert t.torch()._version == v + 1         # one version counter: autograd sees writes through any of them
