@@ -188,6 +188,16 @@ class Tensor(_host_ops.TensorBase):
     def _data(self):
         return self.torch().reshape(-1)
 
+    # copy.copy shares the storage, copy.deepcopy and pickle copy it
+    def __getstate__(self):
+        return dict(self.__dict__, _data=self.torch(), _shape=self.shape(), _precision=self.precision(), lse=self.lse)
+
+    def __setstate__(self, state):
+        state = dict(state)
+        self._set(state.pop("_data"), state.pop("_shape"), state.pop("_precision"))
+        self.lse = state.pop("lse")
+        self.__dict__.update(state)
+
     # -- constructors (src/tensor.rs:63-118, 205-240)
     @staticmethod
     def zeros(shape, precision=Precision.FP32):

@@ -1,5 +1,8 @@
 """The Tensor object itself, on CPU: what it takes for its storage, and what it hands out.  (The ops need a GPU; the object does
 not, as long as the native host side is built.)"""
+import copy
+import pickle
+
 import pytest
 import torch
 
@@ -64,3 +67,24 @@ def test_torch_views_do_not_share_their_form():
     v = t.torch()._version
     t.torch().add_(1.0)
     assert t.torch()._version == v + 1         # one version counter: autograd sees writes through any of them
+
+
+def _lookalike(t, u):
+    return u is not t and u.precision() is t.precision() and u.shape() == t.shape() and torch.equal(u.torch(), t.torch())
+
+
+def test_copies_and_pickles():
+    t = Tensor(torch.arange(6, dtype=torch.float32).to(torch.bfloat16), [2, 3], BF16)
+    t.lse = Tensor(torch.zeros(2), [2], FP32)
+    t.note = "kept"
+    shallow = copy.copy(t)
+    assert _lookalike(t, shallow) and shallow.data_ptr() == t.data_ptr() and shallow.lse is t.lse and shallow.note == "kept"
+    deep = copy.deepcopy(t)
+    assert _lookalike(t, deep) and deep.data_ptr() != t.data_ptr()
+    assert _lookalike(t.lse, deep.lse) and deep.lse.data_ptr() != t.lse.data_ptr() and deep.note == "kept"
+    back = pickle.loads(pickle.dumps(t))
+    assert _lookalike(t, back) and _lookalike(t.lse, back.lse) and back.lse.lse is None and back.note == "kept"
+    # the state of a pickle written when the object was all Python: a flat buffer, shape, precision and lse as attributes
+    old = Tensor.__new__(Tensor)
+    old.__setstate__({"_data": t.torch().reshape(-1), "_shape": [2, 3], "_precision": BF16, "lse": None})
+    assert _lookalike(t, old) and old.lse is None
