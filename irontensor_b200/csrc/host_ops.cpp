@@ -490,14 +490,16 @@ int tensor_clear(PyObject* o) {
   Py_CLEAR(reinterpret_cast<TensorObject*>(o)->lse);
   return 0;
 }
-bool read_shape(PyObject* shape, c10::SmallVector<int64_t, 6>* dims, int64_t* numel) {
+bool read_shape(PyObject* shape, c10::SmallVector<int64_t, 6>* dims, int64_t* numel) {   // numel: -1 where 64 bits do not hold it
   PyObject* seq = PySequence_Fast(shape, "a shape is a sequence of numbers");
   if (seq == nullptr) return false;
   *numel = 1;
+  bool over = false;
   for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq); ++i) {
     dims->push_back(PyLong_AsLongLong(PySequence_Fast_GET_ITEM(seq, i)));
-    *numel *= dims->back();
+    over = __builtin_mul_overflow(*numel, dims->back(), numel) || over;
   }
+  if (over) *numel = -1;
   Py_DECREF(seq);
   return !PyErr_Occurred();
 }
@@ -509,20 +511,23 @@ at::Tensor alias_of(const at::Tensor& t) {
                                                                      /*allow_tensor_metadata_change=*/true));
 }
 // `t` as the declared precision's values: a tensor of that type itself, or integers of its width, or bytes, that carry its
-// bits.  Anything else would be read at a wrong width or as other numbers: undefined, with an exception set.
-at::Tensor as_declared(const at::Tensor& t, PyObject* precision) {
+// bits.  Anything else would be read at a wrong width or as other numbers: undefined, with an exception set.  Of a packed
+// buffer longer than `numel` values, its beginning.
+at::Tensor as_declared(const at::Tensor& t, PyObject* precision, int64_t numel) {
   if (precision != g_fp32 && precision != g_bf16) {
     PyErr_SetString(PyExc_TypeError, "the precision is Precision.FP32 or Precision.BF16");
     return {};
   }
   const at::ScalarType want = precision == g_bf16 ? at::kBFloat16 : at::kFloat, have = t.scalar_type();
-  if (have == want) return t;
   const bool bits = c10::isIntegralType(have, /*includeBool=*/false) && (t.itemsize() == 1 || t.itemsize() == (want == at::kFloat ? 4 : 2));
-  if (!bits) {
+  if (!bits && have != want) {
     PyErr_Format(PyExc_TypeError, "a torch tensor of type %s does not hold %s values", c10::toString(have), precision == g_bf16 ? "BF16" : "FP32");
     return {};
   }
-  return t.view(want);
+  const int64_t per_value = bits ? (want == at::kFloat ? 4 : 2) / t.itemsize() : 1;   // elements of t
+  const bool longer = numel >= 0 && t.numel() / per_value >= numel && t.numel() != numel * per_value && t.is_contiguous();
+  const at::Tensor part = longer ? t.view(-1).narrow(0, 0, numel * per_value) : t;
+  return bits ? part.view(want) : part;
 }
 PyObject* tensor_set(PyObject* o, PyObject* const* a, Py_ssize_t nargs) {   // torch tensor, logical shape, precision
   if (nargs != 3 || !THPVariable_Check(a[0])) {
@@ -533,7 +538,7 @@ PyObject* tensor_set(PyObject* o, PyObject* const* a, Py_ssize_t nargs) {   // t
     c10::SmallVector<int64_t, 6> dims;
     int64_t numel;
     if (!read_shape(a[1], &dims, &numel)) return nullptr;
-    const at::Tensor t = as_declared(THPVariable_Unpack(a[0]), a[2]);
+    const at::Tensor t = as_declared(THPVariable_Unpack(a[0]), a[2], numel);
     if (!t.defined()) return nullptr;
     ten(o) = t.sizes() == at::IntArrayRef(dims) ? alias_of(t) : t.view(dims);
     Py_RETURN_NONE;

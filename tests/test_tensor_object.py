@@ -88,3 +88,20 @@ def test_copies_and_pickles():
     old = Tensor.__new__(Tensor)
     old.__setstate__({"_data": t.torch().reshape(-1), "_shape": [2, 3], "_precision": BF16, "lse": None})
     assert _lookalike(t, old) and old.lse is None
+
+
+def test_a_buffer_may_be_longer_than_the_shape():
+    """A pool's block is handed over whole; the shape says how much of its beginning is the tensor."""
+    pool = torch.arange(20, dtype=torch.float32)
+    t = Tensor(pool, [2, 3], FP32)
+    assert t.shape() == [2, 3] and t.numel() == 6 and t.byte_size() == 24
+    assert t.data_ptr() == pool.data_ptr() and torch.equal(t.torch(), pool[:6].view(2, 3))
+    assert Tensor(pool.view(4, 5), [7], FP32).torch().tolist() == list(range(7))
+    assert Tensor(torch.zeros(9, dtype=torch.int16), [2, 4], BF16).shape() == [2, 4]
+    assert Tensor(torch.zeros(9, dtype=torch.uint8), [2, 2], BF16).shape() == [2, 2]
+    assert Tensor(pool, [0, 3], FP32).numel() == 0 and Tensor(pool, [], FP32).torch().item() == 0.0
+    for shape in ([3, 7], [-2, -3], [2 ** 40, 2 ** 40]):     # longer than the buffer, or no shape at all
+        with pytest.raises(RuntimeError):
+            Tensor(pool, shape, FP32)
+    with pytest.raises(RuntimeError):          # a strided buffer has no such beginning
+        Tensor(pool.view(4, 5)[:, :3], [2, 3], FP32)
