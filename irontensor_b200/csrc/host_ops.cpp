@@ -544,33 +544,48 @@ PyObject* tensor_set(PyObject* o, PyObject* const* a, Py_ssize_t nargs) {   // t
     Py_RETURN_NONE;
   });
 }
+// An accessor: `f` on the held tensor.  ValueError for an object that holds none (Tensor.__new__ alone); nothing throws past it.
+template <typename F>
+PyObject* on_held(PyObject* o, F&& f) {
+  if (!ten(o).defined()) {
+    PyErr_SetString(PyExc_ValueError, "the Tensor holds no storage: its constructor has not run");
+    return nullptr;
+  }
+  return guard([&]() -> PyObject* { return f(ten(o)); });
+}
 PyObject* tensor_torch(PyObject* o, PyObject*) {
-  return guard([&] { return THPVariable_Wrap(alias_of(ten(o))); });
+  return on_held(o, [](const at::Tensor& t) { return THPVariable_Wrap(alias_of(t)); });
 }
 PyObject* tensor_shape(PyObject* o, PyObject*) {
-  const auto s = ten(o).sizes();
-  PyObject* r = PyList_New(static_cast<Py_ssize_t>(s.size()));
-  for (size_t i = 0; r != nullptr && i < s.size(); ++i) PyList_SET_ITEM(r, i, PyLong_FromLongLong(s[i]));
-  return r;
+  return on_held(o, [](const at::Tensor& t) {
+    const auto s = t.sizes();
+    PyObject* r = PyList_New(static_cast<Py_ssize_t>(s.size()));
+    for (size_t i = 0; r != nullptr && i < s.size(); ++i) PyList_SET_ITEM(r, i, PyLong_FromLongLong(s[i]));
+    return r;
+  });
 }
-PyObject* tensor_precision(PyObject* o, PyObject*) { return Py_NewRef(is_bf16(ten(o)) ? g_bf16 : g_fp32); }
-PyObject* tensor_numel(PyObject* o, PyObject*) { return PyLong_FromLongLong(ten(o).numel()); }
+PyObject* tensor_precision(PyObject* o, PyObject*) {
+  return on_held(o, [](const at::Tensor& t) { return Py_NewRef(is_bf16(t) ? g_bf16 : g_fp32); });
+}
+PyObject* tensor_numel(PyObject* o, PyObject*) {
+  return on_held(o, [](const at::Tensor& t) { return PyLong_FromLongLong(t.numel()); });
+}
 PyObject* tensor_data_ptr(PyObject* o, PyObject*) {
-  return guard([&]() -> PyObject* {
-    if (!ten(o).is_contiguous()) {   // the kernels take packed rows, and an address does not tell
+  return on_held(o, [](const at::Tensor& t) -> PyObject* {
+    if (!t.is_contiguous()) {   // the kernels take packed rows, and an address does not tell
       PyErr_SetString(PyExc_ValueError, "the tensor's storage is not contiguous");
       return nullptr;
     }
-    return PyLong_FromVoidPtr(ten(o).data_ptr());
+    return PyLong_FromVoidPtr(t.data_ptr());
   });
 }
 PyObject* tensor_reshaped(PyObject* o, PyObject* shape) {   // the same memory under another shape; None if the sizes differ
-  return guard([&]() -> PyObject* {
+  return on_held(o, [shape](const at::Tensor& t) -> PyObject* {
     c10::SmallVector<int64_t, 6> dims;
     int64_t numel;
     if (!read_shape(shape, &dims, &numel)) return nullptr;
-    if (numel != ten(o).numel()) Py_RETURN_NONE;
-    return wrap(ten(o).view(dims));
+    if (numel != t.numel()) Py_RETURN_NONE;
+    return wrap(t.view(dims));
   });
 }
 

@@ -1,7 +1,10 @@
 """The Tensor object itself, on CPU: what it takes for its storage, and what it hands out.  (The ops need a GPU; the object does
 not, as long as the native host side is built.)"""
 import copy
+import os
 import pickle
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -105,3 +108,19 @@ def test_a_buffer_may_be_longer_than_the_shape():
             Tensor(pool, shape, FP32)
     with pytest.raises(RuntimeError):          # a strided buffer has no such beginning
         Tensor(pool.view(4, 5)[:, :3], [2, 3], FP32)
+
+
+def test_an_object_without_storage_raises():
+    """Tensor.__new__ alone, as an unpickler or a subclass whose __init__ raised leaves it.  In a process of its own: a C++
+    exception that nobody translates ends the process."""
+    code = """
+from irontensor_b200 import Tensor
+t = Tensor.__new__(Tensor)
+for f in (t.shape, t.numel, t.data_ptr, t.precision, t.torch, lambda: t.view([1]), t.byte_size, t.__getstate__):
+    try:
+        f()
+    except ValueError:
+        print("raised")
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=os.path.dirname(os.path.dirname(__file__)))
+    assert (r.returncode, r.stdout.split()) == (0, ["raised"] * 8), r.stderr[-500:]
