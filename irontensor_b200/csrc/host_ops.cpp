@@ -150,20 +150,32 @@ bool plain(PyObject* o, int64_t dim) {
 bool same(const at::Tensor& a, const at::Tensor& b) { return a.sizes() == b.sizes() && a.scalar_type() == b.scalar_type(); }
 it_dtype dtype_of(const at::Tensor& t) { return is_bf16(t) ? IT_BF16 : IT_F32; }
 
-// Whole numbers and the like; false with an exception set.
+// Plain numbers and truth values of 32 bits; false, without an exception, for anything else, which the Python function then
+// converts or refuses.
 bool as_int(PyObject* o, int32_t* v) {
-  const long x = PyLong_AsLong(o);
+  if (!PyIndex_Check(o)) return false;
+  const Py_ssize_t x = PyNumber_AsSsize_t(o, nullptr);   // out of range: clipped
+  if (x == -1 && PyErr_Occurred()) {
+    PyErr_Clear();
+    return false;
+  }
   *v = static_cast<int32_t>(x);
-  if (x != *v && !PyErr_Occurred()) PyErr_SetString(PyExc_OverflowError, "argument does not fit 32 bits");
-  return !PyErr_Occurred();
+  return *v == x;
 }
 bool as_float(PyObject* o, float* v) {
-  *v = static_cast<float>(PyFloat_AsDouble(o));
-  return !PyErr_Occurred();
+  if (!PyFloat_Check(o) && !PyLong_Check(o)) return false;
+  const double x = PyFloat_AsDouble(o);
+  if (x == -1.0 && PyErr_Occurred()) {
+    PyErr_Clear();
+    return false;
+  }
+  *v = static_cast<float>(x);
+  return true;
 }
 bool as_bool(PyObject* o, int32_t* v) {
+  if (!PyLong_Check(o)) return false;
   *v = PyObject_IsTrue(o);
-  return *v >= 0;
+  return true;
 }
 
 #define IT_ARGS(n)                                                                                    \
@@ -200,7 +212,8 @@ PyObject* attention_fwd(PyObject* const* a, bool grouped) {
     }
     int32_t causal;
     Where w;
-    if (!as_bool(a[3], &causal) || !where(&w)) return nullptr;
+    if (!as_bool(a[3], &causal)) Py_RETURN_NONE;
+    if (!where(&w)) return nullptr;
     at::Tensor o = empty(w, q.sizes(), q.scalar_type()), lse = empty(w, {B, H, S}, at::kFloat);
     const void *pq = q.data_ptr(), *pk = k.data_ptr(), *pv = v.data_ptr();
     void* po = o.data_ptr();
@@ -251,7 +264,8 @@ PyObject* attention_bwd(PyObject* const* a, bool grouped) {
     float base = 0.f;
     const bool rope = a[7] != Py_None;
     Where w;
-    if (!as_bool(a[6], &causal) || (rope && (!as_float(a[7], &base) || !as_int(a[8], &pos))) || !where(&w)) return nullptr;
+    if (!as_bool(a[6], &causal) || (rope && (!as_float(a[7], &base) || !as_int(a[8], &pos)))) Py_RETURN_NONE;
+    if (!where(&w)) return nullptr;
     const it_dtype dt = dtype_of(q);
     size_t ws_bytes = 0;
     if (!raise_status(it_flash_attention_bwd_workspace_bytes(dt, B, H, S, D, &ws_bytes))) return nullptr;
@@ -298,8 +312,7 @@ PyObject* attention_decode(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const int64_t B = q.size(0), H = q.size(1), D = q.size(2), max_len = k.size(1), Hkv = k.size(2);
     if (!same(k, v) || q.scalar_type() != k.scalar_type() || k.size(0) != B || k.size(3) != D || H % Hkv != 0 || D > 128) Py_RETURN_NONE;
     int32_t kv_len;
-    if (!as_int(a[3], &kv_len)) return nullptr;
-    if (kv_len < 1 || kv_len > max_len) Py_RETURN_NONE;
+    if (!as_int(a[3], &kv_len) || kv_len < 1 || kv_len > max_len) Py_RETURN_NONE;
     Where w;
     if (!where(&w)) return nullptr;
     size_t ws_bytes = 0;
@@ -322,7 +335,7 @@ PyObject* attention_packed(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (!plain(a[0], 3)) Py_RETURN_NONE;
     const at::Tensor& x = ten(a[0]);
     int32_t H, Hkv, D, causal;
-    if (!as_int(a[1], &H) || !as_int(a[2], &Hkv) || !as_int(a[3], &D) || !as_bool(a[4], &causal)) return nullptr;
+    if (!as_int(a[1], &H) || !as_int(a[2], &Hkv) || !as_int(a[3], &D) || !as_bool(a[4], &causal)) Py_RETURN_NONE;
     const int64_t B = x.size(0), S = x.size(1);
     if (!is_bf16(x) || x.size(2) != (static_cast<int64_t>(H) + 2LL * Hkv) * D || H < 1 || Hkv < 1 || D < 1) Py_RETURN_NONE;
     Where w;
@@ -348,7 +361,7 @@ PyObject* attention_packed_backward(PyObject*, PyObject* const* a, Py_ssize_t na
     float base;
     if (!as_int(a[3], &H) || !as_int(a[4], &Hkv) || !as_int(a[5], &D) || !as_bool(a[6], &causal) || !as_float(a[7], &base) ||
         !as_int(a[8], &pos))
-      return nullptr;
+      Py_RETURN_NONE;
     const int64_t B = x.size(0), S = x.size(1);
     const int64_t want[4] = {B, S, H, D};
     if (!is_bf16(x) || !same(g, o) || !is_bf16(g) || g.sizes() != at::IntArrayRef(want, 4) || lse.numel() != B * H * S || H < 1 || Hkv < 1 ||
@@ -388,7 +401,8 @@ PyObject* rope_qk(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     float base;
     int32_t pos, inverse;
     Where w;
-    if (!as_float(a[2], &base) || !as_int(a[3], &pos) || !as_bool(a[4], &inverse) || !where(&w)) return nullptr;
+    if (!as_float(a[2], &base) || !as_int(a[3], &pos) || !as_bool(a[4], &inverse)) Py_RETURN_NONE;
+    if (!where(&w)) return nullptr;
     at::Tensor out[2] = {empty(w, q.sizes(), q.scalar_type()), two ? empty(w, ten(a[1]).sizes(), q.scalar_type()) : at::Tensor()};
     const void *pq = q.data_ptr(), *pk = two ? ten(a[1]).data_ptr() : nullptr;
     void *oq = out[0].data_ptr(), *ok = two ? out[1].data_ptr() : nullptr;
@@ -444,7 +458,7 @@ PyObject* qkv_rope_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     float base;
     if (!as_int(a[2], &H) || !as_int(a[3], &Hkv) || !as_int(a[4], &D) || !as_float(a[5], &base) || !as_int(a[6], &pos) ||
         !as_bool(a[7], &packed))
-      return nullptr;
+      Py_RETURN_NONE;
     const int64_t B = x.size(0), S = x.size(1), hidden = x.size(2), width = (static_cast<int64_t>(H) + 2LL * Hkv) * D;
     if (!is_bf16(x) || !is_bf16(wt) || H < 1 || Hkv < 1 || D < 2 || D > 128 || D % 2 != 0 || wt.size(0) != width || wt.size(1) != hidden)
       Py_RETURN_NONE;

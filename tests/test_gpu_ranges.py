@@ -368,3 +368,36 @@ def test_decode_of_a_second_wave_less_than_half_full(it_ctx, B, Hkv, kv_len, D):
         want = torch.einsum("hgl,lhd->hgd", torch.softmax(s, -1), v[b, :kv_len].float()).reshape(Hkv * G, D)
         o = got.torch().reshape(B, Hkv * G, D)[b].float()
         assert (o - want).norm() <= 4e-3 * want.norm()   # bf16 output (1.7e-3) and bf16 probabilities (2e-3)
+
+
+def test_arguments_that_are_no_plain_numbers(it_ctx):
+    """What the native host path does not take itself is converted, or refused, as the Python functions do it."""
+    import ctypes
+
+    import torch
+    from irontensor_b200 import Precision, Tensor, attention_decode, flash_attention, rope, rope_qk
+
+    def make(*shape):
+        return Tensor(torch.randn(shape, device="cuda"), list(shape), Precision.FP32)
+
+    x, k = make(1, 40, 2, 32), make(1, 40, 2, 32)
+    want = rope(x, 10000.0, 3).torch()
+    for base, offset in ((10000, 3), ("10000", 3), (np.float32(10000), np.int64(3)), (10000.0, 3.0), (10000.0, True + 2)):
+        assert torch.equal(rope(x, base, offset).torch(), want)
+        assert torch.equal(rope_qk(x, k, base, offset)[0].torch(), want)
+    with pytest.raises(TypeError):
+        rope(x, 10000.0, None)
+    want = flash_attention(x, x, x, True).torch()
+    for causal in (1, 2, np.True_, np.int32(1)):
+        assert torch.equal(flash_attention(x, x, x, causal).torch(), want)
+    for causal in (None, [1]):
+        with pytest.raises(TypeError):
+            flash_attention(x, x, x, causal)
+    q, cache = make(1, 2, 32), make(1, 40, 2, 32)
+    want = attention_decode(q, cache, cache, 7).torch()
+    assert torch.equal(attention_decode(q, cache, cache, np.int64(7)).torch(), want)
+    with pytest.raises(ctypes.ArgumentError):
+        attention_decode(q, cache, cache, 7.0)
+    for kv_len in (0, 41, 2 ** 40, -2 ** 70):
+        with pytest.raises(AssertionError):
+            attention_decode(q, cache, cache, kv_len)
