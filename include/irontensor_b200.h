@@ -53,10 +53,10 @@ it_status it_ctx_destroy(it_ctx* ctx);
 const char* it_last_error(void);
 
 /* CommandBatch::begin (src/command_batch.rs:174-182): a new in-order queue.
- * Every stream object (created or wrapped) holds one 4-byte work-item counter out of a pool of 4096 that the
+ * Every stream object (created or wrapped) holds one 8-byte work-item counter out of a pool of 4096 that the
  * context allocates once: where the bf16 forward has more work items than SMs it starts one CTA per SM, the CTAs
- * draw their next items from the counter, and the last draw leaves it at zero.  Launches through one stream object run one after the other, so one counter is
- * enough; a stream object created when the pool is empty gets none and its forwards start one CTA per item
+ * draw their next items from the counter, and the last one to finish drawing leaves it at zero, also in a launch
+ * that gave up.  Launches through one stream object run one after the other, so one counter is enough; a stream object created when the pool is empty gets none and its forwards start one CTA per item
  * (same results).  A forward captured into a CUDA graph takes a counter of its own for good (61440 per context, then
  * one CTA per item), so the graph may be replayed on any stream. */
 it_status it_stream_create(it_ctx* ctx, it_stream** out);

@@ -57,7 +57,7 @@ struct FwdParams {
   int head_dim;         // columns of the tensors: D, or fewer in the PAD instantiations
   int kv_group;         // query heads per K/V head (grouped-query attention; 1 otherwise)
   int group_slices;     // fa_fwd_sm100_kernel: slices per group of its work-item order
-  int* work_counter;    // fa_fwd_sm100_kernel: zero before and after the launch, when the grid is smaller than the number of work items; else null
+  int* work_counter;    // fa_fwd_sm100_kernel, when the grid is smaller than the number of work items (else null): draws made, CTAs through with drawing; zero before and after the launch
   // decode instantiation of the long-sequence kernel only (one new token against a key/value cache):
   int dec_tiles_per_split;   // key tiles per CTA
   int dec_n_splits;
@@ -228,8 +228,19 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   static_assert(128 * REGS_CTRL + 256 * REGS_SOFTMAX <= 384 * 168, "setmaxnreg budget exceeds the CTA's registers");
   if (warp < 4) {
     setmaxnreg_dec<REGS_CTRL>();
+    // This CTA draws no more.  Every CTA says so once, whether it ran all its items, gave up or did not start, and the last one
+    // leaves both counts at zero for the next launch: no memset stands in front of a launch, and none depends on how many
+    // draws the one before it made.
+    auto done_drawing = [&] {
+      __threadfence();
+      if (atomicAdd(prm.work_counter + 1, 1) == G - 1) {
+        __threadfence();
+        prm.work_counter[0] = 0;
+        prm.work_counter[1] = 0;
+      }
+    };
     if (bad_start) {
-      // nothing to do
+      if (warp == 3 && prm.work_counter != nullptr && elect_one()) done_drawing();
     } else if (warp == 0) {
       // ------------------------------------------------------------ TMA producer
       // (the first item's query tiles and key/value tile 0 were issued by this thread before the set-up barrier)
@@ -352,17 +363,14 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           if (n >= 2 && !mbar_wait(&sched_empty[n & 1], ((n >> 1) - 1) & 1, abort_flag, prm.status, DEV_ERR_TIMEOUT_EMPTY)) break;
           int idx = static_cast<int>(blockIdx.x);
           if (n > 0) {
-            const int drawn = atomicAdd(prm.work_counter, 1);
-            // n_items draws are made in all: n_items - G that find an item and the G that end the CTAs.  The last one leaves the
-            // counter at zero for the next launch on this stream, so no memset stands in front of the launch.
-            if (drawn == n_items - 1) *prm.work_counter = 0;
-            idx = G + drawn;
+            idx = G + atomicAdd(prm.work_counter, 1);
             if (idx >= n_items) idx = -1;
           }
           sched_item[n & 1] = idx;
           mbar_arrive(&sched_full[n & 1]);
           if (idx < 0) break;
         }
+        done_drawing();
       }
     }
   } else {

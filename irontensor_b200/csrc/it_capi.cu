@@ -69,10 +69,12 @@ struct it_ctx {
   cudaEvent_t ev[4][2] = {};
   bool ev_valid[4] = {false, false, false, false};
   std::atomic<uint64_t> launches{0};
-  // Work-item counters of the forward kernel that walks its items in a loop: one int per live stream object (launches
-  // on one stream run one after the other, so a stream needs one counter), handed out from a pool allocated with the
+  // Work-item counters of the forward kernel that walks its items in a loop: a pair of ints per live stream object (launches
+  // on one stream run one after the other, so a stream needs one pair), handed out from a pool allocated with the
   // context so that wrapping a stream calls nothing a stream capture forbids; and behind those one per captured launch.
+  // Zeroed once, here; every launch leaves its pair at zero, also one that gave up.
   static constexpr int WORK_SLOTS = 4096, CAPTURE_SLOTS = 61440;
+  static constexpr size_t WORK_BYTES = 2 * sizeof(int) * (WORK_SLOTS + CAPTURE_SLOTS);
   std::atomic<int> captured{0};
   int* d_work_pool = nullptr;
   std::mutex work_mutex;
@@ -92,20 +94,20 @@ int* take_work_slot(it_ctx* ctx) {
   if (!ctx->work_free.empty()) {
     const int i = ctx->work_free.back();
     ctx->work_free.pop_back();
-    return ctx->d_work_pool + i;
+    return ctx->d_work_pool + 2 * i;
   }
-  return ctx->work_next < it_ctx::WORK_SLOTS ? ctx->d_work_pool + ctx->work_next++ : nullptr;
+  return ctx->work_next < it_ctx::WORK_SLOTS ? ctx->d_work_pool + 2 * ctx->work_next++ : nullptr;
 }
 int* take_capture_slot(it_ctx* ctx) {
   if (ctx->d_work_pool == nullptr || ctx->captured >= it_ctx::CAPTURE_SLOTS) return nullptr;
   const int i = ctx->captured++;
-  return i < it_ctx::CAPTURE_SLOTS ? ctx->d_work_pool + it_ctx::WORK_SLOTS + i : nullptr;
+  return i < it_ctx::CAPTURE_SLOTS ? ctx->d_work_pool + 2 * (it_ctx::WORK_SLOTS + i) : nullptr;
 }
 void give_work_slot(it_ctx* ctx, it_stream* stream) {
   if (ctx == nullptr || stream->d_work == nullptr) return;
   if (stream->work_used) cudaStreamSynchronize(stream->s);   // a kernel in flight may still draw from the counter
   std::lock_guard<std::mutex> lock(ctx->work_mutex);
-  ctx->work_free.push_back(static_cast<int>(stream->d_work - ctx->d_work_pool));
+  ctx->work_free.push_back(static_cast<int>(stream->d_work - ctx->d_work_pool) / 2);
   stream->d_work = nullptr;
 }
 }  // namespace
@@ -973,8 +975,9 @@ it_status it_ctx_create(int device, it_ctx** out) {
   }
   c->encode = reinterpret_cast<EncodeTiledFn>(fn);
   if (cudaMalloc(&c->d_status, sizeof(int)) != cudaSuccess || cudaMemset(c->d_status, 0, sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&c->d_work_pool, (it_ctx::WORK_SLOTS + it_ctx::CAPTURE_SLOTS) * sizeof(int)) != cudaSuccess ||
-      cudaMemset(c->d_work_pool, 0, (it_ctx::WORK_SLOTS + it_ctx::CAPTURE_SLOTS) * sizeof(int)) != cudaSuccess ||
+      cudaMalloc(&c->d_work_pool, it_ctx::WORK_BYTES) != cudaSuccess ||
+      cudaMemset(c->d_work_pool, 0, it_ctx::WORK_BYTES) != cudaSuccess ||
+      cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess ||   // streams that do not wait for the legacy stream may be the first to launch
       cudaMallocHost(&c->h_status, sizeof(int)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->status_stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete c;
@@ -1750,8 +1753,6 @@ it_status it_attention_status_poll(it_ctx* ctx, it_stream* stream, int32_t* devi
   if (rc != IT_OK) return rc;
   *device_status = word;
   if (*device_status != 0) {
-    // a launch that gave up may not have made all its draws: the work-item counters start over as well
-    IT_CUDA(cudaMemsetAsync(ctx->d_work_pool, 0, (it_ctx::WORK_SLOTS + it_ctx::CAPTURE_SLOTS) * sizeof(int), stream->s));
     IT_CUDA(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), stream->s));
     IT_CUDA(cudaStreamSynchronize(stream->s));
     return fail(IT_ERR_TIMEOUT, "a bounded wait inside a kernel ran out (device status %d)", *device_status);

@@ -401,3 +401,31 @@ def test_arguments_that_are_no_plain_numbers(it_ctx):
     for kv_len in (0, 41, 2 ** 40, -2 ** 70):
         with pytest.raises(AssertionError):
             attention_decode(q, cache, cache, kv_len)
+
+
+def test_work_counters_survive_launches_that_did_not_start(it_ctx):
+    """A wait runs out on one stream while forwards that draw their work items from a counter run on another: some of their CTAs
+    start, some see the status word and do not, and the word is cleared while they run.  The next forward computes every row."""
+    import torch
+    from irontensor_b200 import Precision, Tensor, flash_attention
+    B, H, S, D = 8, 16, 1024, 64   # 512 work items
+    q, k, v = (Tensor(torch.randn(B * H * S * D, device="cuda").to(torch.bfloat16), [B, H, S, D], Precision.BF16) for _ in range(3))
+    want = flash_attention(q, k, v, True).torch().clone()
+    busy = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for i in range(6):
+        _lib.check(it_ctx.lib.it_selftest_wait_timeout(it_ctx.handle, it_ctx.stream(), 3 + i))
+        with torch.cuda.stream(busy):
+            for _ in range(150):
+                flash_attention(q, k, v, True)
+        with pytest.raises(_lib.ITError):
+            it_ctx.poll_status()          # of the other stream: clears the word under the busy one
+        with torch.cuda.stream(busy):
+            o = flash_attention(q, k, v, True)
+            o.torch().fill_(float("nan"))
+            busy.synchronize()
+            for _ in range(2):
+                o = flash_attention(q, k, v, True)
+        busy.synchronize()
+        assert it_ctx.poll_status() == 0
+        assert torch.equal(o.torch(), want)
