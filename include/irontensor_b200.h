@@ -57,8 +57,10 @@ const char* it_last_error(void);
  * context allocates once: where the bf16 forward has more work items than SMs it starts one CTA per SM, the CTAs
  * draw their next items from the counter, and the last one to finish drawing leaves it at zero, also in a launch
  * that gave up.  Launches through one stream object run one after the other, so one counter is enough; a stream object created when the pool is empty gets none and its forwards start one CTA per item
- * (same results).  A forward captured into a CUDA graph takes a counter of its own for good (61440 per context, then
- * one CTA per item), so the graph may be replayed on any stream. */
+ * (same results).  A forward captured into a CUDA graph takes a counter of its own (61440 per context, then one CTA
+ * per item), so the graph may be replayed on any stream; it is given back when the graph and the executable graphs
+ * made from it have been destroyed.  The counter belongs to the captured launch: do not run two executable graphs of
+ * one captured graph at the same time, and keep a graph that another executable graph was updated from. */
 it_status it_stream_create(it_ctx* ctx, it_stream** out);
 /* Adopts an existing cudaStream_t (0 = the legacy default stream) without owning it. */
 it_status it_stream_wrap(it_ctx* ctx, void* cuda_stream, it_stream** out);

@@ -13,6 +13,7 @@
 #include <cstring>
 #include <atomic>
 #include <cmath>
+#include <memory>
 #include <mutex>
 #include <new>
 
@@ -55,6 +56,25 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
 
 }  // namespace
 
+// The counters of captured launches.  A graph gives its launches' back when it and the executable graphs made from it are
+// gone, possibly after the context and from a thread of the driver's: hence shared ownership.
+struct CaptureSlots {
+  struct Held {   // what a graph holds
+    std::shared_ptr<CaptureSlots> slots;
+    int i = 0;
+    Held* next = nullptr;
+  };
+  std::mutex mutex;
+  int next = 0;
+  Held *oldest = nullptr, *newest = nullptr;   // given back: reused oldest first, and only once every one has been out
+  ~CaptureSlots() {
+    while (oldest != nullptr) {
+      Held* h = oldest;
+      oldest = h->next;
+      delete h;
+    }
+  }
+};
 struct it_ctx {
   int device = 0;
   int sm_count = 0;
@@ -75,7 +95,7 @@ struct it_ctx {
   // Zeroed once, here; every launch leaves its pair at zero, also one that gave up.
   static constexpr int WORK_SLOTS = 4096, CAPTURE_SLOTS = 61440;
   static constexpr size_t WORK_BYTES = 2 * sizeof(int) * (WORK_SLOTS + CAPTURE_SLOTS);
-  std::atomic<int> captured{0};
+  std::shared_ptr<CaptureSlots> captured;
   int* d_work_pool = nullptr;
   std::mutex work_mutex;
   std::vector<int> work_free;
@@ -98,10 +118,54 @@ int* take_work_slot(it_ctx* ctx) {
   }
   return ctx->work_next < it_ctx::WORK_SLOTS ? ctx->d_work_pool + 2 * ctx->work_next++ : nullptr;
 }
-int* take_capture_slot(it_ctx* ctx) {
-  if (ctx->d_work_pool == nullptr || ctx->captured >= it_ctx::CAPTURE_SLOTS) return nullptr;
-  const int i = ctx->captured++;
-  return i < it_ctx::CAPTURE_SLOTS ? ctx->d_work_pool + 2 * (it_ctx::WORK_SLOTS + i) : nullptr;
+// A counter for the launch that `stream` is about to capture, held by the graph under construction; null if there is none left.
+int* take_capture_slot(it_ctx* ctx, cudaStream_t stream) {
+  using Held = CaptureSlots::Held;
+  cudaStreamCaptureStatus status;
+  unsigned long long id;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(stream, &status, &id, &graph) != cudaSuccess || graph == nullptr) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  Held* held;
+  {
+    CaptureSlots& c = *ctx->captured;
+    std::lock_guard<std::mutex> lock(c.mutex);
+    if (c.next < it_ctx::CAPTURE_SLOTS) {
+      held = new (std::nothrow) Held;
+      if (held == nullptr) return nullptr;
+      held->i = c.next++;
+    } else if (c.oldest != nullptr) {
+      held = c.oldest;
+      c.oldest = held->next;
+      if (c.oldest == nullptr) c.newest = nullptr;
+    } else {
+      return nullptr;
+    }
+  }
+  held->slots = ctx->captured;
+  const int i = held->i;
+  auto give_back = [](void* p) {   // no CUDA calls here, and nothing that allocates
+    Held* h = static_cast<Held*>(p);
+    const std::shared_ptr<CaptureSlots> c = std::move(h->slots);
+    std::lock_guard<std::mutex> lock(c->mutex);
+    h->next = nullptr;
+    (c->newest != nullptr ? c->newest->next : c->oldest) = h;
+    c->newest = h;
+  };
+  cudaUserObject_t object;
+  if (cudaUserObjectCreate(&object, held, give_back, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+    cudaGetLastError();
+    give_back(held);
+    return nullptr;
+  }
+  if (cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    cudaGetLastError();
+    cudaUserObjectRelease(object, 1);   // gives the slot back
+    return nullptr;
+  }
+  return ctx->d_work_pool + 2 * (it_ctx::WORK_SLOTS + i);
 }
 void give_work_slot(it_ctx* ctx, it_stream* stream) {
   if (ctx == nullptr || stream->d_work == nullptr) return;
@@ -452,16 +516,17 @@ it_status launch_fwd_sm100(it_ctx* ctx, it_stream* stream, int B, int H, int S, 
   if (!PP && grid > ctx->sm_count) {
     // One CTA per SM; each draws its next work item from a counter (one per stream: launches on a stream run one
     // after the other), which the launch leaves at zero.  IT_FWD_ONE_ITEM_PER_CTA=1 launches one CTA per item instead.
-    // A captured launch gets a counter of its own, for good: its graph may be replayed on any stream, beside eager launches of
-    // the capturing stream object or other graphs captured through it.
+    // A captured launch gets a counter of its own for the life of its graph, which may be replayed on any stream, beside eager
+    // launches of the capturing stream object or other graphs captured through it.
     const char* one = getenv("IT_FWD_ONE_ITEM_PER_CTA");
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) {   // the legacy stream beside a capture: not captured itself
       cudaGetLastError();
       capture = cudaStreamCaptureStatusNone;
     }
-    int* counter = capture == cudaStreamCaptureStatusNone ? stream->d_work : take_capture_slot(ctx);
-    if (counter != nullptr && (one == nullptr || one[0] != '1')) {
+    const bool loop = one == nullptr || one[0] != '1';
+    int* counter = !loop ? nullptr : capture == cudaStreamCaptureStatusNone ? stream->d_work : take_capture_slot(ctx, s);
+    if (counter != nullptr) {
       if (counter == stream->d_work) stream->work_used = true;
       p.work_counter = counter;
       grid = ctx->sm_count;
@@ -964,6 +1029,12 @@ it_status it_ctx_create(int device, it_ctx** out) {
                 prop.minor);
   it_ctx* c = new (std::nothrow) it_ctx;
   if (c == nullptr) return fail(IT_ERR_CUDA, "out of host memory");
+  try {
+    c->captured = std::make_shared<CaptureSlots>();
+  } catch (...) {
+    delete c;
+    return fail(IT_ERR_CUDA, "out of host memory");
+  }
   c->device = device;
   c->sm_count = prop.multiProcessorCount;
   void* fn = nullptr;

@@ -429,3 +429,42 @@ def test_work_counters_survive_launches_that_did_not_start(it_ctx):
         busy.synchronize()
         assert it_ctx.poll_status() == 0
         assert torch.equal(o.torch(), want)
+
+
+def test_captured_forwards_give_their_counters_back(it_ctx):
+    """More captured forwards than there are counters, a graph at a time: the last one still gets one (its grid is the number of
+    SMs and not the number of work items)."""
+    import torch
+    from cuda.bindings import driver
+    from irontensor_b200 import Precision, Tensor, raw
+    B, H, S, D = 4, 16, 1024, 64   # 256 work items
+    q = Tensor(torch.randn(B * H * S * D, device="cuda").to(torch.bfloat16), [B, H, S, D], Precision.BF16)
+    o, lse = Tensor.empty([B, H, S, D], Precision.BF16), Tensor.empty([B, H, S], Precision.FP32)
+    per_graph, sms = 2000, torch.cuda.get_device_properties(0).multi_processor_count
+
+    def capture(n):
+        g = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(g):
+            for _ in range(n):
+                raw.fwd(_lib.IT_BF16, B, H, S, D, True, q.data_ptr(), q.data_ptr(), q.data_ptr(), o.data_ptr(), lse.data_ptr(), ctx=it_ctx)
+        return g
+
+    for i in range(34):            # 68000
+        g = capture(per_graph)
+        if i % 16 == 0:
+            g.instantiate()
+            g.replay()
+        torch.cuda.synchronize()
+        g.reset()
+    g = capture(1)
+    _, nodes, n = driver.cuGraphGetNodes(g.raw_cuda_graph(), 8)
+    err, params = driver.cuGraphKernelNodeGetParams(nodes[0])
+    assert n == 1 and int(err) == 0 and params.gridDimX == sms
+    raw.fwd(_lib.IT_BF16, B, H, S, D, True, q.data_ptr(), q.data_ptr(), q.data_ptr(), o.data_ptr(), lse.data_ptr(), ctx=it_ctx)
+    want = o.torch().clone()
+    o.torch().fill_(float("nan"))
+    g.instantiate()
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize()
+    assert it_ctx.poll_status() == 0 and torch.equal(o.torch(), want)
