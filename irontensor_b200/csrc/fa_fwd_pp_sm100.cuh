@@ -71,11 +71,15 @@ struct FwdPPTraits {
 // more splits leave unnormalised partial outputs with their reference maxima and row sums for
 // fa_decode_merge_kernel.  The cache is streamed by TMA through the same K and V rings, so
 // the op runs at the rate the memory system delivers tiles, not at the rate CUDA cores can issue loads.
-template <int D, bool DECODE = false>
+// TWO_TERMS: decode of fewer than 256 positions keeps P in two bf16 terms, 16 bits of mantissa, because the result's own rounding
+// is then most of its error: 1.7e-3 off 64 bits as with the fp32 probabilities of fa_decode_kernel, 2.1e-3 with one term (longer
+// caches have always had one).  At most two key tiles exist, so no third S needs their buffers, and the low terms take those.
+template <int D, bool DECODE = false, bool TWO_TERMS = false>
 __global__ void __launch_bounds__(384, 1)
 fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const FwdParams prm) {
   using T = FwdPPTraits<D>;
+  static_assert(DECODE || !TWO_TERMS, "the S buffers are free for the low terms in a decode of two tiles only");
   using namespace ptx;
   extern __shared__ __align__(1024) uint8_t smem[];
 
@@ -270,6 +274,11 @@ fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
           for (int kk = 0; kk < T::BN / 16; ++kk)
             umma_ts(tmem_base + T::COL_O, tmem_base + T::COL_P + kk * 8, sdesc_advance(dv, kk * 2048),
                     IDESC_PV, (j > 0 || kk > 0) ? 1u : 0u);
+          if (TWO_TERMS) {
+#pragma unroll
+            for (int kk = 0; kk < T::BN / 16; ++kk)
+              umma_ts(tmem_base + T::COL_O, tmem_base + T::COL_S + (j & 1) * 128 + kk * 8, sdesc_advance(dv, kk * 2048), IDESC_PV, 1u);
+          }
           umma_commit(&v_empty[st]);
         }
       }
@@ -394,6 +403,7 @@ fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
+          uint32_t pl[16];   // TWO_TERMS
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             const float p0 = ex2(fmaf(__uint_as_float(r[c * 32 + i + 0]), sl2, neg_m));
@@ -406,7 +416,12 @@ fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             l3 += p3;
             r[c * 16 + (i >> 1)] = pack_bf16(p0, p1);       // words [16c, 16c+16) were consumed by chunk c/2
             r[c * 16 + (i >> 1) + 1] = pack_bf16(p2, p3);
+            if (TWO_TERMS) {
+              pl[i >> 1] = pack_bf16_rest(r[c * 16 + (i >> 1)], p0, p1);
+              pl[(i >> 1) + 1] = pack_bf16_rest(r[c * 16 + (i >> 1) + 1], p2, p3);
+            }
           }
+          if (TWO_TERMS) tmem_st_x16(t_s + c * 16, pl);
         }
         l_sum += (l0 + l1) + (l2 + l3);
         if (!__all_sync(0xffffffffu, p_free)) {

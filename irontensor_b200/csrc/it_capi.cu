@@ -881,10 +881,11 @@ it_status launch_decode_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int Hkv
   const int G = H / Hkv;
   const int n_tiles = (kv_len + T::BN - 1) / T::BN;
   const long long base_ctas = static_cast<long long>(B) * Hkv;
-  auto kernel = it::fa_fwd_pp_sm100_kernel<D, true>;
+  auto kernel = kv_len < 256 ? it::fa_fwd_pp_sm100_kernel<D, true, true> : it::fa_fwd_pp_sm100_kernel<D, true>;
   static std::atomic<bool> attr_set[16];   // zero-initialised; setting an attribute twice is harmless
   if (!attr_set[ctx->device & 15]) {
-    IT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES));
+    IT_CUDA(cudaFuncSetAttribute(it::fa_fwd_pp_sm100_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES));
+    IT_CUDA(cudaFuncSetAttribute(it::fa_fwd_pp_sm100_kernel<D, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM_BYTES));
     attr_set[ctx->device & 15] = true;
   }
   // One CTA per SM runs at a time: split the keys until the GPU is covered.  Up to 8 splits (2, 4 or 8, down to one tile each:
@@ -1505,7 +1506,10 @@ it_status it_attention_decode(it_ctx* ctx, it_stream* stream, it_dtype dtype, in
   // B8 with 8, 512: 8.7 / 9.2; head_dim 64: one query head 206 / 179 at 16000 positions, groups of four, B8 with 8, 1000: 9.9 / 8.6.
   const int G = H / Hkv;
   const long long bytes = 4LL * B * Hkv * kv_len * D;   // both caches, bf16
-  const bool short_cache = kv_len < 64 || (G == 1 && (D == 64 || bytes <= 100LL << 20)) ||
+  // Below 256 positions, where the pipeline needs two bf16 terms of P, groups of up to four go to the CUDA cores whatever the batch
+  // (B64 with 8 K/V heads and 32 heads, 200 positions: head_dim 64 23.3 / 12.7, 128 28.1 / 21.8), larger ones do not (B64 with 2
+  // and 64: 5.9 / 25.5 and 7.1 / 39.0; B4 with 2 and 16: 6.6 / 5.7 and 7.2 / 6.7).
+  const bool short_cache = kv_len < (G <= 4 ? 256 : 64) || (G == 1 && (D == 64 || bytes <= 100LL << 20)) ||
                            (G <= 4 && kv_len <= (D == 64 ? 2500 : 1200) && bytes <= (D == 64 ? 16LL : 5LL) << 20);
   if (dtype == IT_BF16 && (D == 64 || D == 128) && G <= 128 && !short_cache)
     return D == 128 ? launch_decode_sm100<128>(ctx, stream->s, B, H, Hkv, kv_len, max_len, q, k_cache, v_cache, o, lse, ws)
