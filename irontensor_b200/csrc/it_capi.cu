@@ -1607,6 +1607,13 @@ it_status it_qkv_rope_fwd(it_ctx* ctx, it_stream* stream, int32_t B, int32_t S, 
     epi.v = base + (static_cast<long long>(H) + Hkv) * D;
     epi.ld_q = epi.ld_kv = out_dim;
   }
+  if (rope_base != 0.f) {   // asked of every call, although a handful of tokens needs no table: a caller finds out at any size
+    size_t need = 0;
+    it_qkv_rope_workspace_bytes(S, D, &need);
+    if (workspace == nullptr || workspace_bytes < need)
+      return fail(IT_ERR_INVALID_ARG, "workspace of %zu bytes needed, %zu given", need, workspace_bytes);
+    if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return fail(IT_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
+  }
   if (use_skinny(n, hidden, out_dim)) {
     it::SkinnyParams p{};
     p.x = static_cast<const __nv_bfloat16*>(x);
@@ -1627,11 +1634,6 @@ it_status it_qkv_rope_fwd(it_ctx* ctx, it_stream* stream, int32_t B, int32_t S, 
   }
   const float2* table = nullptr;
   if (rope_base != 0.f) {
-    size_t need = 0;
-    it_qkv_rope_workspace_bytes(S, D, &need);
-    if (workspace == nullptr || workspace_bytes < need)
-      return fail(IT_ERR_INVALID_ARG, "workspace of %zu bytes needed, %zu given", need, workspace_bytes);
-    if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return fail(IT_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
     const int cells = S * (D / 2);
     IT_CUDA(launch_dependent(it::rope_table_kernel, (cells + 255) / 256, 256, 0, stream->s, static_cast<float2*>(workspace), S, D / 2,
                              make_rope_freqs(D, rope_base, position_offset, true)));

@@ -486,3 +486,25 @@ def test_short_bf16_decode_rounds_its_result_only(it_ctx, B, H, Hkv, D, kv_len):
     qd, kd, vd = q.double().view(B, Hkv, H // Hkv, D), k[:, :kv_len].double(), v[:, :kv_len].double()
     want = torch.einsum("bhgk,bkhd->bhgd", (torch.einsum("bhgd,bkhd->bhgk", qd, kd) / D ** 0.5).softmax(-1), vd).reshape(B, H, D)
     assert ((got - want).norm() / want.norm()).item() < 1.85e-3
+
+
+@pytest.mark.parametrize("tokens", [1, 8, 40])
+def test_qkv_rope_asks_for_its_workspace_at_every_size(it_ctx, tokens):
+    """Few tokens need no table of sines; the call is refused all the same, as it is for more."""
+    import torch
+    H, D, hidden = 4, 64, 256
+    x = torch.zeros(tokens, hidden, dtype=torch.bfloat16, device="cuda")
+    w = torch.zeros(3 * H * D, hidden, dtype=torch.bfloat16, device="cuda")
+    outs = [torch.empty(tokens, H, D, dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+    ws = torch.empty(1 << 20, dtype=torch.uint8, device="cuda")
+
+    def call(base, pointer, nbytes):
+        return it_ctx.lib.it_qkv_rope_fwd(it_ctx.handle, it_ctx.stream(), 1, tokens, hidden, H, H, D, base, 0, x.data_ptr(), w.data_ptr(),
+                                          *(o.data_ptr() for o in outs), pointer, nbytes)
+
+    assert call(10000.0, None, 0) == _lib.IT_ERR_INVALID_ARG
+    assert call(10000.0, ws.data_ptr(), 8 * tokens) == _lib.IT_ERR_INVALID_ARG
+    assert call(10000.0, ws.data_ptr() + 16, 1 << 19) == _lib.IT_ERR_ALIGNMENT
+    assert call(10000.0, ws.data_ptr(), 1 << 20) == _lib.IT_OK
+    assert call(0.0, None, 0) == _lib.IT_OK       # without rotation there is nothing to ask for
+    assert it_ctx.poll_status() == 0
