@@ -111,7 +111,7 @@ class _Missing:
 
     def __init__(self, why):
         class TensorBase:
-            def __init__(self, *a):
+            def __new__(cls, *a, **k):
                 raise ImportError(why)
         self.TensorBase, self.setup = TensorBase, (lambda *a: None)
         self._why = why
@@ -122,8 +122,8 @@ class _Missing:
 
 def host_ops():
     """The native host side of the ops (csrc/host_ops.cpp)."""
-    import torch  # noqa: F401  (the extension links torch's libraries)
     try:
+        import torch  # noqa: F401  (the extension links torch's libraries)
         from . import _host_ops
         return _host_ops
     except ImportError as e:

@@ -184,3 +184,24 @@ def test_workspace_size_functions_of_the_widened_rows():
     assert lib.it_linear_fwd(None, None, 8, 8, 8, None, None, None) == _lib.IT_ERR_INVALID_ARG
     assert lib.it_rope_qk(None, None, _lib.IT_F32, 1, 1, 1, 1, 8, 10000.0, 0, 0, None, None, None, None) == _lib.IT_ERR_INVALID_ARG
     assert lib.it_attention_decode(None, None, _lib.IT_BF16, 1, 1, 1, 64, 1, 1, None, None, None, None, None, None, 0) == _lib.IT_ERR_INVALID_ARG
+
+
+def _python(code):
+    return subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=240, cwd=ROOT)
+
+
+def test_importing_the_package_does_not_import_torch():
+    """torch is needed on use; a tool that reads constants or builds the library does not wait for it."""
+    r = _python("import sys, irontensor_b200\nassert 'torch' not in sys.modules\n"
+                "from irontensor_b200 import _lib, synth, build\nassert _lib.IT_OK == 0 and 'torch' not in sys.modules\n"
+                "from irontensor_b200 import *\nimport irontensor_b200 as it\n"
+                "assert Tensor is it.Tensor is it.ops.Tensor and set(dir(it)) >= {'flash_attention', 'context', 'raw', 'ops', 'synth'}\n"
+                "try:\n    it.no_such_name\nexcept AttributeError:\n    print('fine')")
+    assert (r.returncode, r.stdout.strip()) == (0, "fine"), r.stderr[-800:]
+
+
+def test_without_torch_the_package_imports_and_use_raises():
+    r = _python("import sys\nsys.modules['torch'] = None\nimport irontensor_b200\nfrom irontensor_b200 import Tensor, Precision, flash_attention\n"
+                "for use in (lambda: Tensor(None, [1], Precision.FP32), lambda: flash_attention(1, 2, 3, True), lambda: Tensor.zeros([1])):\n"
+                "    try:\n        use()\n    except ImportError:\n        print('raised')")
+    assert (r.returncode, r.stdout.split()) == (0, ["raised"] * 3), r.stderr[-800:]
