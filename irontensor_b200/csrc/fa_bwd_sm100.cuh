@@ -581,7 +581,12 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       int g_m = g0, qi = q0, t_m = 0;
       for (int n = 0; n < n_iter; ++n, advance(g_m, qi, t_m)) {
         const int st = n & 1;
-        const bool diag = prm.causal && (qi == kt + t_m);   // the key tile's own query tile: keys after the query are masked
+        // Masked: in the key tile's own query tile the keys after the query, under the causal mask; without it, in the last key
+        // tile, the keys past the sequence (their scores are 0, and 2^-LSE of a query whose scores are all below -88 is
+        // infinite).  A query column below k_mask is masked.
+        const bool diag = prm.causal && (qi == kt + t_m);
+        const bool masked = diag || (!prm.causal && (kt + t_m + 1) * T::BM > S);
+        const int k_mask = diag ? k_local : (kt + t_m) * T::BM + k_local < S ? 0 : T::BN;
         const float* lse_s = reinterpret_cast<const float*>(smem + T::SMEM_LSE + st * 512) + half * 64;
         const float* dl_s = reinterpret_cast<const float*>(smem + T::SMEM_DELTA + st * 512) + half * 64;
         // lse/delta for this query tile ride on the Q barrier
@@ -599,12 +604,12 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), sl2, -l4.y));
             float p2 = ex2(fmaf(__uint_as_float(r[i + 2]), sl2, -l4.z));
             float p3 = ex2(fmaf(__uint_as_float(r[i + 3]), sl2, -l4.w));
-            if (diag) {   // key after the query: masked
+            if (masked) {
               const int qc = half * 64 + c * 16 + i;
-              if (k_local > qc + 0) p0 = 0.f;
-              if (k_local > qc + 1) p1 = 0.f;
-              if (k_local > qc + 2) p2 = 0.f;
-              if (k_local > qc + 3) p3 = 0.f;
+              if (k_mask > qc + 0) p0 = 0.f;
+              if (k_mask > qc + 1) p1 = 0.f;
+              if (k_mask > qc + 2) p2 = 0.f;
+              if (k_mask > qc + 3) p3 = 0.f;
             }
             p_keep[c * 8 + (i >> 1)] = pack_bf16(p0, p1);
             p_keep[c * 8 + (i >> 1) + 1] = pack_bf16(p2, p3);

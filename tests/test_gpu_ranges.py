@@ -508,3 +508,32 @@ def test_qkv_rope_asks_for_its_workspace_at_every_size(it_ctx, tokens):
     assert call(10000.0, ws.data_ptr(), 1 << 20) == _lib.IT_OK
     assert call(0.0, None, 0) == _lib.IT_OK       # without rotation there is nothing to ask for
     assert it_ctx.poll_status() == 0
+
+
+@pytest.mark.parametrize("dtype,D", [("bf16", 96), ("bf16", 64), ("bf16", 128), ("bf16", 40), ("fp32", 64), ("fp32", 32)])
+def test_keys_past_the_sequence_weigh_nothing(it_ctx, dtype, D):
+    """Without the causal mask the last key tile of a ragged sequence holds rows past it.  Where all scores of a query are very
+    low, 2^(0 - LSE) of such a row is infinite; it must not meet its zeros."""
+    import torch
+    from irontensor_b200 import Precision, Tensor, attention_backward_recompute, flash_attention
+    B, H, S = 1, 2, 200
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v, d_o = (torch.randn(B, H, S, D, generator=gen, device="cuda") for _ in range(4))
+    up = round(math.sqrt(200.0 * math.sqrt(D)))    # one column that puts all scores around -200
+    q[..., 0], k[..., 0] = up, -up
+    t = torch.bfloat16 if dtype == "bf16" else torch.float32
+    q, k, v, d_o = (x.to(t) for x in (q, k, v, d_o))
+    args = [Tensor(x, [B, H, S, D], Precision.BF16 if dtype == "bf16" else Precision.FP32) for x in (q, k, v, d_o)]
+    o = flash_attention(*args[:3], False)
+    grads = attention_backward_recompute(args[3], *args[:3], o, o.lse, causal=False)
+    assert it_ctx.poll_status() == 0
+    qd, kd, vd = (x.double().requires_grad_() for x in (q, k, v))
+    want = ((qd @ kd.transpose(-1, -2)) / D ** 0.5).softmax(-1) @ vd
+    want.backward(d_o.double())
+    for got, exact in zip((o,) + tuple(grads), (want.detach(), qd.grad, kd.grad, vd.grad)):
+        got = got.torch().double()
+        assert torch.isfinite(got).all()
+        # Column 0 of dQ and dK is a difference of large terms.  Scores of 200 are held to 200 * 2^-24 * log2(e) in fp32, and each
+        # of the D products rounds: probabilities are off by about 1e-4, whatever the type.
+        err = (got - exact)[..., 1:].norm() / exact[..., 1:].norm()
+        assert err.item() < (1e-2 if dtype == "bf16" else 5e-4)
