@@ -30,6 +30,7 @@
 #include "fa_fwd_f32_sm100.cuh"
 #include "rope.cuh"
 #include "sm100_ptx.cuh"
+#include "visible_pairs.cuh"
 
 namespace it {
 
@@ -131,6 +132,28 @@ __device__ __forceinline__ void f32_tile_store(uint8_t* planes, int t, const flo
     *reinterpret_cast<uint2*>(planes + 2 * PB + off) = make_uint2(l0, l1);
   }
   ptx::fence_proxy_async_smem();
+}
+
+// `width` columns of the finished row x_idx of dQ (KV: of dK or dV) from column `col` on, over the visible pairs alone.  For rows
+// that are not finite; see visible_pairs.cuh.  `bh`: the row's query slice (KV: the first of the group).
+template <bool KV>
+__device__ __noinline__ void fa_bwd_f32_visible(const BwdF32Params& prm, int bh, int x_idx, bool is_dv, int col, int width, float* out) {
+  const VisiblePairs<float> t{prm.q, prm.k, prm.v, prm.d_o, prm.st, prm.st_kv, prm.D, prm.scale_log2};
+  constexpr float LOG2E = 1.4426950408889634f;
+  for (int i = 0; i < width; i += 4) {
+    float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int h = 0; h < (KV ? prm.st_kv.group : 1); ++h) {
+      const size_t r = static_cast<size_t>(bh + h) * prm.S;
+      w = KV ? visible_dkv(t, !is_dv, bh + h, x_idx, x_idx, prm.S, col + i, prm.lse + r, LOG2E, prm.delta + r, w)
+             : visible_dq(t, bh, x_idx, x_idx + 1, col + i, prm.lse[r + x_idx] * LOG2E, prm.delta[r + x_idx]);
+    }
+    if (!is_dv) {
+      w = make_float4(w.x * prm.scale, w.y * prm.scale, w.z * prm.scale, w.w * prm.scale);
+      if (prm.rope_table != nullptr)
+        w = rotate_back(w, *reinterpret_cast<const float4*>(prm.rope_table + static_cast<size_t>(x_idx) * (prm.D >> 1) + ((col + i) >> 1)));
+    }
+    *reinterpret_cast<float4*>(out + i) = w;
+  }
 }
 
 // KV = true: dK/dV CTA; false: dQ CTA.  `tile` is the CTA's stationary tile, `slice` the query slice (dQ) or
@@ -334,6 +357,7 @@ __device__ __forceinline__ void fa_bwd_f32_body(const BwdF32Params& prm, uint8_t
         prev[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (n > 0 && x_idx < S && 4 * i < width) prev[i] = reinterpret_cast<const float4*>(out)[i];
       }
+      float z = 0.f;   // NaN: the row is not finite
       bool got = mbar_wait(y0_free, n & 1, abort_flag, prm.status, DEV_ERR_TIMEOUT_MMA);   // the tile's MMAs are complete
       got = __all_sync(0xffffffffu, got);
       if (!got) return false;
@@ -353,14 +377,13 @@ __device__ __forceinline__ void fa_bwd_f32_body(const BwdF32Params& prm, uint8_t
             const float4 pv = prev[c * 8 + (i >> 2)];
             float4 w = make_float4((__uint_as_float(a[i]) + pv.x) * f, (__uint_as_float(a[i + 1]) + pv.y) * f,
                                    (__uint_as_float(a[i + 2]) + pv.z) * f, (__uint_as_float(a[i + 3]) + pv.w) * f);
-            if (rotate) {
-              const float4 cs = *reinterpret_cast<const float4*>(tab + (i >> 1));   // (cos, sin) of two pairs
-              w = make_float4(w.x * cs.x + w.y * cs.y, w.y * cs.x - w.x * cs.y, w.z * cs.z + w.w * cs.w, w.w * cs.z - w.z * cs.w);
-            }
+            if (rotate) w = rotate_back(w, *reinterpret_cast<const float4*>(tab + (i >> 1)));   // (cos, sin) of two pairs
+            if (last) z = nonfinite(nonfinite(nonfinite(nonfinite(z, w.x), w.y), w.z), w.w);
             *reinterpret_cast<float4*>(out + c * 32 + i) = w;
           }
         }
       }
+      if (last && prm.causal && z != 0.f) fa_bwd_f32_visible<KV>(prm, bh0, x_idx, KV && g, KV ? 0 : g * 32, KV ? D : min(32, width), out);
       return true;
     };
     for (int n = 0; n < n_iter; ++n) {
@@ -434,7 +457,7 @@ __device__ __forceinline__ void fa_bwd_f32_body(const BwdF32Params& prm, uint8_t
 
 // Grid: for each rank (0 = most streamed tiles under the causal mask) the dK/dV CTAs of every K/V slice, then the dQ CTAs
 // of every query slice: the longest CTAs start first.
-__global__ void __launch_bounds__(416, 1) fa_bwd_f32_sm100_kernel(const BwdF32Params prm) {
+__global__ void __launch_bounds__(416, 1) fa_bwd_f32_sm100_kernel(const __grid_constant__ BwdF32Params prm) {
   using T = BwdF32Traits;
   using namespace ptx;
   extern __shared__ __align__(1024) uint8_t smem[];

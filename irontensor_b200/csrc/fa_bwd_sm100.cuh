@@ -32,6 +32,7 @@
 
 #include "rope.cuh"
 #include "sm100_ptx.cuh"
+#include "visible_pairs.cuh"
 
 namespace it {
 
@@ -72,6 +73,7 @@ struct BwdParams {
   __nv_bfloat16* dk;       // [BH, S, D]
   __nv_bfloat16* dv;       // [BH, S, D]
   int* status;
+  const __nv_bfloat16 *q, *k, *v, *d_o;   // PAD: for rows computed again (visible_pairs.cuh)
   int S;
   int S_pad;
   int BH;
@@ -181,12 +183,36 @@ __global__ void fa_bwd_prepare_kernel(const __nv_bfloat16* __restrict__ o, const
   }
 }
 
+// Rows that are not finite, over the pairs that the causal mask leaves visible (visible_pairs.cuh).
+__device__ __forceinline__ VisiblePairs<__nv_bfloat16> fa_bwd_pairs(const BwdParams& prm) {
+  return {prm.q, prm.k, prm.v, prm.d_o, prm.st, prm.st_kv, prm.head_dim, prm.scale_log2};
+}
+// Columns [col, col + n) of a finished row of dK or dV, over all query heads of the group.
+__device__ __noinline__ void fa_bwd_visible_dkv(const BwdParams& prm, bool is_dk, int bh0, int row, int col, int n) {
+  const VisiblePairs<__nv_bfloat16> t = fa_bwd_pairs(prm);
+  __nv_bfloat16* out = (is_dk ? prm.dk : prm.dv) + prm.st_kv.slice(bh0) + static_cast<long long>(row) * prm.st_kv.row;
+  for (int c = col; c < min(col + n, prm.head_dim); c += 4) {
+    float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int h = 0; h < prm.st_kv.group; ++h) {
+      const size_t r = static_cast<size_t>(bh0 + h) * prm.S_pad;
+      g = visible_dkv(t, is_dk, bh0 + h, row, row, prm.S, c, prm.lse2_pad + r, 1.f, prm.delta_pad + r, g);
+    }
+    if (is_dk && prm.rope_table != nullptr)
+      g = rotate_back(g, *reinterpret_cast<const float4*>(prm.rope_table + static_cast<size_t>(row) * (prm.head_dim >> 1) + (c >> 1)));
+    const float f = is_dk ? prm.scale : 1.0f;
+    *reinterpret_cast<uint2*>(out + c) = make_uint2(ptx::pack_bf16(g.x * f, g.y * f), ptx::pack_bf16(g.z * f, g.w * f));
+  }
+}
+
 // ------------------------------------------------------------------ (3) finish
 // With a rotary table the gradient is rotated back through the rotary embedding on its way out
 // (src/shaders/backward/rope.metal:25-62), so dq is the gradient of the un-rotated queries.
-__global__ void fa_bwd_finish_kernel(const float* __restrict__ dq_accum, __nv_bfloat16* __restrict__ dq,
+// PAD: under the causal mask a gradient that is not finite is computed again over the keys that its query sees.  (The launch
+// bound keeps the registers of that rare call from halving the threads that wait for memory: 1 of 12 us.)
+template <bool PAD>
+__global__ void __launch_bounds__(256, 8) fa_bwd_finish_kernel(const float* __restrict__ dq_accum, __nv_bfloat16* __restrict__ dq,
                                      size_t n_vec4, float scale, int S, int D, ptx::TensorStrides st,
-                                     const float2* __restrict__ rope_table) {
+                                     const float2* __restrict__ rope_table, const __grid_constant__ BwdParams prm) {
   ptx::grid_dep_wait();   // every reduce-add of the main kernel has landed
   const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n_vec4) return;
@@ -196,10 +222,12 @@ __global__ void fa_bwd_finish_kernel(const float* __restrict__ dq_accum, __nv_bf
   const int d = static_cast<int>(e - row * D);
   const int bh = static_cast<int>(row / S);
   const int s_ = static_cast<int>(row - static_cast<size_t>(bh) * S);
-  if (rope_table != nullptr) {
-    const float4 cs = *reinterpret_cast<const float4*>(rope_table + static_cast<size_t>(s_) * (D >> 1) + (d >> 1));
-    v = make_float4(v.x * cs.x + v.y * cs.y, v.y * cs.x - v.x * cs.y, v.z * cs.z + v.w * cs.w, v.w * cs.z - v.z * cs.w);
+  if (PAD && prm.causal && any_nonfinite(v)) {
+    const size_t r = static_cast<size_t>(bh) * prm.S_pad + s_;
+    v = visible_dq(fa_bwd_pairs(prm), bh, s_, s_ + 1, d, prm.lse2_pad[r], prm.delta_pad[r]);
   }
+  if (rope_table != nullptr)
+    v = rotate_back(v, *reinterpret_cast<const float4*>(rope_table + static_cast<size_t>(s_) * (D >> 1) + (d >> 1)));
   uint2 w;
   w.x = ptx::pack_bf16(v.x * scale, v.y * scale);
   w.y = ptx::pack_bf16(v.z * scale, v.w * scale);
@@ -220,7 +248,7 @@ template <int D, int KT = 1, bool PAD = false, bool SPLIT = false>
 __global__ void __launch_bounds__(512, 1)
 fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
-                    const __grid_constant__ CUtensorMap tmap_dq, const BwdParams prm) {
+                    const __grid_constant__ CUtensorMap tmap_dq, const __grid_constant__ BwdParams prm) {
   using T = BwdTraits<D, KT>;
   using namespace ptx;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -717,7 +745,8 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 *reinterpret_cast<uint4*>(srow + c * 16 + v4 * 4) = make_uint4(ra[v4 * 4], ra[v4 * 4 + 1], ra[v4 * 4 + 2], ra[v4 * 4 + 3]);
             }
           }
-        } else
+        } else {
+        uint32_t again = 0;   // PAD: the thread's 16-column pieces that are not finite
 #pragma unroll 1
         for (int tw = 0; tw < 2 * nk_cta; ++tw) {   // dV then dK of each of the CTA's key tiles
           const int t = tw >> 1, which = tw & 1;
@@ -732,6 +761,13 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           for (int c = 0; c < HC / 16; ++c) {
             tmem_ld_x16(t_lane + col + c * 16, ra);
             tmem_wait_ld();
+            if (PAD) {
+              float z = 0.f;
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (half * HC + c * 16 + i < prm.head_dim) z = nonfinite(z, __uint_as_float(ra[i]));
+              if (z != 0.f && k_row < S) again |= 1u << (tw * (HC / 16) + c);
+            }
             if (which && prm.rope_table != nullptr && k_row < S) {   // dK leaves through the inverse rotary rotation of its key position
               const int d0 = half * HC + c * 16;
               const float4* tab = reinterpret_cast<const float4*>(
@@ -761,6 +797,13 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
               }
             }
           }
+        }
+        if (PAD && prm.causal && again != 0)
+          for (int b = 0; b < 2 * KT * (HC / 16); ++b)
+            if (again >> b & 1) {
+              const int tw = b / (HC / 16);
+              fa_bwd_visible_dkv(prm, tw & 1, bh0, (kt + (tw >> 1)) * T::BM + k_local, half * HC + b % (HC / 16) * 16, 16);
+            }
         }
       }
     }
@@ -823,6 +866,9 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       // together.  A part with no iterations left nothing to add.
       constexpr int N4 = 2 * T::BM * (D / 4);
       const int total = per_head * G, step = 256 * n_split;
+      uint32_t again = 0;   // PAD: the thread's float4s that are not finite
+      static_assert(N4 / (2 * 256) <= 16, "one bit each, from clusters of two on");
+      int bit = 0;
       for (int first = rank * 256 + static_cast<int>(threadIdx.x) - 128; first < N4; first += 4 * step) {
         float4 a[4];
 #pragma unroll
@@ -840,20 +886,27 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           for (int u = 0; u < 4; ++u) a[u] = make_float4(a[u].x + x[u].x, a[u].y + x[u].y, a[u].z + x[u].z, a[u].w + x[u].w);
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < 4; ++u, ++bit) {
           const int i = first + u * step;
           const int which = i / (T::BM * (D / 4)), row = (i / (D / 4)) % T::BM, d = (i % (D / 4)) * 4;
           const int k_row = kt * T::BM + row;
           if (i >= N4 || k_row >= S || (PAD && d >= prm.head_dim)) continue;
           float4 g = a[u];
+          if (PAD && any_nonfinite(g)) again |= 1u << bit;
           if (which && prm.rope_table != nullptr) {   // dK leaves through the inverse rotary rotation of its key position
             const float4 cs = *reinterpret_cast<const float4*>(
                 prm.rope_table + static_cast<size_t>(k_row) * ((PAD ? prm.head_dim : D) >> 1) + (d >> 1));
-            g = make_float4(g.x * cs.x + g.y * cs.y, g.y * cs.x - g.x * cs.y, g.z * cs.z + g.w * cs.w, g.w * cs.z - g.z * cs.w);
+            g = rotate_back(g, cs);
           }
           const float f = which ? prm.scale : 1.0f;
           __nv_bfloat16* out = (which ? prm.dk : prm.dv) + prm.st_kv.slice(bh0) + static_cast<long long>(k_row) * prm.st_kv.row + d;
           *reinterpret_cast<uint2*>(out) = make_uint2(pack_bf16(g.x * f, g.y * f), pack_bf16(g.z * f, g.w * f));
+        }
+      }
+      if (PAD && prm.causal && again != 0) {
+        for (int b = 0; b < 16; ++b) {
+          const int i = rank * 256 + static_cast<int>(threadIdx.x) - 128 + b * step;
+          if (again >> b & 1) fa_bwd_visible_dkv(prm, i >= T::BM * (D / 4), bh0, kt * T::BM + (i / (D / 4)) % T::BM, (i % (D / 4)) * 4, 4);
         }
       }
     }

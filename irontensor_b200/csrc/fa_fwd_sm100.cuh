@@ -22,6 +22,7 @@
 // TMEM columns (512 allocated): S0 [0,128) S1 [128,256) O0 [256,256+D) O1 [256+D,256+2D).
 #pragma once
 #include "sm100_ptx.cuh"
+#include "visible_pairs.cuh"
 
 namespace it {
 
@@ -72,10 +73,19 @@ struct FwdParams {
 // They also take full-width tensors of fewer than 128 rows.  The probabilities of these shapes are kept to 16 bits of
 // mantissa, as two bf16 terms in the 128 columns that S leaves (P V is two products): the CUDA-core kernels that had these
 // shapes before computed P in fp32, and one bf16 term would put O 2.0e-3 off 64 bits where the rounding of O itself is 1.6e-3.
+// PAD: a row that is not finite, over the keys that it sees alone.
+using FwdPairs = VisiblePairs<__nv_bfloat16>;
+__device__ __noinline__ void fa_fwd_visible(const FwdPairs& t, int bh, int row, float m, float inv_l, __nv_bfloat16* orow) {
+  for (int c = 0; c < t.D; c += 4) {
+    const float4 w = visible_o(t, bh, row, c, m, inv_l);
+    *reinterpret_cast<uint2*>(orow + c) = make_uint2(ptx::pack_bf16(w.x, w.y), ptx::pack_bf16(w.z, w.w));
+  }
+}
+
 template <int D, bool PAD = false>
 __global__ void __launch_bounds__(384, 1)
 fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                    const __grid_constant__ CUtensorMap tmap_v, const FwdParams prm) {
+                    const __grid_constant__ CUtensorMap tmap_v, const FwdParams prm, const __grid_constant__ FwdPairs pairs) {
   using T = FwdTraits<D>;
   using namespace ptx;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -495,9 +505,13 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       for (int c = 0; c < D / 32; ++c) tmem_ld_x32(t_o + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[c * 32]));
       tmem_wait_ld();
       if (q_row < S) {
+        float z = 0.f;   // PAD: NaN if the row is not finite
 #pragma unroll
         for (int v = 0; v < D / 8; ++v) {
           if (PAD && v * 8 >= prm.head_dim) break;
+          if (PAD)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) z = nonfinite(z, __uint_as_float(r[v * 8 + i]));
           uint4 w;
           w.x = pack_bf16(__uint_as_float(r[v * 8 + 0]) * inv_l, __uint_as_float(r[v * 8 + 1]) * inv_l);
           w.y = pack_bf16(__uint_as_float(r[v * 8 + 2]) * inv_l, __uint_as_float(r[v * 8 + 3]) * inv_l);
@@ -505,6 +519,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           w.w = pack_bf16(__uint_as_float(r[v * 8 + 6]) * inv_l, __uint_as_float(r[v * 8 + 7]) * inv_l);
           *reinterpret_cast<uint4*>(orow + v * 8) = w;
         }
+        if (PAD && prm.causal && z != 0.f) fa_fwd_visible(pairs, it.bh, q_row, m_used, inv_l, orow);
         if (prm.lse != nullptr)
           prm.lse[static_cast<size_t>(it.bh) * S + q_row] = (m_used + lg2(l_sum)) * 0.6931471805599453f;
       }

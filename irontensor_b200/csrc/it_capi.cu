@@ -468,7 +468,10 @@ it_status launch_fwd_sm100(it_ctx* ctx, it_stream* stream, int B, int H, int S, 
   const int Hkv = H / skv.group;
   cudaStream_t s = stream->s;
   using T = std::conditional_t<PP, it::FwdPPTraits<D>, it::FwdTraits<D>>;
-  auto kernel = PP ? it::fa_fwd_pp_sm100_kernel<D> : it::fa_fwd_sm100_kernel<D, PAD>;
+  const auto kernel = [] {
+    if constexpr (PP) return it::fa_fwd_pp_sm100_kernel<D>;
+    else return it::fa_fwd_sm100_kernel<D, PAD>;
+  }();
   CUtensorMap mq, mk, mv;
   it_status st;
   if ((st = make_tmap(ctx, &mq, q, B, H, S, head_dim, sq, 128)) != IT_OK) return st;
@@ -533,7 +536,12 @@ it_status launch_fwd_sm100(it_ctx* ctx, it_stream* stream, int B, int H, int S, 
     }
   }
   if (ctx->timing >= 2) IT_CUDA(cudaEventRecord(ctx->ev[0][0], s));
-  IT_CUDA(launch_dependent(kernel, static_cast<unsigned>(grid), T::THREADS, T::SMEM_BYTES, s, mq, mk, mv, p));
+  if constexpr (PP)
+    IT_CUDA(launch_dependent(kernel, static_cast<unsigned>(grid), T::THREADS, T::SMEM_BYTES, s, mq, mk, mv, p));
+  else
+    IT_CUDA(launch_dependent(kernel, static_cast<unsigned>(grid), T::THREADS, T::SMEM_BYTES, s, mq, mk, mv, p,
+                             it::FwdPairs{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
+                                          static_cast<const __nv_bfloat16*>(v), nullptr, stv, skv, head_dim, p.scale_log2}));
   if (ctx->timing >= 2) {
     IT_CUDA(cudaEventRecord(ctx->ev[0][1], s));
     ctx->ev_valid[0] = true;
@@ -665,6 +673,10 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
   p.dk = static_cast<__nv_bfloat16*>(dk);
   p.dv = static_cast<__nv_bfloat16*>(dv);
   p.status = ctx->d_status;
+  p.q = static_cast<const __nv_bfloat16*>(q);
+  p.k = static_cast<const __nv_bfloat16*>(k);
+  p.v = static_cast<const __nv_bfloat16*>(v);
+  p.d_o = static_cast<const __nv_bfloat16*>(d_o);
   p.S = S;
   p.S_pad = w.S_pad;
   p.BH = BH;
@@ -703,8 +715,8 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
   }
   if (ctx->timing >= 3) IT_CUDA(cudaEventRecord(ctx->ev[3][0], s));
   const size_t n4 = n_dq / 4;
-  IT_CUDA(launch_dependent(it::fa_bwd_finish_kernel, static_cast<unsigned>((n4 + 255) / 256), 256, 0, s,
-                           static_cast<const float*>(dq_accum), static_cast<__nv_bfloat16*>(dq), n4, p.scale, S, head_dim, sq, static_cast<const float2*>(rope_table)));
+  IT_CUDA(launch_dependent(it::fa_bwd_finish_kernel<PAD>, static_cast<unsigned>((n4 + 255) / 256), 256, 0, s,
+                           static_cast<const float*>(dq_accum), static_cast<__nv_bfloat16*>(dq), n4, p.scale, S, head_dim, sq, static_cast<const float2*>(rope_table), p));
   if (ctx->timing >= 3) {
     IT_CUDA(cudaEventRecord(ctx->ev[3][1], s));
     ctx->ev_valid[3] = true;

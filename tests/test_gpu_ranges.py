@@ -537,3 +537,73 @@ def test_keys_past_the_sequence_weigh_nothing(it_ctx, dtype, D):
         # of the D products rounds: probabilities are off by about 1e-4, whatever the type.
         err = (got - exact)[..., 1:].norm() / exact[..., 1:].norm()
         assert err.item() < (1e-2 if dtype == "bf16" else 5e-4)
+
+
+def visible_pairs_oracle(q, k, v, d_o, o, lse):
+    """Causal attention and its gradients, [B, S, H, D] in 64 bits, each row from the rows that it sees and no others."""
+    import torch
+    B, S, H, D = q.shape
+    G = H // k.shape[2]
+    kk, vv = (t.repeat_interleave(G, 2) for t in (k, v))
+    out, dq, dk, dv = (torch.zeros_like(q) for _ in range(4))
+    delta = (d_o * o).sum(-1)
+    for i in range(S):
+        s = torch.einsum("bhd,bkhd->bhk", q[:, i], kk[:, :i + 1]) / D ** 0.5
+        out[:, i] = torch.einsum("bhk,bkhd->bhd", s.softmax(-1), vv[:, :i + 1])
+        p = (s - lse[:, :, i, None]).exp()
+        ds = p * (torch.einsum("bhd,bkhd->bhk", d_o[:, i], vv[:, :i + 1]) - delta[:, i, :, None])
+        dq[:, i] = torch.einsum("bhk,bkhd->bhd", ds, kk[:, :i + 1]) / D ** 0.5
+        s = torch.einsum("bqhd,bhd->bhq", q[:, i:], kk[:, i]) / D ** 0.5
+        p = (s - lse[:, :, i:]).exp()
+        ds = p * (torch.einsum("bqhd,bhd->bhq", d_o[:, i:], vv[:, i]) - delta[:, i:].transpose(1, 2))
+        dk[:, i] = torch.einsum("bhq,bqhd->bhd", ds, q[:, i:]) / D ** 0.5
+        dv[:, i] = torch.einsum("bhq,bqhd->bhd", p, d_o[:, i:])
+    return out, dq, dk.view(B, S, H // G, G, D).sum(3), dv.view(B, S, H // G, G, D).sum(3)
+
+
+@pytest.mark.parametrize("dtype,B,S,H,Hkv,D,env", [
+    ("fp32", 2, 200, 2, 2, 64, {}), ("fp32", 1, 300, 4, 2, 32, {}), ("fp32", 2, 40, 2, 1, 60, {}),
+    ("bf16", 1, 300, 4, 4, 96, {"IT_BWD_SPLIT": "1"}), ("bf16", 1, 300, 8, 2, 96, {"IT_BWD_SPLIT": "2"}),
+    ("bf16", 1, 300, 4, 2, 40, {"IT_BWD_SPLIT": "4"}), ("bf16", 1, 300, 4, 4, 48, {"IT_BWD_KEY_TILES": "2"}),
+    ("bf16", 2, 100, 2, 2, 64, {}), ("bf16", 2, 70, 4, 1, 128, {}),
+])
+@pytest.mark.parametrize("where,value", [("tail of K and V", float("nan")), ("tail of K and V", float("inf")), ("head of Q and dO", float("nan")),
+                                         ("one value of V", float("-inf")), ("one value of dO", float("inf"))])
+def test_rows_that_are_not_finite_stay_with_those_who_see_them(it_ctx, monkeypatch, dtype, B, S, H, Hkv, D, env, where, value):
+    """A masked probability of 0 times an infinity is no 0: on the diagonal tile it must not meet one.  Every row of O, dQ, dK and dV
+    that sees finite rows only is finite, and right; the others are not finite, as in the oracle."""
+    import torch
+    from irontensor_b200 import Precision, Tensor, attention_gqa, attention_gqa_backward
+    for name, val in env.items():
+        monkeypatch.setenv(name, val)
+    gen = torch.Generator(device="cuda").manual_seed(S + D)
+    t = torch.bfloat16 if dtype == "bf16" else torch.float32
+    q, d_o = (torch.randn(B, S, H, D, generator=gen, device="cuda").to(t) for _ in range(2))
+    k, v = (torch.randn(B, S, Hkv, D, generator=gen, device="cuda").to(t) for _ in range(2))
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double().repeat_interleave(H // Hkv, 2)) / D ** 0.5
+    s = s.masked_fill(torch.ones(S, S, device="cuda").triu(1).bool(), float("-inf"))
+    o = torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1), v.double().repeat_interleave(H // Hkv, 2)).to(t).contiguous()
+    lse = s.logsumexp(-1).float().contiguous()
+    at = S - 25
+    if where == "tail of K and V":
+        k[:, at:, 0, 1], v[:, at:, 0] = value, value
+    elif where == "head of Q and dO":
+        q[:, :25, 0, 0], d_o[:, :25, H - 1] = value, value
+    elif where == "one value of V":
+        v[:, at, 0, 3] = value
+    else:
+        d_o[:, 30, 0, D - 1] = value
+    want = visible_pairs_oracle(*(x.double() for x in (q, k, v, d_o, o, lse)))
+    P = Precision.BF16 if dtype == "bf16" else Precision.FP32
+    args = [Tensor(x, list(x.shape), P) for x in (q, k, v, d_o, o)]
+    got = [attention_gqa(*args[:3], True)]
+    args[4].lse = Tensor(lse, [B, H, S], Precision.FP32)
+    got += attention_gqa_backward(args[3], *args[:3], args[4], True)
+    assert it_ctx.poll_status() == 0
+    tol = 6e-3 if dtype == "bf16" else 1e-5
+    for name, g, w in zip(("o", "dq", "dk", "dv"), got, want):
+        if name == "o" and dtype == "fp32":
+            continue       # the fp32 forward's row tiles multiply masked zeros, as they always did
+        g, fine = g.torch().double(), torch.isfinite(w)
+        assert torch.equal(torch.isfinite(g), fine), f"{name}: {(torch.isfinite(g) != fine).sum().item()} values of {fine.numel()}"
+        assert ((g - w)[fine].norm() / w[fine].norm()).item() < tol if fine.any() else True, name
