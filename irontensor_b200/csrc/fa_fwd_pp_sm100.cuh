@@ -372,7 +372,7 @@ fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
           const bool grow = m_new > m_cur + 8.0f;
           if (__any_sync(0xffffffffu, grow)) {   // rare: raise the reference and rescale O in TMEM
             m_next = fmaxf(m_cur, m_new);
-            const float f = ex2(m_cur - m_next);
+            const float f = (TWO_TERMS && m_cur == m_next) ? 1.0f : ex2(m_cur - m_next);   // both may be -inf
             // O holds tiles 0..j-1 once P(j-1) V(j-1) is complete; P(j) V(j) cannot start before this
             // group has written P(j).
             ok = mbar_wait(&v_empty[(j - 1) % T::STAGES], ((j - 1) / T::STAGES) & 1, abort_flag, prm.status,
@@ -399,7 +399,8 @@ fa_fwd_pp_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         // the one P buffer: P(j-1) V(j-1) must have read it before P(j) goes in; probed here, needed after the exponentials
         const bool p_free = (j == 0) || mbar_test_wait(&v_empty[(j - 1) % T::STAGES], ((j - 1) / T::STAGES) & 1);
         // P = 2^(s*scale - m), packed bf16 in place over the row's registers
-        const float neg_m = -m_used;
+        // heads whose scores are all -inf so far stay at (-inf, 0), as in fa_decode_kernel
+        const float neg_m = (TWO_TERMS && m_used == -INFINITY) ? 0.f : -m_used;
         float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {

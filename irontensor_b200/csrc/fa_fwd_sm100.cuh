@@ -444,7 +444,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           const bool grow = m_new > m_used + 8.0f;
           if (__any_sync(0xffffffffu, grow)) {   // rare: raise the reference and rescale O in TMEM
             const float m_next = fmaxf(m_used, m_new);
-            const float f = ex2(m_used - m_next);
+            const float f = (PAD && m_used == m_next) ? 1.0f : ex2(m_used - m_next);   // both may be -inf
             l_sum *= f;
             m_used = m_next;
             uint32_t tmp[16];
@@ -460,7 +460,8 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           }
         }
         // P = 2^(s*scale - m), packed bf16, written over S 32 keys at a time
-        const float neg_m = -m_used;
+        // A row whose scores are all -inf so far stays at (-inf, 0), as in the CUDA-core kernels that had the padded shapes.
+        const float neg_m = (PAD && m_used == -INFINITY) ? 0.f : -m_used;
         float l0 = 0.f, l1 = 0.f, l2 = 0.f, l3 = 0.f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {

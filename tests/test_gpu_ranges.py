@@ -607,3 +607,40 @@ def test_rows_that_are_not_finite_stay_with_those_who_see_them(it_ctx, monkeypat
         g, fine = g.torch().double(), torch.isfinite(w)
         assert torch.equal(torch.isfinite(g), fine), f"{name}: {(torch.isfinite(g) != fine).sum().item()} values of {fine.numel()}"
         assert ((g - w)[fine].norm() / w[fine].norm()).item() < tol if fine.any() else True, name
+
+
+@pytest.mark.parametrize("lowest", [float("-inf"), -3e38])
+def test_leading_keys_that_score_minus_infinity(it_ctx, lowest):
+    """Keys switched off by a column of the lowest value: a whole first tile of scores of -inf weighs nothing, in the padded forward
+    and in the decode of fewer than 256 positions (fp32 tensors too)."""
+    import torch
+    from irontensor_b200 import Precision, Tensor, attention_decode, attention_gqa
+    gen = torch.Generator(device="cuda").manual_seed(3)
+
+    def softmax_v(q, k, v, G):     # q [.., h, n, d] over the keys that are on
+        k, v = (x.double().repeat_interleave(G, 2).transpose(1, 2) for x in (k, v))
+        s = (q[..., 1:].double() @ k[..., 1:].transpose(-1, -2) + q[..., :1].double() * k[..., :1].transpose(-1, -2).clamp(min=-1e30)) / q.shape[-1] ** 0.5
+        return s, v
+
+    for t, P in ((torch.bfloat16, Precision.BF16), (torch.float32, Precision.FP32)):
+        B, S, H, D, off = 1, 300, 2, 96 if t == torch.bfloat16 else 64, 140
+        q, k, v = (torch.randn(B, S, H, D, generator=gen, device="cuda").to(t) for _ in range(3))
+        q[..., 0], k[..., 0] = 100.0, 0.0
+        k[:, :off, :, 0] = lowest
+        if t == torch.bfloat16:    # fp32 operands beyond bf16's range are beyond the split of the fp32 tensor-core forward
+            o = attention_gqa(*(Tensor(x, list(x.shape), P) for x in (q, k, v)), True).torch().double()
+            s, vd = softmax_v(q.transpose(1, 2), k, v, 1)
+            s = s.masked_fill(torch.ones(S, S, device="cuda").triu(1).bool(), float("-inf"))
+            want = (s.softmax(-1) @ vd).transpose(1, 2)
+            assert torch.isfinite(o[:, off:]).all()
+            assert ((o - want)[:, off:].norm() / want[:, off:].norm()).item() < 6e-3
+        for H, Hkv, n, off in ((16, 2, 250, 130), (16, 2, 100, 70), (32, 1, 255, 128), (8, 8, 250, 130)):
+            q = torch.randn(2, H, 64, generator=gen, device="cuda").to(t)
+            k, v = (torch.randn(2, 256, Hkv, 64, generator=gen, device="cuda").to(t) for _ in range(2))
+            q[..., 0], k[..., 0] = 100.0, 0.0
+            k[:, :off, :, 0] = lowest
+            o = attention_decode(*(Tensor(x, list(x.shape), P) for x in (q, k, v)), n).torch().double()
+            s, vd = softmax_v(q[:, :, None], k[:, :n], v[:, :n], H // Hkv)
+            want = (s.softmax(-1) @ vd)[:, :, 0]
+            assert ((o - want).norm() / want.norm()).item() < (1.85e-3 if t == torch.bfloat16 else 1e-5)
+    assert it_ctx.poll_status() == 0
