@@ -134,8 +134,9 @@ __device__ __forceinline__ void f32_tile_store(uint8_t* planes, int t, const flo
   ptx::fence_proxy_async_smem();
 }
 
-// `width` columns of the finished row x_idx of dQ (KV: of dK or dV) from column `col` on, over the visible pairs alone.  For rows
-// that are not finite; see visible_pairs.cuh.  `bh`: the row's query slice (KV: the first of the group).
+// `width` columns of the finished row x_idx of dQ (KV: of dK or dV) from column `col` on, over the visible pairs alone and in fp32
+// throughout.  For rows that are not finite; see visible_pairs.cuh.  Without the causal mask these too: a finite value above bf16's
+// largest (3.39e38, as in masks of the lowest fp32 value) has no three bf16 terms, and infinities become NaN there.  `bh`: the row's query slice (KV: the first of the group).
 template <bool KV>
 __device__ __noinline__ void fa_bwd_f32_visible(const BwdF32Params& prm, int bh, int x_idx, bool is_dv, int col, int width, float* out) {
   const VisiblePairs<float> t{prm.q, prm.k, prm.v, prm.d_o, prm.st, prm.st_kv, prm.D, prm.scale_log2};
@@ -144,8 +145,8 @@ __device__ __noinline__ void fa_bwd_f32_visible(const BwdF32Params& prm, int bh,
     float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int h = 0; h < (KV ? prm.st_kv.group : 1); ++h) {
       const size_t r = static_cast<size_t>(bh + h) * prm.S;
-      w = KV ? visible_dkv(t, !is_dv, bh + h, x_idx, x_idx, prm.S, col + i, prm.lse + r, LOG2E, prm.delta + r, w)
-             : visible_dq(t, bh, x_idx, x_idx + 1, col + i, prm.lse[r + x_idx] * LOG2E, prm.delta[r + x_idx]);
+      w = KV ? visible_dkv(t, !is_dv, bh + h, x_idx, prm.causal ? x_idx : 0, prm.S, col + i, prm.lse + r, LOG2E, prm.delta + r, w)
+             : visible_dq(t, bh, x_idx, prm.causal ? x_idx + 1 : prm.S, col + i, prm.lse[r + x_idx] * LOG2E, prm.delta[r + x_idx]);
     }
     if (!is_dv) {
       w = make_float4(w.x * prm.scale, w.y * prm.scale, w.z * prm.scale, w.w * prm.scale);
@@ -383,7 +384,7 @@ __device__ __forceinline__ void fa_bwd_f32_body(const BwdF32Params& prm, uint8_t
           }
         }
       }
-      if (last && prm.causal && z != 0.f) fa_bwd_f32_visible<KV>(prm, bh0, x_idx, KV && g, KV ? 0 : g * 32, KV ? D : min(32, width), out);
+      if (last && z != 0.f) fa_bwd_f32_visible<KV>(prm, bh0, x_idx, KV && g, KV ? 0 : g * 32, KV ? D : min(32, width), out);
       return true;
     };
     for (int n = 0; n < n_iter; ++n) {

@@ -644,3 +644,31 @@ def test_leading_keys_that_score_minus_infinity(it_ctx, lowest):
             want = (s.softmax(-1) @ vd)[:, :, 0]
             assert ((o - want).norm() / want.norm()).item() < (1.85e-3 if t == torch.bfloat16 else 1e-5)
     assert it_ctx.poll_status() == 0
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("S,D", [(200, 64), (40, 32)])
+def test_fp32_backward_with_keys_at_the_lowest_value(it_ctx, causal, S, D):
+    """Keys switched off by a column of -FLT_MAX, which no bf16 term holds: their probabilities are 0 and so are their parts."""
+    import torch
+    from irontensor_b200 import Precision, Tensor, attention_backward_recompute
+    gen = torch.Generator(device="cuda").manual_seed(S)
+    B, H = 1, 2
+    q, k, v, d_o = (torch.randn(B, H, S, D, generator=gen, device="cuda") for _ in range(4))
+    q[..., 0], k[..., 0] = 1000.0, 0.0
+    on = torch.arange(S, device="cuda") % 5 != 3
+    k[:, :, ~on, 0] = torch.finfo(torch.float32).min
+    seen = (torch.ones(S, S, device="cuda").tril().bool() if causal else torch.ones(S, S, device="cuda").bool()) & on
+    qd, kd, vd = (x.double().requires_grad_() for x in (q, k.masked_fill(~on[None, None, :, None], 0.0), v))
+    s = ((qd @ kd.transpose(-1, -2)) / D ** 0.5).masked_fill(~seen, float("-inf"))
+    o = s.softmax(-1) @ vd
+    o.backward(d_o.double())
+    args = [Tensor(x.contiguous(), [B, H, S, D], Precision.FP32) for x in (d_o, q, k, v, o.detach().float())]
+    lse = Tensor(s.detach().logsumexp(-1).float().contiguous(), [B, H, S], Precision.FP32)
+    got = attention_backward_recompute(*args, lse, causal=causal)
+    assert it_ctx.poll_status() == 0
+    for g, want in zip(got, (qd.grad, kd.grad, vd.grad)):
+        g = g.torch().double()
+        assert torch.isfinite(g).all()
+        err = (g - want)[..., 1:].norm() / want[..., 1:].norm()     # column 0: differences of terms 1000 times larger
+        assert err.item() < 1e-5
