@@ -688,7 +688,7 @@ it_status launch_bwd_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int S, int
   // At head_dim 64 a CTA can own two key tiles (tensor memory holds four accumulators of 64 columns): half as many
   // CTAs, so half as many start-ups and epilogues for the same work.  Taken when the launch has CTAs to spare (more
   // than two per SM with one key tile each); a launch that does not even fill the GPU is a latency case and keeps
-  // the shorter CTAs.  IT_BWD_KEY_TILES=1 or 2 in the environment overrides the choice (the tests run both forms).
+  // the shorter CTAs.  IT_BWD_KEY_TILES=1 or 2 in the environment overrides the choice.
   const char* force = getenv("IT_BWD_KEY_TILES");
   const bool two_tiles = (D == 64) && n_kt >= 2 &&
                          (force != nullptr ? force[0] == '2' : static_cast<long long>(n_kt) * B * Hkv > 2LL * ctx->sm_count);

@@ -298,8 +298,8 @@ def test_bf16_backward_split_over_a_cluster(it_ctx, monkeypatch, split, B, S, H,
 
 
 @pytest.mark.parametrize("S,D", [(100, 64), (127, 128), (300, 96), (200, 32), (260, 40)])
-def test_bf16_padded_shapes_keep_fp32_probabilities(it_ctx, S, D):
-    """Shapes of the padded tiles against 64 bits.  Rounding a result to bf16 costs 1.66e-3 of its norm (2^-9 of each element,
+def test_bf16_padded_shapes_round_their_results_only(it_ctx, S, D):
+    """Shapes of the padded tiles, whose P and dS are two bf16 terms, against 64 bits.  Rounding a result to bf16 costs 1.66e-3 of its norm (2^-9 of each element,
     uniform over the binades); delta, computed from the rounded O, adds to dQ and dK (1.9e-3 in all).  One bf16 term for P and
     dS would add as much again (2.0e-3, 2.3e-3 and 3.0e-3)."""
     import torch
@@ -672,3 +672,49 @@ def test_fp32_backward_with_keys_at_the_lowest_value(it_ctx, causal, S, D):
         assert torch.isfinite(g).all()
         err = (g - want)[..., 1:].norm() / want[..., 1:].norm()     # column 0: differences of terms 1000 times larger
         assert err.item() < 1e-5
+
+
+def _attention_and_gradients(q, k, v, d_o, causal, rope_base=None):
+    """O, dQ, dK, dV of [B, S, heads, D] tensors in 64 bits; with `rope_base` q and k are rotated tensors and dQ, dK those of the
+    tensors before the rotation."""
+    import torch
+    B, S, H, D = q.shape
+    q, k, v = (x.double().detach().requires_grad_() for x in (q, k, v))
+    kk, vv = (x.repeat_interleave(H // k.shape[2], 2) for x in (k, v))
+    s = torch.einsum("bqhd,bkhd->bhqk", q, kk) / D ** 0.5
+    if causal:
+        s = s.masked_fill(torch.ones(S, S, device="cuda").triu(1).bool(), float("-inf"))
+    o = torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1), vv)
+    o.backward(d_o.double())
+    dq, dk = q.grad, k.grad
+    if rope_base is not None:
+        inv = 1.0 / rope_base ** (torch.arange(0, D, 2, device="cuda").double() / D)
+        angle = torch.arange(S, device="cuda").double()[:, None, None] * inv
+        c, sn = angle.cos(), angle.sin()
+        dq, dk = (torch.stack((g[..., 0::2] * c + g[..., 1::2] * sn, g[..., 1::2] * c - g[..., 0::2] * sn), -1).flatten(-2) for g in (dq, dk))
+    return o.detach(), dq, dk, v.grad
+
+
+@pytest.mark.parametrize("B,S,H,Hkv,D,causal,rope,force", [
+    (1, 300, 4, 4, 32, True, True, True), (1, 300, 4, 2, 40, False, False, True), (2, 512, 4, 1, 56, True, True, True),
+    (1, 257, 4, 4, 56, False, True, True), (2, 130, 4, 2, 24, True, False, True), (1, 640, 2, 2, 40, True, False, True),
+    (16, 300, 8, 8, 32, True, True, False), (32, 200, 8, 8, 48, False, True, False),    # more than two CTAs per SM with one tile each
+])
+def test_bf16_padded_backward_with_two_key_tiles_per_cta(it_ctx, monkeypatch, B, S, H, Hkv, D, causal, rope, force):
+    """The padded backward whose CTAs own two key tiles, odd and even numbers of them: by the switch, and by the launcher's own rule."""
+    import torch
+    from irontensor_b200 import Precision, Tensor, attention_gqa, attention_gqa_backward
+    if force:
+        monkeypatch.setenv("IT_BWD_KEY_TILES", "2")
+    gen = torch.Generator(device="cuda").manual_seed(S + D)
+    q, d_o = (torch.randn(B, S, H, D, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(B, S, Hkv, D, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(2))
+    args = [Tensor(x, list(x.shape), Precision.BF16) for x in (q, k, v, d_o)]
+    o = attention_gqa(*args[:3], causal)
+    got = (o,) + tuple(attention_gqa_backward(args[3], *args[:3], o, causal, rope_base=10000.0 if rope else None))
+    assert it_ctx.poll_status() == 0
+    want = _attention_and_gradients(q, k, v, d_o, causal, 10000.0 if rope else None)
+    # the bounds of test_bf16_padded_shapes_round_their_results_only, 6 % wider for dV: some of these tensors have 6000 values
+    for name, g, w, bound in zip(("o", "dq", "dk", "dv"), got, want, (1.75e-3, 2.1e-3, 2.1e-3, 1.85e-3)):
+        rel = ((g.torch().double() - w).norm() / w.norm()).item()
+        assert rel < bound, f"{name}: {rel:.2e}"
