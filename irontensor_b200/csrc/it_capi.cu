@@ -553,21 +553,24 @@ it_status launch_fwd_sm100(it_ctx* ctx, it_stream* stream, int B, int H, int S, 
 
 // Which forward kernel takes a full-width bf16 launch: one query tile per CTA whose two softmax groups alternate over the key
 // tiles (true), or two query tiles per work item (false).  Where the launch does not fill the GPU, what counts is how long a
-// CTA walks its key tiles: 0.83 us per tile with one query tile, 1.8 us per pair of tiles with two (each group then waits for
-// its own S, softmax and P V in turn).  Where it does, what counts is the time per tile with every SM busy: 0.85 us against
-// 1.6 (head_dim 64) or 1.9 us (128) per PAIR, and a CTA's set-up and epilogue: 3.5 us for each wave of CTAs against 3 us per
-// item of a CTA that walks items in a loop.  Fitted to 165 shapes, 4 to 256 slices of 128 to 8192 rows, both kernels timed on
-// each: the estimate picks the slower one by more than 3 % on three of them (8 to 18 %, 32 slices of 2048 and 3000 rows).
+// CTA walks its key tiles: about 1 us per tile with one query tile, 1.65 us per pair of tiles with two (each group then waits for
+// its own S, softmax and P V in turn); without the causal mask every CTA walks all of them, and a second or third wave of CTAs
+// costs half of that again.  Where it does, what counts is the time per tile with every SM busy: 0.74 us against 1.65 (head_dim 64)
+// or 1.75 us (128) per PAIR, and a CTA's set-up and epilogue: 3.6 us for each wave of CTAs against 3 us per item of a CTA that
+// walks items in a loop.  Fitted to 399 shapes, 4 to 256 slices of 128 to 8192 rows, causal and not, both kernels timed on each:
+// where the estimate takes one query tile it is nowhere more than 1.1 % behind, and all in all 1.6 % from the better choice.
 // one against two, us: 8 slices of 2048 rows 17 and 31 (head_dim 64), 19 and 35 (128); 16 of 3000, head_dim 64, 43 and 56;
-// 64 of 4096 247 and 209 (64), 280 and 277 (128); 64 of 8192, head_dim 128, 958 and 1057; 256 of 1024 118 and 76 (64).
+// 64 of 4096 247 and 209 (64), 280 and 277 (128); 64 of 8192, head_dim 128, 958 and 1057; 256 of 1024 118 and 76 (64);
+// 48 of 513 15.0 and 13.0 (64), 17.6 and 15.5 (128); 32 of 513 without the mask 16.4 and 14.5 (64).
 bool fwd_one_tile(int sm_count, int D, long long slices, int S, int causal) {
   const long long nt = (S + 127) / 128, pairs = (nt + 1) / 2;
   // key tiles per slice, walked by query tiles or by pairs of them; under the causal mask pair p sees min(2p + 2, nt)
   const long long one_tiles = causal ? nt * (nt + 1) / 2 : nt * nt;
   const long long two_tiles = causal ? pairs * (pairs + 1) - (nt & 1) : pairs * nt;
-  const double sms = sm_count, items = static_cast<double>(slices * pairs);
-  const double one = std::max(0.83 * nt, 0.85 * slices * one_tiles / sms) + 3.5 * std::ceil(slices * nt / sms);
-  const double two = std::max(1.8 * nt, (D == 64 ? 1.6 : 1.9) * slices * two_tiles / sms) + 3.0 * std::max(1.0, items / sms);
+  const double sms = sm_count, items = static_cast<double>(slices * pairs), waves = std::ceil(slices * nt / sms);
+  const double walk = 0.98 * nt * (causal || waves > 3.0 ? 1.0 : 0.5 * (1.0 + waves));
+  const double one = std::max(walk, 0.74 * slices * one_tiles / sms) + 3.6 * waves;
+  const double two = std::max(1.65 * nt, (D == 64 ? 1.65 : 1.75) * slices * two_tiles / sms) + 3.0 * std::max(1.0, items / sms);
   return one < two;
 }
 
