@@ -32,12 +32,10 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
   return t;
 }
 
-// True in exactly one lane of a converged warp.  Single-thread roles branch on this and not on `lane == 0`: the compiler then
-// knows that one thread runs the branch, keeps addresses, descriptors and loop state in uniform registers and feeds them to
-// tcgen05.mma and TMA directly; under a lane test every operand of every instruction is moved there first, and the thread
-// that issues the MMAs is what the pipelines wait for.  Measured, lane test -> elect (backward main kernel): B4 H16 S8192
-// D128 3.28 -> 2.65 ms, B32 H12 S1024 D64 312 -> 275 us; forward of the latter 139 -> 121 us; fp32 B8 H12 S512 D64 forward
-// 74 -> 64 us, backward 183 -> 153 us.
+// True in exactly one lane of a converged warp (elect.sync).  Single-thread roles branch on this and not on `lane == 0`, which says
+// the same without saying that it is one thread.  Measured, lane test -> elect, kernels alone: B4 H16 S8192 D128 backward main
+// 3.28 -> 2.65 ms; fp32 B8 H12 S512 D64 forward 74 -> 64 us, backward 183 -> 153 us.  Whole steps gain less, as the GPU's clock
+// falls under load (B32 H12 S1024 D64, forward + backward, with all else of the time: 502 -> 465 us).
 __device__ __forceinline__ bool elect_one() {
   uint32_t ok;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
