@@ -917,6 +917,10 @@ it_status launch_decode_sm100(it_ctx* ctx, cudaStream_t s, int B, int H, int Hkv
     // clusters that are all resident at once: one of 8 needs 8 free SMs in one GPC, and a second wave doubles the launch
     // (16 clusters of 8: 15.6 us for 1000 positions, 16 of 4: 9)
     while (c > 2 && base_ctas > max_clusters<D>(ctx, c)) c /= 2;
+    // two CTAs of two or three tiles each lose to one: what they save is a tile or two, and the merge costs as much (16 heads,
+    // 2 K/V heads, 300 positions: head_dim 64 6.8 and 5.8 us, 128 7.6 and 6.7; 640: 7.7 and 7.2, 1000: 8.5 and 9.7); at head_dim 128
+    // four of one or two tiles lose too (B8, 4 K/V heads, 500 positions 8.3 and 7.5)
+    if (n_tiles < 6 && (c == 2 || (D == 128 && c == 4))) c = 1;
     // Two waves of CTAs of which the second is less than half full: half as long CTAs run in three.  A wave costs 10 us besides, so
     // from 64 tiles on: 160 (batch, K/V head) pairs of 8190 positions 106 -> 95 us at head_dim 64, 133 -> 123 at 128; 16000
     // positions 196 -> 162 (64); 200 pairs 106 -> 97 and 137 -> 135.  4000 positions: 58 and 59, 72 and 73.  216 pairs at
@@ -1523,8 +1527,10 @@ it_status it_attention_decode(it_ctx* ctx, it_stream* stream, it_dtype dtype, in
   const long long bytes = 4LL * B * Hkv * kv_len * D;   // both caches, bf16
   // Below 256 positions, where the pipeline needs two bf16 terms of P, groups of up to four go to the CUDA cores whatever the batch
   // (B64 with 8 K/V heads and 32 heads, 200 positions: head_dim 64 23.3 / 12.7, 128 28.1 / 21.8), larger ones do not (B64 with 2
-  // and 64: 5.9 / 25.5 and 7.1 / 39.0; B4 with 2 and 16: 6.6 / 5.7 and 7.2 / 6.7).
-  const bool short_cache = kv_len < (G <= 4 ? 256 : 64) || (G == 1 && (D == 64 || bytes <= 100LL << 20)) ||
+  // and 64: 5.9 / 25.5 and 7.1 / 39.0; B32 with 2 and 16, 63 positions: 5.2 / 5.3 and 5.9 / 11.2), and only the shortest caches
+  // are read sooner by CUDA cores there (B4 with 2 and 16, head_dim 64, 32 positions 4.9 / 4.1, 48: 4.9 / 5.1; 128, 16: 5.4 / 4.2,
+  // 24: 5.4 / 5.7).
+  const bool short_cache = kv_len < (G <= 4 ? 256 : D == 64 ? 48 : 24) || (G == 1 && (D == 64 || bytes <= 100LL << 20)) ||
                            (G <= 4 && kv_len <= (D == 64 ? 2500 : 1200) && bytes <= (D == 64 ? 16LL : 5LL) << 20);
   if (dtype == IT_BF16 && (D == 64 || D == 128) && G <= 128 && !short_cache)
     return D == 128 ? launch_decode_sm100<128>(ctx, stream->s, B, H, Hkv, kv_len, max_len, q, k_cache, v_cache, o, lse, ws)

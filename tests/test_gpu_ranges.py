@@ -471,7 +471,8 @@ def test_captured_forwards_give_their_counters_back(it_ctx):
 
 
 @pytest.mark.parametrize("B,H,Hkv,D,kv_len", [(4, 16, 2, 64, 64), (4, 16, 2, 128, 255), (4, 32, 1, 128, 129), (2, 96, 1, 64, 200),
-                                              (64, 32, 8, 128, 200), (40, 16, 16, 128, 255)])
+                                              (64, 32, 8, 128, 200), (40, 16, 16, 128, 255), (4, 16, 2, 128, 24),
+                                              (32, 16, 2, 64, 48), (2, 40, 4, 128, 23)])
 def test_short_bf16_decode_rounds_its_result_only(it_ctx, B, H, Hkv, D, kv_len):
     """Below 256 positions the rounding of the result is all the error, whatever the group and the batch (fp32 probabilities, or two
     bf16 terms of them).  Rounding to 8 bits costs a value
