@@ -823,7 +823,9 @@ it_status launch_gemm(it_ctx* ctx, cudaStream_t s, int M, int N, int K, const vo
   };
   int bn = 256;
   if (!RS) {
-    const double c256 = cost(256, 1.0), c128 = cost(128, 0.575), c64 = cost(64, 0.42);
+    // (Fewer than 32 rows of A make a launch of 64-column tiles up to twice as slow, of 128-column ones not: 24 x 2048 -> 6144
+    // 14.5, 8.9 and 12.4 us with 64, 128 and 256, 32 rows 7.4, 7.8 and 12.7.  The cause is not known.)
+    const double c256 = cost(256, 1.0), c128 = cost(128, 0.575), c64 = cost(64, LAYOUT == 0 && M < 32 ? 0.9 : 0.42);
     bn = c64 < c128 && c64 < c256 ? 64 : c128 < c256 ? 128 : 256;
     const long long pair_tiles = static_cast<long long>((M + 255) / 256) * ((N + 255) / 256), pairs = std::max(1, ctx->sm_count / 2);
     const double c_pair = static_cast<double>((pair_tiles + pairs - 1) / pairs) * 0.89;
