@@ -1463,7 +1463,11 @@ it_status it_rope_qk(it_ctx* ctx, it_stream* stream, it_dtype dtype, int32_t B, 
   if ((row_bytes & 15) == 0 && aligned16(q_in) && aligned16(q_out) && aligned16(k_in) && aligned16(k_out)) {
     // as many positions per CTA as have one sine per thread, as long as that leaves four CTAs per SM
     const int64_t rows = static_cast<int64_t>(B) * S;
-    const int n_pos = static_cast<int>(std::clamp<int64_t>(rows / (4LL * ctx->sm_count), 1, 256 / half));
+    // ... and no more than four chunks a thread, all its loads in flight together, unless the launch is long anyway (us, before and
+    // now: fp32 2 x 1003 positions of 16 + 4 heads of 96: 8.8 and 8.1; 3000 of 32 + 8 of 128: fp32 31.4 and 28.3, bf16 20.0 and 18.8)
+    int n_pos = static_cast<int>(std::clamp<int64_t>(rows / (4LL * ctx->sm_count), 1, 256 / half));
+    const int batch = std::max(2, 1024 / (n_heads * row_bytes / 16));
+    if (n_pos > batch && rows <= 16LL * ctx->sm_count * batch) n_pos = batch;
     const unsigned ctas = static_cast<unsigned>((rows + n_pos - 1) / n_pos);
 #define IT_ROPE_CHUNKS(ST, INV)                                                                                               \
   IT_CUDA(launch_dependent(it::rope_qk_chunks_kernel<ST, INV>, ctas, 256, 0, stream->s, static_cast<const ST*>(q_in),         \
