@@ -28,7 +28,7 @@ def check_bf16(got, want, name, rel_scale=1.0):
 # H is chosen so that a tensor has at least 4000 elements: the relative-L2 bounds of check_bf16 lie 10 % above the worst
 # figure of large tensors, and the relative error of an L2 norm estimated from N values is 1 / sqrt(2 N) = 1.1 %.
 @pytest.mark.parametrize("S,H,D,causal", [
-    (2, 256, 8, True), (31, 16, 16, True), (65, 8, 40, False), (127, 8, 64, True), (127, 4, 128, False),   # shorter than a tile
+    (2, 256, 8, True), (31, 16, 16, True), (64, 160, 16, True), (50, 150, 16, False), (65, 8, 40, False), (127, 8, 64, True), (127, 4, 128, False),   # shorter than a tile
     (128, 4, 32, True), (129, 4, 8, True), (300, 3, 24, True), (257, 2, 56, False),                        # padded to 64 columns
     (130, 4, 72, True), (300, 3, 80, False), (1003, 2, 96, True), (256, 2, 120, True), (385, 2, 104, False),   # padded to 128
 ])
